@@ -242,6 +242,11 @@ struct hm_handle {
     bool vp_wide = false;                 // every leaf panel row-major with ld == width == 20 (leaf_up_w)
     int wide_tree = 1;                    // lane-per-RHS tree kernels: 0 never, 1 from 32 RHS, 2 from 2 (HM_OPT_WIDE_TREE)
     int ring_tile = 0;                    // per-warp ring tile (HM_OPT_RING_TILE)
+    // the panels with those of more than kPartRows rows split by rows (leaf_up's
+    // parts), or none when no panel is that tall
+    hm_vpanel *d_vp_split = nullptr;
+    hm_vpart *d_vparts = nullptr;
+    int n_vp_split = 0, n_part_slots = 0, n_part_counts = 0;
     hm_xfer *d_up = nullptr;
     std::vector<int> up_ptr;
     hm_m2l_row *d_m2l_rows = nullptr;
@@ -282,6 +287,7 @@ struct hm_handle {
     struct StreamCtx {
         void *p = nullptr;
         size_t bytes = 0;
+        int *count = nullptr;       // leaf_up's arrival counters (n_part_counts zeros between products)
         cudaStream_t side = nullptr;
         cudaEvent_t fork = nullptr, join = nullptr;
         cudaEvent_t mid = nullptr;  // a point inside the tree passes where the near field may start
@@ -487,6 +493,60 @@ void set_vp_caps(hm_handle *h, const std::vector<hm_vpanel> &vps)
     h->vp_covers_x = ok && cur == h->ny;
 }
 
+// Rows of a basis panel one warp takes: a taller panel is split into parts of
+// this many rows, its parts into groups of kPartGroup (leaf_up).  128 rows is
+// what leaf_up stages in shared memory; a 16,384-row HODLR product in FP64 took
+// 1,350 us with one warp per panel and takes 47 us (what issuing its five launches takes) with these parts.
+constexpr int kPartRows = 128, kPartGroup = 64;
+
+int split_tall_panels(hm_handle *h, const std::vector<hm_vpanel> &vps, cudaStream_t st)
+{
+    bool tall = false;
+    for (const hm_vpanel &p : vps) tall |= p.nrows > kPartRows;
+    if (!tall || h->storage == HM_DF64) return HM_OK;
+    std::vector<hm_vpanel> recs;
+    std::vector<hm_vpart> parts;
+    int64_t nslots = 0, ngroups = 0, npanels = 0;
+    for (const hm_vpanel &p : vps) {
+        if (p.nrows <= kPartRows) {
+            recs.push_back(p);
+            parts.push_back(hm_vpart{});
+            continue;
+        }
+        const int np = (p.nrows + kPartRows - 1) / kPartRows, ng = (np + kPartGroup - 1) / kPartGroup;
+        for (int i = 0; i < np; ++i) {
+            hm_vpanel q = p;
+            q.row0 += (int64_t)i * kPartRows;
+            q.off += (int64_t)i * kPartRows * p.ld;
+            q.nrows = std::min(kPartRows, p.nrows - i * kPartRows);
+            recs.push_back(q);
+            const int g = i / kPartGroup;
+            hm_vpart v;
+            v.part = (int32_t)(nslots + i);
+            v.part0 = (int32_t)(nslots + (int64_t)g * kPartGroup);
+            v.nparts = std::min(kPartGroup, np - g * kPartGroup);
+            v.group = (int32_t)(ngroups + g);
+            v.group0 = (int32_t)ngroups;
+            v.ngroups = ng;
+            v.gpart = (int32_t)(nslots + np);
+            v.panel = (int32_t)npanels;          // + the group counters, below
+            parts.push_back(v);
+        }
+        nslots += np + (ng > 1 ? ng : 0);
+        ngroups += ng;
+        npanels += 1;
+    }
+    if ((int64_t)recs.size() > INT32_MAX || nslots > INT32_MAX) return HM_OK;      // whole panels
+    for (hm_vpart &v : parts) v.panel += (int32_t)ngroups;
+    HM_TRY(h->upload(&h->d_vp_split, recs, st));
+    HM_TRY(h->upload(&h->d_vparts, parts, st));
+    HM_CK(cudaStreamSynchronize(st));             // the host vectors go
+    h->n_vp_split = (int)recs.size();
+    h->n_part_slots = (int)nslots;
+    h->n_part_counts = (int)(ngroups + npanels);
+    return HM_OK;
+}
+
 // HM_DF64 storage: the FP64 panel values become (h, l) FP32 pairs in place;
 // a value too large for the pair is an error (HM_ERR_UNSUPPORTED).
 int to_double_float(hm_handle *h, double *P, int64_t n, cudaStream_t st)
@@ -529,6 +589,7 @@ int build_device(hm_handle *h, const Plan &P, const std::vector<double> &cheb, c
     HM_TRY(h->upload(&vpf, P.vpanel_fill, st));
     h->d_vp = vp; h->n_vp = (int)P.vpanels.size();
     set_vp_caps(h, P.vpanels);
+    HM_TRY(split_tall_panels(h, P.vpanels, st));
     HM_TRY(h->upload(&h->d_up, P.up, st));
     h->up_ptr = P.up_level_ptr;
     HM_TRY(h->upload(&h->d_m2l_rows, P.m2l_rows, st));
@@ -644,6 +705,7 @@ int build_hier_device(hm_handle *h, const Plan &P, const std::vector<double> &vs
     HM_TRY(h->upload(&vp, P.vpanels, st));
     h->d_vp = vp; h->n_vp = (int)P.vpanels.size();
     set_vp_caps(h, P.vpanels);
+    HM_TRY(split_tall_panels(h, P.vpanels, st));
     HM_TRY(h->upload(&h->d_m2l_rows, P.m2l_rows, st));
     h->n_m2l_rows = (int)P.m2l_rows.size();
     HM_TRY(h->upload(&h->d_m2l_ents, P.m2l_ents, st));
@@ -721,12 +783,18 @@ ScratchLayout scratch_layout(const hm_handle *h, int k)
 }
 
 // Per-call scratch of hm_mul: the coefficients plus, for up to kPartMaxK
-// right-hand sides with the side stream, the far-field rows (nx x k, type A).
+// right-hand sides with the side stream, the far-field rows (nx x k, type A),
+// then the partial sums of split basis panels.
 template <typename A>
-size_t stream_scratch_bytes(const hm_handle *h, int k)
+size_t parts_off(const hm_handle *h, int k)
 {
     const ScratchLayout L = scratch_layout<A>(h, k);
     return L.yfar_off + (k <= 8 ? align256((size_t)h->nx * k * sizeof(A)) : 0);
+}
+template <typename A>
+size_t stream_scratch_bytes(const hm_handle *h, int k)
+{
+    return parts_off<A>(h, k) + align256((size_t)h->n_part_slots * k * 32 * sizeof(A));
 }
 
 // Scratch, side stream and fork/join events for products issued on stream st.
@@ -747,6 +815,12 @@ int stream_ctx(hm_handle *h, cudaStream_t st, size_t bytes, hm_handle::StreamCtx
         sc.p = nullptr; sc.bytes = 0;
         HM_CK(device_malloc_async(&sc.p, bytes, st));
         sc.bytes = bytes;
+    }
+    if (h->n_part_counts && !sc.count) {
+        void *c = nullptr;
+        HM_CK(device_malloc_async(&c, (size_t)h->n_part_counts * sizeof(int), st));
+        HM_CK(cudaMemsetAsync(c, 0, (size_t)h->n_part_counts * sizeof(int), st));
+        sc.count = static_cast<int *>(c);
     }
     *out = &sc;
     return HM_OK;
@@ -796,7 +870,7 @@ inline int last_band(const std::vector<int> &ptr)
 // field, downward transfers level by level.  QC right-hand sides per warp.
 template <typename S, typename A, int QC>
 int launch_tree_qc(hm_handle *h, const MulArgs<S> &ma, cudaStream_t st, A *t, A *s, bool timing, cudaEvent_t mid,
-                   int mid_after, bool *ends_with_kernel)
+                   int mid_after, bool *ends_with_kernel, const LeafParts<A> &lp)
 {
     const int r = h->r, k = ma.k;
     // a launch may be a programmatic dependent while the previous operation on
@@ -823,10 +897,11 @@ int launch_tree_qc(hm_handle *h, const MulArgs<S> &ma, cudaStream_t st, A *t, A 
             }
         }
         if (h->n_vp && !leaf_done) {
-            const size_t smem = (size_t)kWarpsPerCta * leaf_up_warp_bytes<S, A, QC>(h->vp_cap, h->vp_wcap);
+            const int cap = lp.rec ? kPartRows : h->vp_cap, n = lp.rec ? h->n_vp_split : h->n_vp;
+            const size_t smem = (size_t)kWarpsPerCta * leaf_up_warp_bytes<S, A, QC>(cap, h->vp_wcap);
             HM_TRY(ensure_smem(leaf_up<S, A, QC>, smem));
-            leaf_up<S, A, QC><<<warp_ctas(h->n_vp), 32 * kWarpsPerCta, smem, st>>>(
-                ma, h->d_vp, h->n_vp, static_cast<const S *>(h->d_V), t, r, h->vp_cap, h->vp_wcap);
+            leaf_up<S, A, QC><<<warp_ctas(n), 32 * kWarpsPerCta, smem, st>>>(
+                ma, lp.rec ? h->d_vp_split : h->d_vp, n, static_cast<const S *>(h->d_V), t, r, cap, h->vp_wcap, lp);
             HM_CK_LAUNCH("leaf_up");
             chain = true;
         }
@@ -1019,7 +1094,7 @@ int launch_tree_wide(hm_handle *h, const MulArgs<S> &ma, cudaStream_t st, A *t, 
             const size_t smem = (size_t)kWarpsPerCta * leaf_up_warp_bytes<S, A, 8>(h->vp_cap, h->vp_wcap);
             HM_TRY(ensure_smem(leaf_up<S, A, 8>, smem));
             leaf_up<S, A, 8><<<warp_ctas(h->n_vp), 32 * kWarpsPerCta, smem, st>>>(
-                ma, h->d_vp, h->n_vp, static_cast<const S *>(h->d_V), t, h->r, h->vp_cap, h->vp_wcap);
+                ma, h->d_vp, h->n_vp, static_cast<const S *>(h->d_V), t, h->r, h->vp_cap, h->vp_wcap, LeafParts<A>{});
             HM_CK_LAUNCH("leaf_up");
             chain = true;
         } else if (h->n_vp) {
@@ -1080,8 +1155,8 @@ int launch_tree_wide(hm_handle *h, const MulArgs<S> &ma, cudaStream_t st, A *t, 
 }
 
 template <typename S, typename A>
-int launch_tree(hm_handle *h, const MulArgs<S> &ma, cudaStream_t st, A *t, A *s, bool timing,
-                cudaEvent_t mid = nullptr, int mid_after = 0, bool *ends_with_kernel = nullptr)
+int launch_tree(hm_handle *h, const MulArgs<S> &ma, cudaStream_t st, A *t, A *s, bool timing, cudaEvent_t mid,
+                int mid_after, bool *ends_with_kernel, const LeafParts<A> &lp)
 {
     bool ends = false;
     int rc;
@@ -1095,8 +1170,8 @@ int launch_tree(hm_handle *h, const MulArgs<S> &ma, cudaStream_t st, A *t, A *s,
             return rc;
         }
     }
-    rc = ma.k == 1 ? launch_tree_qc<S, A, 1>(h, ma, st, t, s, timing, mid, mid_after, &ends)
-                   : launch_tree_qc<S, A, 8>(h, ma, st, t, s, timing, mid, mid_after, &ends);
+    rc = ma.k == 1 ? launch_tree_qc<S, A, 1>(h, ma, st, t, s, timing, mid, mid_after, &ends, lp)
+                   : launch_tree_qc<S, A, 8>(h, ma, st, t, s, timing, mid, mid_after, &ends, lp);
     if (ends_with_kernel) *ends_with_kernel = ends;
     return rc;
 }
@@ -1277,7 +1352,7 @@ int launch_expand_k(hm_handle *h, const MulArgs<S> &ma, const A *s, const A *t, 
 template <typename S, typename A>
 int launch_pipeline(hm_handle *h, const MulArgs<S> &ma, cudaStream_t st, cudaStream_t side, cudaEvent_t fork,
                     cudaEvent_t join, void *scratch, bool timing, const void *panels = nullptr,
-                    cudaEvent_t mid = nullptr)
+                    cudaEvent_t mid = nullptr, int *part_count = nullptr)
 {
     if (!panels) panels = h->d_P;
     const int k = ma.k;
@@ -1286,6 +1361,14 @@ int launch_pipeline(hm_handle *h, const MulArgs<S> &ma, cudaStream_t st, cudaStr
     A *s = reinterpret_cast<A *>(static_cast<char *>(scratch) + L.s_off);
     const bool split = side != st;
     const bool tree = h->n_vp || h->n_m2l_rows;
+    // split basis panels where the call has arrival counters (not hm_mul_noalloc,
+    // whose scratch has no room for partial sums)
+    LeafParts<A> lp;
+    if (part_count && h->d_vparts) {
+        lp.rec = h->d_vparts;
+        lp.sums = reinterpret_cast<A *>(static_cast<char *>(scratch) + parts_off<A>(h, k));
+        lp.count = part_count;
+    }
     bool tree_chain = false;         // the tree passes ended with a kernel: the next launch may be dependent
     if (tree) {
         if (split) {
@@ -1293,7 +1376,8 @@ int launch_pipeline(hm_handle *h, const MulArgs<S> &ma, cudaStream_t st, cudaStr
             HM_CK(cudaStreamWaitEvent(side, fork, 0));
         }
         HM_TRY((launch_tree<S, A>(h, ma, split ? side : st, t, s, timing, split ? mid : nullptr,
-                                  cur_sched(h).overlap == 3 ? 1 : cur_sched(h).overlap == 4 ? 2 : 0, &tree_chain)));
+                                  cur_sched(h).overlap == 3 ? 1 : cur_sched(h).overlap == 4 ? 2 : 0, &tree_chain,
+                                  lp)));
         if (split && (k > kPartMaxK || !h->n_segs)) HM_CK(cudaEventRecord(join, side));
     }
     if (!h->n_segs) {
@@ -1348,7 +1432,7 @@ int run_mul(hm_handle *h, MulArgs<S> ma, cudaStream_t st, const void *panels = n
     HM_TRY(stream_ctx(h, st, stream_scratch_bytes<A>(h, ma.k), &sc));
     StageTimer whole(h, 4, st);
     return launch_pipeline<S, A>(h, ma, st, sched.overlap ? sc->side : st, sc->fork, sc->join, sc->p, true, panels,
-                                 sched.overlap >= 2 ? sc->mid : nullptr);
+                                 sched.overlap >= 2 ? sc->mid : nullptr, sc->count);
 }
 
 // Row-derivative panels (same layout as the panels), filled once.
@@ -2443,6 +2527,7 @@ void hm_free(hm_handle *h)
     if (h->trans) hm_free(h->trans);
     for (auto &kv : h->streams) {
         if (kv.second.p) cudaFree(kv.second.p);
+        if (kv.second.count) cudaFree(kv.second.count);
         if (kv.second.side) cudaStreamDestroy(kv.second.side);
         if (kv.second.fork) cudaEventDestroy(kv.second.fork);
         if (kv.second.join) cudaEventDestroy(kv.second.join);

@@ -170,16 +170,61 @@ __device__ __forceinline__ void ld_vec(const A *p, A *v)
     }
 }
 
+// Adds `n` consecutive partial slots of lane's column in order, eight loads in
+// flight, for one right-hand side.
+template <typename A>
+__device__ __forceinline__ A sum_parts(const A *sums, int64_t first, int n, int k, int q, int lane)
+{
+    A v = A(0);
+    const A *p = sums + (first * k + q) * 32 + lane;
+    const int64_t step = (int64_t)k * 32;
+    int i = 0;
+    for (; i + 8 <= n; i += 8) {
+        A u[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) u[j] = __ldcg(p + (i + j) * step);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v += u[j];
+    }
+    for (; i < n; ++i) v += __ldcg(p + i * step);
+    return v;
+}
+
+// True in every lane of the warp that arrives last of `n` at *count, which is
+// set back to zero for the next product; the others' writes are then visible.
+__device__ __forceinline__ bool last_arrival(int *count, int n, int lane)
+{
+    __threadfence();
+    __syncwarp();
+    int old = 0;
+    if (lane == 0) {
+        old = atomicAdd(count, 1);
+        if (old == n - 1) *count = 0;
+    }
+    old = __shfl_sync(0xffffffffu, old, 0);
+    __threadfence();
+    return old == n - 1;
+}
+
 // t[slot][col0 + m] = (V^T x)[m] for each explicit basis panel.  One warp
 // per panel, looping over chunks of QC right-hand sides; lane m owns column m
-// of the row-major panel (width <= 32, row stride ld).  Panels of up to cap
+// of the row-major panel (width <= 32, row stride ld).  With at most 16
+// columns 32 / width rows go at once, one per lane group, and the groups are
+// added at the end (an FP64 warp instruction takes 64 cycles of its pipe
+// whatever lanes are active).  Panels of more than 128 rows (the low-rank
+// factors of a user-assembled matrix) come as parts of at most 128 rows, one
+// warp each, whose sums the last warp of a group to finish adds in part order
+// (hm_vpart): one warp per 8,192-row panel took 1.30 ms of a 16,384-row FP64
+// HODLR product, latency of one serial FP64 chain with 508 of 608
+// sub-partitions idle.  Panels of up to cap
 // rows and wcap columns (the handle's largest, up to 128 rows) are staged
 // once in shared memory (cp.async) and the chunks' x values double-buffered
 // beside them; longer panels are read directly.  Plain FMA accumulation
 // (the coefficients feed only the far field).  Coefficients of a slot are r
 // apart per right-hand side.
 template <typename S, typename A, int QC>
-__global__ void leaf_up(MulArgs<S> ma, const hm_vpanel *vp, int npanels, const S *V, A *t, int r, int cap, int wcap)
+__global__ void leaf_up(MulArgs<S> ma, const hm_vpanel *vp, int npanels, const S *V, A *t, int r, int cap, int wcap,
+                        LeafParts<A> lp)
 {
     extern __shared__ unsigned char smem_raw[];
     pdl_trigger();
@@ -194,11 +239,16 @@ __global__ void leaf_up(MulArgs<S> ma, const hm_vpanel *vp, int npanels, const S
     // right-hand sides read from xin (and copied into x as they pass) or from x
     const S *xsrc = ma.xin ? ma.xin : ma.x;
     S *xcopy = ma.xin ? const_cast<S *>(ma.x) : nullptr;
+    hm_vpart part{};
+    if (lp.rec) part = lp.rec[w];
+    // a whole panel's sums are its coefficients, a part's go to its partial slot
+    A *out = part.nparts ? lp.sums + (int64_t)part.part * k * 32 : t + (int64_t)P.slot * k * r + P.col0;
+    const int ldo = part.nparts ? 32 : r;
     auto store = [&](int q0, int qc, PlainAcc<A> *acc) {
         if (lane < pw) {
 #pragma unroll
             for (int qq = 0; qq < QC; ++qq)
-                if (qq < qc) t[((int64_t)P.slot * k + q0 + qq) * r + P.col0 + lane] = acc[qq].value();
+                if (qq < qc) out[(int64_t)(q0 + qq) * ldo + lane] = acc[qq].value();
         }
     };
     if (P.nrows <= cap && P.ld == pw && pw <= wcap) {
@@ -247,13 +297,25 @@ __global__ void leaf_up(MulArgs<S> ma, const hm_vpanel *vp, int npanels, const S
 #pragma unroll
             for (int qq = 0; qq < QC; ++qq) acc[qq].zero();
             const A *xb = xs + b * cap * QC;
-            if (lane < pw) {
-                for (int j = 0; j < P.nrows; ++j) {
-                    const A v = (A)Vs[j * pw + lane];
-                    A xv[QC];
-                    ld_vec<QC>(xb + j * QC, xv);
+            auto row = [&](int j, int m) {
+                const A v = (A)Vs[j * pw + m];
+                A xv[QC];
+                ld_vec<QC>(xb + j * QC, xv);
 #pragma unroll
-                    for (int qq = 0; qq < QC; ++qq) acc[qq].add(v, xv[qq]);
+                for (int qq = 0; qq < QC; ++qq) acc[qq].add(v, xv[qq]);
+            };
+            if (pw > 16) {
+                if (lane < pw)
+                    for (int j = 0; j < P.nrows; ++j) row(j, lane);
+            } else {
+                const int groups = 32 / pw, jr = lane / pw, m = lane % pw;
+                if (jr < groups)
+                    for (int j = jr; j < P.nrows; j += groups) row(j, m);
+#pragma unroll
+                for (int qq = 0; qq < QC; ++qq) {         // add the row groups, in order
+                    A v = acc[qq].s;
+                    for (int g = 1; g < groups; ++g) v += __shfl_sync(0xffffffffu, acc[qq].s, (lane + g * pw) & 31);
+                    acc[qq].s = v;
                 }
             }
             store(q0, min(QC, k - q0), acc);
@@ -282,6 +344,20 @@ __global__ void leaf_up(MulArgs<S> ma, const hm_vpanel *vp, int npanels, const S
                     }
             store(q0, qc, acc);
         }
+    }
+    if (part.nparts && last_arrival(lp.count + part.group, part.nparts, lane)) {
+        A *tp = t + (int64_t)P.slot * k * r + P.col0 + lane;
+        A *gp = lp.sums + (int64_t)(part.gpart + part.group - part.group0) * k * 32 + lane;
+        if (lane < pw) {
+            for (int q = 0; q < k; ++q) {
+                const A v = sum_parts(lp.sums, part.part0, part.nparts, k, q, lane);
+                if (part.ngroups == 1) tp[(int64_t)q * r] = v;
+                else gp[(int64_t)q * 32] = v;
+            }
+        }
+        __syncwarp();
+        if (part.ngroups > 1 && last_arrival(lp.count + part.panel, part.ngroups, lane) && lane < pw)
+            for (int q = 0; q < k; ++q) tp[(int64_t)q * r] = sum_parts(lp.sums, part.gpart, part.ngroups, k, q, lane);
     }
 }
 
@@ -1507,8 +1583,8 @@ __global__ void expand_k(MulArgs<S> ma, const hm_seg *segs, const hm_piece *piec
 HM_INST_FAR(float, float, 4) HM_INST_FAR(float, float, 8) HM_INST_FAR(double, double, 4)
 HM_INST_FAR(double, double, 8)
 #define HM_INST_MV(S, A)                                                                             \
-    template __global__ void leaf_up<S, A, 1>(MulArgs<S>, const hm_vpanel *, int, const S *, A *, int, int, int); \
-    template __global__ void leaf_up<S, A, 8>(MulArgs<S>, const hm_vpanel *, int, const S *, A *, int, int, int); \
+    template __global__ void leaf_up<S, A, 1>(MulArgs<S>, const hm_vpanel *, int, const S *, A *, int, int, int, LeafParts<A>); \
+    template __global__ void leaf_up<S, A, 8>(MulArgs<S>, const hm_vpanel *, int, const S *, A *, int, int, int, LeafParts<A>); \
     template __global__ void m2l<S, A, 1>(const hm_m2l_row *, int, const hm_m2l_ent *, const S *, int,    \
                                           const A *, A *, int, int);                                    \
     template __global__ void m2l<S, A, 8>(const hm_m2l_row *, int, const hm_m2l_ent *, const S *, int,    \

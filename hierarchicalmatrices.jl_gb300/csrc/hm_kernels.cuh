@@ -164,8 +164,18 @@ __global__ void fill_segments(FillArgs fa, const hm_seg *segs, const hm_piece *p
 
 // ---------------------------------------------------------------- matvec
 
+// Tall basis panels split by rows: one hm_vpart per vp record (nullptr when no
+// panel is split), `sums` 32 values per (partial slot, right-hand side) and
+// `count` one zeroed arrival counter per group and panel (left zero again).
+template <typename A>
+struct LeafParts {
+    const hm_vpart *rec = nullptr;
+    A *sums = nullptr;
+    int *count = nullptr;
+};
 template <typename S, typename A, int QC>
-__global__ void leaf_up(MulArgs<S> ma, const hm_vpanel *vp, int npanels, const S *V, A *t, int r, int cap, int wcap);
+__global__ void leaf_up(MulArgs<S> ma, const hm_vpanel *vp, int npanels, const S *V, A *t, int r, int cap, int wcap,
+                        LeafParts<A> lp);
 
 // Shared memory of one leaf_up warp: a panel of cap x wcap values of S and two
 // x chunks of cap x QC values of A (16-byte multiples: cap is a multiple of 32).

@@ -29,6 +29,18 @@ struct hm_vpanel {      // explicit basis panel: coef[slot][col0 + m] = (P^T x[r
     int32_t pad;
 };
 
+// One row part of a tall basis panel (a hm_vpanel record of its own, with the
+// panel's slot and col0): its partial sums go to partial slot `part`, groups
+// of parts are added in order into partial slot `gpart`, and a panel's groups
+// in order into the coefficients; a panel of one group skips the second step.
+// nparts == 0 marks a panel that is not split.
+struct hm_vpart {
+    int32_t part, part0, nparts;    // this part; the first part and the parts of its group
+    int32_t group, group0, ngroups; // this group's index; the first group and the groups of its panel
+    int32_t gpart;                  // partial slot of group0's sums (the panel's groups are consecutive)
+    int32_t panel;                  // counter of the panel, after the group counters
+};
+
 struct hm_xfer {        // coefficient transfer between a node and its two children
     int32_t slot, c0, c1, pad;
 };
