@@ -1,6 +1,7 @@
 // CUDA kernels: batched compression (fill) and the hierarchical matvec.
 #include "hm_kernels.cuh"
 #include "hm_async.cuh"
+#include "hm_tree.cuh"
 
 #include <type_traits>
 
@@ -146,219 +147,20 @@ template __global__ void fill_segments<float, true>(FillArgs, const hm_seg *, co
 // expand_part<.., true> adds the far field U s.
 
 
-// N consecutive values from 16-byte aligned shared memory, as 16-byte loads
-// where N values fill them (the chunks of right-hand sides below are stored
-// right-hand side fastest, so that one step's N values are adjacent).
-template <int N, typename A>
-__device__ __forceinline__ void ld_vec(const A *p, A *v)
-{
-    if constexpr (sizeof(A) == 4 && N % 4 == 0) {
-#pragma unroll
-        for (int i = 0; i < N / 4; ++i) {
-            const float4 w = reinterpret_cast<const float4 *>(p)[i];
-            v[4 * i] = w.x; v[4 * i + 1] = w.y; v[4 * i + 2] = w.z; v[4 * i + 3] = w.w;
-        }
-    } else if constexpr (sizeof(A) == 8 && N % 2 == 0) {
-#pragma unroll
-        for (int i = 0; i < N / 2; ++i) {
-            const double2 w = reinterpret_cast<const double2 *>(p)[i];
-            v[2 * i] = w.x; v[2 * i + 1] = w.y;
-        }
-    } else {
-#pragma unroll
-        for (int i = 0; i < N; ++i) v[i] = p[i];
-    }
-}
-
-// Adds `n` consecutive partial slots of lane's column in order, eight loads in
-// flight, for one right-hand side.
-template <typename A>
-__device__ __forceinline__ A sum_parts(const A *sums, int64_t first, int n, int k, int q, int lane)
-{
-    A v = A(0);
-    const A *p = sums + (first * k + q) * 32 + lane;
-    const int64_t step = (int64_t)k * 32;
-    int i = 0;
-    for (; i + 8 <= n; i += 8) {
-        A u[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) u[j] = __ldcg(p + (i + j) * step);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) v += u[j];
-    }
-    for (; i < n; ++i) v += __ldcg(p + i * step);
-    return v;
-}
-
-// True in every lane of the warp that arrives last of `n` at *count, which is
-// set back to zero for the next product; the others' writes are then visible.
-__device__ __forceinline__ bool last_arrival(int *count, int n, int lane)
-{
-    __threadfence();
-    __syncwarp();
-    int old = 0;
-    if (lane == 0) {
-        old = atomicAdd(count, 1);
-        if (old == n - 1) *count = 0;
-    }
-    old = __shfl_sync(0xffffffffu, old, 0);
-    __threadfence();
-    return old == n - 1;
-}
-
-// t[slot][col0 + m] = (V^T x)[m] for each explicit basis panel.  One warp
-// per panel, looping over chunks of QC right-hand sides; lane m owns column m
-// of the row-major panel (width <= 32, row stride ld).  With at most 16
-// columns 32 / width rows go at once, one per lane group, and the groups are
-// added at the end (an FP64 warp instruction takes 64 cycles of its pipe
-// whatever lanes are active).  Panels of more than 128 rows (the low-rank
-// factors of a user-assembled matrix) come as parts of at most 128 rows, one
-// warp each, whose sums the last warp of a group to finish adds in part order
-// (hm_vpart): one warp per 8,192-row panel took 1.30 ms of a 16,384-row FP64
-// HODLR product, latency of one serial FP64 chain with 508 of 608
-// sub-partitions idle.  Panels of up to cap
-// rows and wcap columns (the handle's largest, up to 128 rows) are staged
-// once in shared memory (cp.async) and the chunks' x values double-buffered
-// beside them; longer panels are read directly.  Plain FMA accumulation
-// (the coefficients feed only the far field).  Coefficients of a slot are r
-// apart per right-hand side.
+// One warp per explicit basis panel (leaf_panel, hm_tree.cuh).
 template <typename S, typename A, int QC>
 __global__ void leaf_up(MulArgs<S> ma, const hm_vpanel *vp, int npanels, const S *V, A *t, int r, int cap, int wcap,
                         LeafParts<A> lp)
 {
     extern __shared__ unsigned char smem_raw[];
     pdl_trigger();
-    const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
     const int64_t w = (int64_t)blockIdx.x * (blockDim.x >> 5) + wib;
     if (w >= (int64_t)npanels) return;
-    const hm_vpanel P = vp[w];
-    const int pw = P.width;
-    const S *Vp = V + P.off;
-    const int k = ma.k;
-    // right-hand sides read from xin (and copied into x as they pass) or from x
-    const S *xsrc = ma.xin ? ma.xin : ma.x;
-    S *xcopy = ma.xin ? const_cast<S *>(ma.x) : nullptr;
     hm_vpart part{};
     if (lp.rec) part = lp.rec[w];
-    // a whole panel's sums are its coefficients, a part's go to its partial slot
-    A *out = part.nparts ? lp.sums + (int64_t)part.part * k * 32 : t + (int64_t)P.slot * k * r + P.col0;
-    const int ldo = part.nparts ? 32 : r;
-    auto store = [&](int q0, int qc, PlainAcc<A> *acc) {
-        if (lane < pw) {
-#pragma unroll
-            for (int qq = 0; qq < QC; ++qq)
-                if (qq < qc) out[(int64_t)(q0 + qq) * ldo + lane] = acc[qq].value();
-        }
-    };
-    if (P.nrows <= cap && P.ld == pw && pw <= wcap) {
-        // the panel once; x chunks of QC right-hand sides double-buffered,
-        // row major xs[b][j * QC + qq] (lanes walk rows)
-        S *Vs = reinterpret_cast<S *>(smem_raw + (size_t)wib * leaf_up_warp_bytes<S, A, QC>(cap, wcap));
-        A *xs = reinterpret_cast<A *>(Vs + cap * wcap);
-        const int nel = P.nrows * pw;
-        if (sizeof(S) * nel % 16 == 0 && (P.off * sizeof(S)) % 16 == 0) {
-            const char *src = reinterpret_cast<const char *>(Vp);
-            char *dst = reinterpret_cast<char *>(Vs);
-            for (int i = lane; i < (int)(nel * sizeof(S) / 16); i += 32) async_copy16(dst + 16 * i, src + 16 * i);
-        } else {
-            for (int i = lane; i < nel; i += 32) async_copy<sizeof(S)>(Vs + i, Vp + i);
-        }
-        auto fetch = [&](int q0, int b) {
-            const int qc = min(QC, k - q0);
-            A *d = xs + b * cap * QC;
-#pragma unroll
-            for (int qq = 0; qq < QC; ++qq)
-                for (int j = lane; j < P.nrows; j += 32) {
-                    const int64_t e = (P.row0 + j) * ma.incx + (int64_t)(q0 + qq) * ma.ldx;
-                    if (qq >= qc) {
-                        d[j * QC + qq] = A(0);
-                    } else if (xcopy) {
-                        // host-mapped source: plain loads, stored here and into x
-                        const S v = xsrc[e];
-                        d[j * QC + qq] = (A)v;
-                        xcopy[e] = v;
-                    } else {
-                        async_copy<sizeof(A)>(d + j * QC + qq, ma.x + e);
-                    }
-                }
-            async_commit();
-        };
-        fetch(0, 0);
-        for (int q0 = 0, b = 0; q0 < k; q0 += QC, b ^= 1) {
-            if (q0 + QC < k) {
-                fetch(q0 + QC, b ^ 1);
-                asm volatile("cp.async.wait_group 1;" ::: "memory");
-            } else {
-                async_wait_all();
-            }
-            __syncwarp();
-            PlainAcc<A> acc[QC];
-#pragma unroll
-            for (int qq = 0; qq < QC; ++qq) acc[qq].zero();
-            const A *xb = xs + b * cap * QC;
-            auto row = [&](int j, int m) {
-                const A v = (A)Vs[j * pw + m];
-                A xv[QC];
-                ld_vec<QC>(xb + j * QC, xv);
-#pragma unroll
-                for (int qq = 0; qq < QC; ++qq) acc[qq].add(v, xv[qq]);
-            };
-            if (pw > 16) {
-                if (lane < pw)
-                    for (int j = 0; j < P.nrows; ++j) row(j, lane);
-            } else {
-                const int groups = 32 / pw, jr = lane / pw, m = lane % pw;
-                if (jr < groups)
-                    for (int j = jr; j < P.nrows; j += groups) row(j, m);
-#pragma unroll
-                for (int qq = 0; qq < QC; ++qq) {         // add the row groups, in order
-                    A v = acc[qq].s;
-                    for (int g = 1; g < groups; ++g) v += __shfl_sync(0xffffffffu, acc[qq].s, (lane + g * pw) & 31);
-                    acc[qq].s = v;
-                }
-            }
-            store(q0, min(QC, k - q0), acc);
-            __syncwarp();                                 // buffer b is refilled next
-        }
-    } else {
-        for (int q0 = 0; q0 < k; q0 += QC) {
-            const int qc = min(QC, k - q0);
-            PlainAcc<A> acc[QC];
-#pragma unroll
-            for (int qq = 0; qq < QC; ++qq) acc[qq].zero();
-            if (lane < pw) {
-                const S *col = Vp + lane;
-                for (int j = 0; j < P.nrows; ++j) {
-                    const A v = (A)col[(int64_t)j * P.ld];
-#pragma unroll
-                    for (int qq = 0; qq < QC; ++qq)
-                        if (qq < qc) acc[qq].add(v, (A)xsrc[(P.row0 + j) * ma.incx + (int64_t)(q0 + qq) * ma.ldx]);
-                }
-            }
-            if (xcopy)
-                for (int qq = 0; qq < qc; ++qq)
-                    for (int j = lane; j < P.nrows; j += 32) {
-                        const int64_t e = (P.row0 + j) * ma.incx + (int64_t)(q0 + qq) * ma.ldx;
-                        xcopy[e] = xsrc[e];
-                    }
-            store(q0, qc, acc);
-        }
-    }
-    if (part.nparts && last_arrival(lp.count + part.group, part.nparts, lane)) {
-        A *tp = t + (int64_t)P.slot * k * r + P.col0 + lane;
-        A *gp = lp.sums + (int64_t)(part.gpart + part.group - part.group0) * k * 32 + lane;
-        if (lane < pw) {
-            for (int q = 0; q < k; ++q) {
-                const A v = sum_parts(lp.sums, part.part0, part.nparts, k, q, lane);
-                if (part.ngroups == 1) tp[(int64_t)q * r] = v;
-                else gp[(int64_t)q * 32] = v;
-            }
-        }
-        __syncwarp();
-        if (part.ngroups > 1 && last_arrival(lp.count + part.panel, part.ngroups, lane) && lane < pw)
-            for (int q = 0; q < k; ++q) tp[(int64_t)q * r] = sum_parts(lp.sums, part.gpart, part.ngroups, k, q, lane);
-    }
+    leaf_panel<S, A, QC>(ma, vp[w], part, V, t, r, cap, wcap,
+                         smem_raw + (size_t)wib * leaf_up_warp_bytes<S, A, QC>(cap, wcap), lp);
 }
 
 // Upward transfers of one band: t[parent][m] = sum_c sum_m' T_c[m', m] t[child_c][m'].
@@ -410,16 +212,8 @@ __global__ void xfer_up_band(const hm_task *tasks, const hm_step *steps, const h
     }
 }
 
-// Band tasks with shared-memory-resident coefficients, one CTA per (task,
-// chunk of QC right-hand sides: blockIdx.y): the task's
-// external inputs (and T) are fetched once with cp.async, every level then
-// reads and writes shared memory only, with a CTA barrier between levels;
-// each coefficient the task produces is also written to global memory.
-// Task-local numbering (records' pad, set by the planner): upward, record i
-// produces local i and reads locals pad & 0xffff, pad >> 16; downward,
-// record i's children are locals 2i, 2i + 1 and its parent is local pad.
-// Upward, L holds r x QC values per local, right-hand side fastest
-// (L[local][m][qq]); downward QC x r (L[local][qq][m]).
+// Band tasks, one CTA per (task, chunk of QC right-hand sides: blockIdx.y)
+// (xfer_up_fetch / xfer_up_levels and the downward pair, hm_tree.cuh).
 template <typename A, int QC>
 __global__ void xfer_up_task(const hm_task *tasks, const hm_step *steps, const hm_xfer *ents, const A *T, A *t,
                              int r, int k, int early)
@@ -428,210 +222,53 @@ __global__ void xfer_up_task(const hm_task *tasks, const hm_step *steps, const h
     A *Ts = reinterpret_cast<A *>(smem_raw);
     A *L = Ts + 2 * HM_RMAX * HM_RMAX;
     const hm_task tk = tasks[blockIdx.x];
-    const int e0 = steps[tk.step0].e0, e1 = steps[tk.step1 - 1].e1, nrec = e1 - e0;
-    const int q0 = blockIdx.y * QC, qc = min(QC, k - q0);      // this CTA's right-hand sides
+    const int q0 = blockIdx.y * QC;                            // this CTA's right-hand sides
     if (early) pdl_trigger();     // the next band may be scheduled now (a small grid; not before a large one)
     for (int i = threadIdx.x; i < 2 * r * r; i += blockDim.x) async_copy<sizeof(A)>(Ts + i, T + i);
     pdl_wait();                                                // the children's coefficients are ready
-    // external children: warps take records, lanes coefficients
-    for (int rec = threadIdx.x >> 5; rec < nrec; rec += blockDim.x >> 5) {
-        const hm_xfer X = ents[e0 + rec];
-        const int ln = threadIdx.x & 31;
-#pragma unroll
-        for (int c = 0; c < 2; ++c) {
-            const int lc = c ? (X.pad >> 16) : (X.pad & 0xffff);
-            if (lc < nrec || ln >= r) continue;           // produced by an earlier level of this task
-            const A *src = t + ((int64_t)(c ? X.c1 : X.c0) * k + q0) * r + ln;
-            A *d = L + (int64_t)lc * QC * r + ln * QC;
-#pragma unroll
-            for (int qq = 0; qq < QC; ++qq) {
-                if (qq < qc) async_copy<sizeof(A)>(d + qq, src + (int64_t)qq * r);
-                else d[qq] = A(0);
-            }
-        }
-    }
+    xfer_up_fetch<A, QC>(tk, steps, ents, t, L, r, k, q0);
     async_wait_all();
     __syncthreads();
-    const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    for (int st = tk.step0; st < tk.step1; ++st) {
-        const hm_step S = steps[st];
-        for (int w = threadIdx.x >> 5; w < S.e1 - S.e0; w += nw) {
-            const int e = S.e0 + w;
-            const hm_xfer X = ents[e];
-            const A *c0 = L + (int64_t)(X.pad & 0xffff) * QC * r;
-            const A *c1 = L + (int64_t)(X.pad >> 16) * QC * r;
-            A *out = L + (int64_t)(e - e0) * QC * r;
-            if (lane < r) {
-                A acc[QC];
-#pragma unroll
-                for (int qq = 0; qq < QC; ++qq) acc[qq] = 0;
-                for (int mp = 0; mp < r; ++mp) {
-                    const A a0 = Ts[mp * r + lane], a1 = Ts[r * r + mp * r + lane];
-                    A v0[QC], v1[QC];
-                    ld_vec<QC>(c0 + mp * QC, v0);
-                    ld_vec<QC>(c1 + mp * QC, v1);
-#pragma unroll
-                    for (int qq = 0; qq < QC; ++qq) acc[qq] += a0 * v0[qq] + a1 * v1[qq];
-                }
-#pragma unroll
-                for (int qq = 0; qq < QC; ++qq) {
-                    out[lane * QC + qq] = acc[qq];
-                    if (qq < qc) t[((int64_t)X.slot * k + q0 + qq) * r + lane] = acc[qq];
-                }
-            }
-        }
-        __syncthreads();
-    }
+    if (r == 20) xfer_up_levels<A, QC, 20>(tk, steps, ents, Ts, t, L, r, k, q0);
+    else xfer_up_levels<A, QC, 0>(tk, steps, ents, Ts, t, L, r, k, q0);
 }
 
 template <typename A, int QC>
 __global__ void xfer_down_task(const hm_task *tasks, const hm_step *steps, const hm_xfer *ents, const A *T, A *s,
-                               int r, int k, int early)
+                             int r, int k, int early)
 {
     extern __shared__ unsigned char smem_raw[];
     A *Ts = reinterpret_cast<A *>(smem_raw);
     A *L = Ts + 2 * HM_RMAX * HM_RMAX;
     const hm_task tk = tasks[blockIdx.x];
-    const int e0 = steps[tk.step0].e0, e1 = steps[tk.step1 - 1].e1, nrec = e1 - e0;
-    const int q0 = blockIdx.y * QC, qc = min(QC, k - q0);      // this CTA's right-hand sides
+    const int q0 = blockIdx.y * QC;                            // this CTA's right-hand sides
     if (early) pdl_trigger();
     for (int i = threadIdx.x; i < 2 * r * r; i += blockDim.x) async_copy<sizeof(A)>(Ts + i, T + i);
     pdl_wait();                                                // far-field and parent coefficients are ready
-    // children start from their far-field (m2l) coefficients; external parents as computed
-    // warps take records, lanes coefficients
-    for (int rec = threadIdx.x >> 5; rec < nrec; rec += blockDim.x >> 5) {
-        const hm_xfer X = ents[e0 + rec];
-        const int ln = threadIdx.x & 31;
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            int lc, slot;
-            if (c < 2) {
-                lc = 2 * rec + c;
-                slot = c ? X.c1 : X.c0;
-            } else {
-                lc = X.pad;
-                slot = X.slot;
-                if (lc < 2 * nrec) continue;              // a child of an earlier level of this task
-            }
-            if (ln >= r) continue;
-            const A *src = s + ((int64_t)slot * k + q0) * r + ln;
-            A *d = L + (int64_t)lc * QC * r + ln;
-#pragma unroll
-            for (int qq = 0; qq < QC; ++qq) {
-                if (qq < qc) async_copy<sizeof(A)>(d + qq * r, src + (int64_t)qq * r);
-                else d[qq * r] = A(0);
-            }
-        }
-    }
+    xfer_down_fetch<A, QC>(tk, steps, ents, s, L, r, k, q0);
     async_wait_all();
     __syncthreads();
-    const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    for (int st = tk.step0; st < tk.step1; ++st) {
-        const hm_step S = steps[st];
-        for (int w = threadIdx.x >> 5; w < S.e1 - S.e0; w += nw) {
-            const int e = S.e0 + w;
-            const hm_xfer X = ents[e];
-            const A *p = L + (int64_t)X.pad * QC * r;
-            A *o0 = L + (int64_t)(2 * (e - e0)) * QC * r;
-            A *o1 = o0 + QC * r;
-            if (lane < r) {
-                A a0[QC], a1[QC];
-#pragma unroll
-                for (int qq = 0; qq < QC; ++qq) { a0[qq] = 0; a1[qq] = 0; }
-                for (int m = 0; m < r; ++m) {
-                    const A t0 = Ts[lane * r + m], t1 = Ts[r * r + lane * r + m];
-#pragma unroll
-                    for (int qq = 0; qq < QC; ++qq) {
-                        const A v = p[qq * r + m];
-                        a0[qq] += t0 * v;
-                        a1[qq] += t1 * v;
-                    }
-                }
-#pragma unroll
-                for (int qq = 0; qq < QC; ++qq) {
-                    const A v0 = o0[qq * r + lane] + a0[qq], v1 = o1[qq * r + lane] + a1[qq];
-                    o0[qq * r + lane] = v0;
-                    o1[qq * r + lane] = v1;
-                    if (qq < qc) {
-                        s[((int64_t)X.c0 * k + q0 + qq) * r + lane] = v0;
-                        s[((int64_t)X.c1 * k + q0 + qq) * r + lane] = v1;
-                    }
-                }
-            }
-        }
-        __syncthreads();
-    }
+    if (r == 20) xfer_down_levels<A, QC, 20>(tk, steps, ents, Ts, s, L, r, k, q0);
+    else xfer_down_levels<A, QC, 0>(tk, steps, ents, Ts, s, L, r, k, q0);
 }
 
-// Far field: s[slot][m] = sum_e sum_n F_e[m + r n] t[yslot_e][n]
-// (the F stage of src/algebra.jl:258-265, grouped by row cluster).  One warp
-// per (row slot, chunk of up to QC right-hand sides).  The r x r blocks of the
-// row and the column coefficients they multiply are double-buffered in
-// shared memory with cp.async: block e + 1 is in flight while block e is
-// used for every right-hand side of the chunk.  Lane m accumulates row m.
+// One warp per (row slot, chunk of up to QC right-hand sides) (m2l_row, hm_tree.cuh).
 template <typename S, typename A, int QC>
 __global__ void m2l(const hm_m2l_row *rows, int nrows, const hm_m2l_ent *ents, const S *F, int fstride,
                     const A *t, A *s, int r, int k)
 {
     extern __shared__ unsigned char smem_raw[];
-    // per warp: two F blocks (fstride values of S) and two column-coefficient chunks (QC * HM_RMAX of A)
     const int wib = threadIdx.x >> 5;
-    const size_t wbytes = 2 * (size_t)fstride * sizeof(S) + 2 * (size_t)QC * HM_RMAX * sizeof(A);
-    S *Fb = reinterpret_cast<S *>(smem_raw + wib * wbytes);
-    A *Tb = reinterpret_cast<A *>(Fb + 2 * fstride);
-    const int lane = threadIdx.x & 31;
     const int nq = (k + QC - 1) / QC;
     const int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     pdl_trigger();
     pdl_wait();                                                // the upward pass's coefficients are ready
     if (w >= (int64_t)nrows * nq) return;
+    unsigned char *smem = smem_raw + wib * m2l_warp_bytes<S, A, QC>(fstride);
     const hm_m2l_row R = rows[w / nq];
-    const int q0 = (int)(w % nq) * QC, qc = min(QC, k - q0);
-    auto fetch = [&](int e, int buf) {
-        const hm_m2l_ent E = ents[e];
-        const char *src = reinterpret_cast<const char *>(F + E.foff);
-        char *dst = reinterpret_cast<char *>(Fb + buf * fstride);
-        for (int i = lane; i < (int)(fstride * sizeof(S) / 16); i += 32) async_copy16(dst + 16 * i, src + 16 * i);
-        A *tb = Tb + buf * QC * HM_RMAX;
-        if (lane < r) {
-            const A *src = t + ((int64_t)E.yslot * k + q0) * r + lane;
-#pragma unroll
-            for (int qq = 0; qq < QC; ++qq) {
-                if (qq < qc) async_copy<sizeof(A)>(tb + qq * HM_RMAX + lane, src + (int64_t)qq * r);
-                else tb[qq * HM_RMAX + lane] = A(0);
-            }
-        }
-        async_commit();
-    };
-    A acc[QC];
-#pragma unroll
-    for (int qq = 0; qq < QC; ++qq) acc[qq] = 0;
-    if (R.begin < R.end) fetch(R.begin, 0);
-    for (int e = R.begin; e < R.end; ++e) {
-        const int buf = (e - R.begin) & 1;
-        if (e + 1 < R.end) {
-            fetch(e + 1, buf ^ 1);
-            asm volatile("cp.async.wait_group 1;" ::: "memory");
-        } else {
-            async_wait_all();
-        }
-        __syncwarp();
-        const S *fb = Fb + buf * fstride;
-        const A *tb = Tb + buf * QC * HM_RMAX;
-        if (lane < r) {
-            for (int n = 0; n < r; ++n) {
-                const A f = (A)fb[lane + r * n];
-#pragma unroll
-                for (int qq = 0; qq < QC; ++qq) acc[qq] += f * tb[qq * HM_RMAX + n];
-            }
-        }
-        __syncwarp();                         // buffer buf is refilled by the next fetch
-    }
-    if (lane < r) {
-#pragma unroll
-        for (int qq = 0; qq < QC; ++qq)
-            if (qq < qc) s[((int64_t)R.slot * k + q0 + qq) * r + lane] = acc[qq];
-    }
+    const int q0 = (int)(w % nq) * QC;
+    if (r == 20) m2l_row<S, A, QC, 20>(R, q0, ents, F, fstride, t, s, r, k, smem);
+    else m2l_row<S, A, QC, 0>(R, q0, ents, F, fstride, t, s, r, k, smem);
 }
 
 // Far field for many right-hand sides (k > QC): one CTA (4 warps) per row
@@ -776,52 +413,6 @@ __global__ void xfer_down_band(const hm_task *tasks, const hm_step *steps, const
 // are staged per warp in shared memory (g[c * KB + q]).  KB = 1 accumulates
 // with compensated (TwoProd/TwoSum) sums, KB > 1 with FMA per piece folded
 // in with TwoSum.
-template <typename A, int KB>
-struct SegAcc;
-template <typename A>
-struct SegAcc<A, 1> {
-    Acc<A> a;
-    __device__ __forceinline__ void zero() { a.zero(); }
-    __device__ __forceinline__ void add(A p, const A *g) { a.add(p, g[0]); }
-    __device__ __forceinline__ void fold() {}
-    __device__ __forceinline__ A hi(int) const { return a.s_hi(); }
-    __device__ __forceinline__ A lo(int) const { return a.s_lo(); }
-    __device__ __forceinline__ A merged(int, A so, A co) const { return a.merged(so, co); }
-};
-template <typename A, int KB>
-struct SegAcc {
-    A part[KB], h[KB], l[KB];
-    __device__ __forceinline__ void zero()
-    {
-#pragma unroll
-        for (int q = 0; q < KB; ++q) { part[q] = 0; h[q] = 0; l[q] = 0; }
-    }
-    __device__ __forceinline__ void add(A p, const A *g)
-    {
-#pragma unroll
-        for (int q = 0; q < KB; ++q) part[q] = fma(p, g[q], part[q]);
-    }
-    __device__ __forceinline__ void fold()   // end of a piece: compensated fold of the partial sums
-    {
-#pragma unroll
-        for (int q = 0; q < KB; ++q) {
-            const A t = h[q] + part[q];
-            const A bp = t - h[q];
-            l[q] += (h[q] - (t - bp)) + (part[q] - bp);
-            h[q] = t;
-            part[q] = 0;
-        }
-    }
-    __device__ __forceinline__ A hi(int q) const { return h[q]; }
-    __device__ __forceinline__ A lo(int q) const { return l[q]; }
-    __device__ __forceinline__ A merged(int q, A so, A co) const
-    {
-        const A t = h[q] + so;
-        const A bp = t - h[q];
-        return t + (((h[q] - (t - bp)) + (so - bp)) + (l[q] + co));
-    }
-};
-
 // Near field (FAR = false: y (+)= D x) or far field (FAR = true: U s) of one
 // row segment per warp.  The far field goes to yfar (leading dimension ldf)
 // when given, else it is added into y.

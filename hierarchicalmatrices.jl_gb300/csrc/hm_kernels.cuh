@@ -195,6 +195,12 @@ template <typename A, int QC>
 __global__ void xfer_up_band(const hm_task *tasks, const hm_step *steps, const hm_xfer *ents, const A *T, A *t,
                              int r, int k);
 
+// Shared memory of one m2l warp: two F blocks and two chunks of column coefficients.
+template <typename S, typename A, int QC>
+__host__ __device__ constexpr size_t m2l_warp_bytes(int fstride)
+{
+    return 2 * (size_t)fstride * sizeof(S) + 2 * (size_t)QC * HM_RMAX * sizeof(A);
+}
 template <typename S, typename A, int QC>
 __global__ void m2l(const hm_m2l_row *rows, int nrows, const hm_m2l_ent *ents, const S *F, int fstride,
                     const A *t, A *s, int r, int k);
