@@ -287,7 +287,9 @@ struct hm_handle {
     struct StreamCtx {
         void *p = nullptr;
         size_t bytes = 0;
-        int *count = nullptr;       // leaf_up's arrival counters (n_part_counts zeros between products)
+        // before the scratch in the same allocation, zero between products:
+        // leaf_up's n_part_counts arrival counters
+        int *sync = nullptr;
         cudaStream_t side = nullptr;
         cudaEvent_t fork = nullptr, join = nullptr;
         cudaEvent_t mid = nullptr;  // a point inside the tree passes where the near field may start
@@ -810,17 +812,16 @@ int stream_ctx(hm_handle *h, cudaStream_t st, size_t bytes, hm_handle::StreamCtx
         HM_CK(cudaEventCreateWithFlags(&sc.join, cudaEventDisableTiming));
         HM_CK(cudaEventCreateWithFlags(&sc.mid, cudaEventDisableTiming));
     }
-    if (sc.bytes < bytes) {
-        if (sc.p) HM_CK(cudaFreeAsync(sc.p, st));
-        sc.p = nullptr; sc.bytes = 0;
-        HM_CK(device_malloc_async(&sc.p, bytes, st));
+    if (sc.bytes < bytes || !sc.sync) {
+        if (sc.sync) HM_CK(cudaFreeAsync(sc.sync, st));
+        sc.p = nullptr; sc.sync = nullptr; sc.bytes = 0;
+        const size_t head = align256(std::max<size_t>(1, (size_t)h->n_part_counts) * sizeof(int));
+        void *q = nullptr;
+        HM_CK(device_malloc_async(&q, head + bytes, st));
+        sc.sync = static_cast<int *>(q);
+        HM_CK(cudaMemsetAsync(q, 0, head, st));
+        sc.p = static_cast<char *>(q) + head;
         sc.bytes = bytes;
-    }
-    if (h->n_part_counts && !sc.count) {
-        void *c = nullptr;
-        HM_CK(device_malloc_async(&c, (size_t)h->n_part_counts * sizeof(int), st));
-        HM_CK(cudaMemsetAsync(c, 0, (size_t)h->n_part_counts * sizeof(int), st));
-        sc.count = static_cast<int *>(c);
     }
     *out = &sc;
     return HM_OK;
@@ -975,7 +976,7 @@ int launch_tree_qc(hm_handle *h, const MulArgs<S> &ma, cudaStream_t st, A *t, A 
                 done = true;
             }
         }
-        if constexpr (QC > 1) {
+        if constexpr (QC == 8) {
             if (!done && h->n_m2l_rows && nq > 1) {
                 // many right-hand sides: one CTA per row box, its blocks staged once
                 const size_t smem = 8 * (size_t)h->fstride * sizeof(S) +
@@ -1154,6 +1155,13 @@ int launch_tree_wide(hm_handle *h, const MulArgs<S> &ma, cudaStream_t st, A *t, 
     return HM_OK;
 }
 
+// Right-hand sides a chunk of the tree kernels holds for k of them.  A chunk
+// computes all its places whatever k: with two FP64 right-hand sides in chunks
+// of 8 the tree passes issued four times the FMAs they needed on the FP64 pipe
+// (n = 65,536: 451 -> 215 us per product; four right-hand sides at n = 262,144
+// 1,402 -> 1,037 us; FP32 with two 127 -> 97 us).
+inline int tree_chunk(int k) { return k == 1 ? 1 : k == 2 ? 2 : k <= 4 ? 4 : 8; }
+
 template <typename S, typename A>
 int launch_tree(hm_handle *h, const MulArgs<S> &ma, cudaStream_t st, A *t, A *s, bool timing, cudaEvent_t mid,
                 int mid_after, bool *ends_with_kernel, const LeafParts<A> &lp)
@@ -1170,7 +1178,10 @@ int launch_tree(hm_handle *h, const MulArgs<S> &ma, cudaStream_t st, A *t, A *s,
             return rc;
         }
     }
-    rc = ma.k == 1 ? launch_tree_qc<S, A, 1>(h, ma, st, t, s, timing, mid, mid_after, &ends, lp)
+    const int qc = tree_chunk(ma.k);
+    rc = qc == 1   ? launch_tree_qc<S, A, 1>(h, ma, st, t, s, timing, mid, mid_after, &ends, lp)
+         : qc == 2 ? launch_tree_qc<S, A, 2>(h, ma, st, t, s, timing, mid, mid_after, &ends, lp)
+         : qc == 4 ? launch_tree_qc<S, A, 4>(h, ma, st, t, s, timing, mid, mid_after, &ends, lp)
                    : launch_tree_qc<S, A, 8>(h, ma, st, t, s, timing, mid, mid_after, &ends, lp);
     if (ends_with_kernel) *ends_with_kernel = ends;
     return rc;
@@ -1432,7 +1443,7 @@ int run_mul(hm_handle *h, MulArgs<S> ma, cudaStream_t st, const void *panels = n
     HM_TRY(stream_ctx(h, st, stream_scratch_bytes<A>(h, ma.k), &sc));
     StageTimer whole(h, 4, st);
     return launch_pipeline<S, A>(h, ma, st, sched.overlap ? sc->side : st, sc->fork, sc->join, sc->p, true, panels,
-                                 sched.overlap >= 2 ? sc->mid : nullptr, sc->count);
+                                 sched.overlap >= 2 ? sc->mid : nullptr, sc->sync);
 }
 
 // Row-derivative panels (same layout as the panels), filled once.
@@ -2526,8 +2537,7 @@ void hm_free(hm_handle *h)
     cudaDeviceSynchronize();
     if (h->trans) hm_free(h->trans);
     for (auto &kv : h->streams) {
-        if (kv.second.p) cudaFree(kv.second.p);
-        if (kv.second.count) cudaFree(kv.second.count);
+        if (kv.second.sync) cudaFree(kv.second.sync);
         if (kv.second.side) cudaStreamDestroy(kv.second.side);
         if (kv.second.fork) cudaEventDestroy(kv.second.fork);
         if (kv.second.join) cudaEventDestroy(kv.second.join);

@@ -22,33 +22,9 @@
 // memory.
 #include "hm_kernels.cuh"
 #include "hm_async.cuh"
+#include "hm_df.cuh"
 
 namespace hm {
-
-namespace {
-
-__device__ __forceinline__ float2 df_split(double v)
-{
-    const float h = __double2float_rn(v);
-    return make_float2(h, __double2float_rn(__dsub_rn(v, (double)h)));
-}
-
-// (sh, sl) += (ph + pl) (gh + gl)
-__device__ __forceinline__ void df_fma(float &sh, float &sl, float ph, float pl, float gh, float gl)
-{
-    const float h = __fmul_rn(ph, gh);
-    float e = __fmaf_rn(ph, gh, -h);
-    e = __fmaf_rn(ph, gl, e);
-    e = __fmaf_rn(pl, gh, e);
-    const float s = __fadd_rn(sh, h);
-    const float bp = __fsub_rn(s, sh);
-    float t = __fadd_rn(__fsub_rn(sh, __fsub_rn(s, bp)), __fsub_rn(h, bp));
-    t = __fadd_rn(t, __fadd_rn(sl, e));
-    sh = __fadd_rn(s, t);
-    sl = __fsub_rn(t, __fsub_rn(sh, s));
-}
-
-}  // namespace
 
 // In place: every FP64 value of P becomes its (h, l) pair; *bad is set when a
 // value's magnitude is at or above 2^127, where the pair would overflow.
@@ -165,47 +141,10 @@ __global__ void leaf_up_df(MulArgs<double> ma, const hm_vpanel *vp, int npanels,
 {
     extern __shared__ float2 leaf_df_smem[];
     pdl_trigger();
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    const int wib = threadIdx.x >> 5;
     const int64_t w = (int64_t)blockIdx.x * (blockDim.x >> 5) + wib;
     if (w >= (int64_t)npanels) return;
-    const hm_vpanel P = vp[w];
-    float2 *xs = leaf_df_smem + (size_t)wib * cap;
-    const float2 *Vp = V + P.off;
-    const double *xsrc = ma.xin ? ma.xin : ma.x;
-    double *xcopy = ma.xin ? const_cast<double *>(ma.x) : nullptr;
-    const int nr = min((int)P.nrows, cap);
-    for (int q = 0; q < ma.k; ++q) {
-        for (int j = lane; j < P.nrows; j += 32) {
-            const int64_t e = (P.row0 + j) * ma.incx + (int64_t)q * ma.ldx;
-            const double v = xsrc[e];
-            if (xcopy) xcopy[e] = v;
-            if (j < nr) xs[j] = df_split(v);
-        }
-        __syncwarp();
-        if (lane < P.width) {
-            float sh = 0.f, sl = 0.f;
-            int j = 0;
-            for (; j + 8 <= nr; j += 8) {
-                float2 v[8];
-#pragma unroll
-                for (int u = 0; u < 8; ++u) v[u] = Vp[(int64_t)(j + u) * P.ld + lane];
-#pragma unroll
-                for (int u = 0; u < 8; ++u) df_fma(sh, sl, v[u].x, v[u].y, xs[j + u].x, xs[j + u].y);
-            }
-            for (; j < nr; ++j) {
-                const float2 v = Vp[(int64_t)j * P.ld + lane];
-                df_fma(sh, sl, v.x, v.y, xs[j].x, xs[j].y);
-            }
-            // rows past the staged ones (panels longer than cap) straight from x
-            for (j = nr; j < P.nrows; ++j) {
-                const float2 v = Vp[(int64_t)j * P.ld + lane];
-                const float2 xv = df_split(xsrc[(P.row0 + j) * ma.incx + (int64_t)q * ma.ldx]);
-                df_fma(sh, sl, v.x, v.y, xv.x, xv.y);
-            }
-            t[((int64_t)P.slot * ma.k + q) * r + P.col0 + lane] = __dadd_rn((double)sh, (double)sl);
-        }
-        __syncwarp();
-    }
+    leaf_panel_df(ma, vp[w], V, t, r, cap, leaf_df_smem + (size_t)wib * cap);
 }
 
 // Far-field blocks with HM_DF64 storage (F as (h, l) pairs, r x r column-major
@@ -265,59 +204,13 @@ __global__ void __launch_bounds__(kM2lDfWarps * 32)
 {
     extern __shared__ __align__(16) unsigned char m2l_smem[];
     __shared__ float2 tsh[kM2lDfWarps][32];
-    constexpr int R20 = 20, BLK = R20 * R20;
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    constexpr int BLK = 20 * 20;
+    const int wib = threadIdx.x >> 5;
     const int64_t w = (int64_t)blockIdx.x * kM2lDfWarps + wib;
     pdl_trigger();
     pdl_wait();                                                // the upward pass's coefficients are ready
     if (w >= (int64_t)nrows) return;
-    float2 *ring = reinterpret_cast<float2 *>(m2l_smem) + (size_t)wib * NS * BLK;
-    float2 *ts = tsh[wib];
-    const hm_m2l_row R = rows[w];
-    const int ne = R.end - R.begin;
-    auto issue = [&](int i, int stage) {
-        const hm_m2l_ent E = ents[R.begin + i];
-        float2 *dst = ring + stage * BLK;
-        const float2 *src = F + E.foff;
-        if ((E.foff & 1) == 0) {
-            for (int c = lane; c < BLK / 2; c += 32) async_copy16(dst + 2 * c, src + 2 * c);
-        } else {
-            for (int c = lane; c < BLK; c += 32) async_copy<8>(dst + c, src + c);
-        }
-    };
-    for (int q = 0; q < k; ++q) {
-        float sh = 0.f, sl = 0.f;
-        double tc = 0.0;
-        if (ne > 0 && lane < R20) tc = t[((int64_t)ents[R.begin].yslot * k + q) * R20 + lane];
-#pragma unroll
-        for (int i = 0; i < NS - 1; ++i) {
-            if (i < ne) issue(i, i);
-            async_commit();
-        }
-        for (int e = 0; e < ne; ++e) {
-            const int ei = e + NS - 1;
-            if (ei < ne) issue(ei, ei % NS);
-            async_commit();
-            asm volatile("cp.async.wait_group %0;" ::"n"(NS - 1) : "memory");
-            if (lane < R20) ts[lane] = df_split(tc);
-            __syncwarp();                                      // block e and the coefficients visible
-            double tn = 0.0;
-            if (e + 1 < ne && lane < R20) tn = t[((int64_t)ents[R.begin + e + 1].yslot * k + q) * R20 + lane];
-            if (lane < R20) {
-                const float2 *f = ring + (e % NS) * BLK + lane;
-#pragma unroll
-                for (int n = 0; n < R20; ++n) {
-                    const float2 v = f[R20 * n];
-                    df_fma(sh, sl, v.x, v.y, ts[n].x, ts[n].y);
-                }
-            }
-            __syncwarp();                                      // the stage and ts are free again
-            tc = tn;
-        }
-        async_wait_all();
-        __syncwarp();
-        if (lane < R20) s[((int64_t)R.slot * k + q) * R20 + lane] = __dadd_rn((double)sh, (double)sl);
-    }
+    m2l_row_df<NS>(rows[w], ents, F, t, s, k, reinterpret_cast<float2 *>(m2l_smem) + (size_t)wib * NS * BLK, tsh[wib]);
 }
 template __global__ void m2l_df_ring<kM2lDfStages>(const hm_m2l_row *, int, const hm_m2l_ent *, const float2 *,
                                                    const double *, double *, int);
@@ -376,70 +269,19 @@ __global__ void xfer_df(const hm_task *tasks, const hm_step *steps, const hm_xfe
                         double *coef, int r, int k, int early)
 {
     extern __shared__ float2 xfer_df_smem[];
+    __shared__ TaskRecs recs;
     float2 *Ts = xfer_df_smem;                                 // 2 r r pairs
     float2 *L = Ts + 2 * HM_RMAX * HM_RMAX;                    // r pairs per local
-    const hm_task tk = tasks[blockIdx.x];
-    const int e0 = steps[tk.step0].e0, e1 = steps[tk.step1 - 1].e1, nrec = e1 - e0;
     const int q = blockIdx.y;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     if (early) pdl_trigger();
     for (int i = threadIdx.x; i < 2 * r * r; i += blockDim.x) Ts[i] = T[i];
-    pdl_wait();                                                // inputs of the band are ready
-    for (int rec = warp; rec < nrec; rec += nw) {
-        const hm_xfer X = ents[e0 + rec];
-        if (lane >= r) continue;
-#pragma unroll
-        for (int c = 0; c < (UP ? 2 : 3); ++c) {
-            int lc, slot;
-            if (UP) {
-                lc = c ? (X.pad >> 16) : (X.pad & 0xffff);
-                slot = c ? X.c1 : X.c0;
-                if (lc < nrec) continue;                       // produced by an earlier level of this task
-            } else if (c < 2) {
-                lc = 2 * rec + c;                              // children start from their far-field values
-                slot = c ? X.c1 : X.c0;
-            } else {
-                lc = X.pad;
-                slot = X.slot;
-                if (lc < 2 * nrec) continue;                   // a child of an earlier level of this task
-            }
-            L[lc * r + lane] = df_split(coef[((int64_t)slot * k + q) * r + lane]);
-        }
-    }
+    load_task(tasks + blockIdx.x, steps, ents, recs);
     __syncthreads();
-    for (int st = tk.step0; st < tk.step1; ++st) {
-        const hm_step S = steps[st];
-        for (int w = warp; w < S.e1 - S.e0; w += nw) {
-            const int e = S.e0 + w;
-            const hm_xfer X = ents[e];
-            if (lane >= r) continue;
-            if (UP) {
-                const float2 *c0 = L + (X.pad & 0xffff) * r, *c1 = L + (X.pad >> 16) * r;
-                float sh = 0.f, sl = 0.f;
-                for (int mp = 0; mp < r; ++mp) {
-                    const float2 a0 = Ts[mp * r + lane], a1 = Ts[r * r + mp * r + lane];
-                    df_fma(sh, sl, a0.x, a0.y, c0[mp].x, c0[mp].y);
-                    df_fma(sh, sl, a1.x, a1.y, c1[mp].x, c1[mp].y);
-                }
-                L[(e - e0) * r + lane] = make_float2(sh, sl);
-                coef[((int64_t)X.slot * k + q) * r + lane] = __dadd_rn((double)sh, (double)sl);
-            } else {
-                const float2 *p = L + X.pad * r;
-                float2 *o0 = L + (2 * (e - e0)) * r, *o1 = o0 + r;
-                float h0 = o0[lane].x, l0 = o0[lane].y, h1 = o1[lane].x, l1 = o1[lane].y;
-                for (int m = 0; m < r; ++m) {
-                    const float2 t0 = Ts[lane * r + m], t1 = Ts[r * r + lane * r + m];
-                    df_fma(h0, l0, t0.x, t0.y, p[m].x, p[m].y);
-                    df_fma(h1, l1, t1.x, t1.y, p[m].x, p[m].y);
-                }
-                o0[lane] = make_float2(h0, l0);
-                o1[lane] = make_float2(h1, l1);
-                coef[((int64_t)X.c0 * k + q) * r + lane] = __dadd_rn((double)h0, (double)l0);
-                coef[((int64_t)X.c1 * k + q) * r + lane] = __dadd_rn((double)h1, (double)l1);
-            }
-        }
-        __syncthreads();
-    }
+    pdl_wait();                                                // inputs of the band are ready
+    xfer_df_fetch<UP>(recs, coef, L, r, k, q);
+    __syncthreads();
+    if (r == 20) xfer_df_levels<UP, 20>(recs, Ts, coef, L, r, k, q);
+    else xfer_df_levels<UP, 0>(recs, Ts, coef, L, r, k, q);
 }
 template __global__ void xfer_df<true>(const hm_task *, const hm_step *, const hm_xfer *, const float2 *, double *,
                                        int, int, int);

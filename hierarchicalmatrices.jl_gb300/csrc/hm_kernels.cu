@@ -219,18 +219,20 @@ __global__ void xfer_up_task(const hm_task *tasks, const hm_step *steps, const h
                              int r, int k, int early)
 {
     extern __shared__ unsigned char smem_raw[];
+    __shared__ TaskRecs recs;
     A *Ts = reinterpret_cast<A *>(smem_raw);
     A *L = Ts + 2 * HM_RMAX * HM_RMAX;
-    const hm_task tk = tasks[blockIdx.x];
     const int q0 = blockIdx.y * QC;                            // this CTA's right-hand sides
     if (early) pdl_trigger();     // the next band may be scheduled now (a small grid; not before a large one)
     for (int i = threadIdx.x; i < 2 * r * r; i += blockDim.x) async_copy<sizeof(A)>(Ts + i, T + i);
+    load_task(tasks + blockIdx.x, steps, ents, recs);
+    __syncthreads();
     pdl_wait();                                                // the children's coefficients are ready
-    xfer_up_fetch<A, QC>(tk, steps, ents, t, L, r, k, q0);
+    xfer_up_fetch<A, QC>(recs, t, L, r, k, q0);
     async_wait_all();
     __syncthreads();
-    if (r == 20) xfer_up_levels<A, QC, 20>(tk, steps, ents, Ts, t, L, r, k, q0);
-    else xfer_up_levels<A, QC, 0>(tk, steps, ents, Ts, t, L, r, k, q0);
+    if (r == 20) xfer_up_levels<A, QC, 20>(recs, Ts, t, L, r, k, q0);
+    else xfer_up_levels<A, QC, 0>(recs, Ts, t, L, r, k, q0);
 }
 
 template <typename A, int QC>
@@ -238,18 +240,20 @@ __global__ void xfer_down_task(const hm_task *tasks, const hm_step *steps, const
                              int r, int k, int early)
 {
     extern __shared__ unsigned char smem_raw[];
+    __shared__ TaskRecs recs;
     A *Ts = reinterpret_cast<A *>(smem_raw);
     A *L = Ts + 2 * HM_RMAX * HM_RMAX;
-    const hm_task tk = tasks[blockIdx.x];
     const int q0 = blockIdx.y * QC;                            // this CTA's right-hand sides
     if (early) pdl_trigger();
     for (int i = threadIdx.x; i < 2 * r * r; i += blockDim.x) async_copy<sizeof(A)>(Ts + i, T + i);
+    load_task(tasks + blockIdx.x, steps, ents, recs);
+    __syncthreads();
     pdl_wait();                                                // far-field and parent coefficients are ready
-    xfer_down_fetch<A, QC>(tk, steps, ents, s, L, r, k, q0);
+    xfer_down_fetch<A, QC>(recs, s, L, r, k, q0);
     async_wait_all();
     __syncthreads();
-    if (r == 20) xfer_down_levels<A, QC, 20>(tk, steps, ents, Ts, s, L, r, k, q0);
-    else xfer_down_levels<A, QC, 0>(tk, steps, ents, Ts, s, L, r, k, q0);
+    if (r == 20) xfer_down_levels<A, QC, 20>(recs, Ts, s, L, r, k, q0);
+    else xfer_down_levels<A, QC, 0>(recs, Ts, s, L, r, k, q0);
 }
 
 // One warp per (row slot, chunk of up to QC right-hand sides) (m2l_row, hm_tree.cuh).
@@ -261,11 +265,16 @@ __global__ void m2l(const hm_m2l_row *rows, int nrows, const hm_m2l_ent *ents, c
     const int wib = threadIdx.x >> 5;
     const int nq = (k + QC - 1) / QC;
     const int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    pdl_trigger();
-    pdl_wait();                                                // the upward pass's coefficients are ready
-    if (w >= (int64_t)nrows * nq) return;
     unsigned char *smem = smem_raw + wib * m2l_warp_bytes<S, A, QC>(fstride);
-    const hm_m2l_row R = rows[w / nq];
+    const bool live = w < (int64_t)nrows * nq;
+    pdl_trigger();
+    hm_m2l_row R{};
+    if (live) {
+        R = rows[w / nq];
+        m2l_first(R, ents, F, fstride, smem);
+    }
+    pdl_wait();                                                // the upward pass's coefficients are ready
+    if (!live) return;
     const int q0 = (int)(w % nq) * QC;
     if (r == 20) m2l_row<S, A, QC, 20>(R, q0, ents, F, fstride, t, s, r, k, smem);
     else m2l_row<S, A, QC, 0>(R, q0, ents, F, fstride, t, s, r, k, smem);
@@ -421,227 +430,35 @@ __global__ void expand_part(MulArgs<S> ma, const hm_seg *segs, int nsegs, const 
                             const A *s, const A *t, int r, int maxw, S *yfar, int64_t ldf)
 {
     extern __shared__ unsigned char smem_raw[];
-    const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
     const int seg = blockIdx.x * (blockDim.x >> 5) + wib;
     if constexpr (FAR) pdl_wait();                             // the downward pass's coefficients are ready
     if (seg >= nsegs) return;
     A *g = reinterpret_cast<A *>(smem_raw) + (int64_t)wib * maxw * KB;
     const hm_seg G = segs[seg];
-    const int k = ma.k;
-    // gather the right-hand sides of the columns this part uses; the part's
-    // pieces are one contiguous column run [c0, c1) of the panel
-    int c0 = -1, c1 = 0, col = 0;
-    for (int pc = 0; pc < G.npieces; ++pc) {
-        const hm_piece Q = pieces[G.piece0 + pc];
-        const bool take = FAR ? (Q.kind != HM_PIECE_X) : (Q.kind == HM_PIECE_X);
-        if (take) {
-            if (c0 < 0) c0 = col;
-            const A *coef = Q.kind == HM_PIECE_TCOEF ? t : s;
-            // fire-and-forget copies into shared memory for every piece, one
-            // wait after the loop (no load-to-store round trip per piece)
-            const int n = Q.width * KB;
-            for (int i = lane; i < n; i += 32) {
-                const int c = i / KB, q = i % KB;
-                A *d = g + (col + c) * KB + q;
-                if (q >= k) {
-                    *d = A(0);
-                } else if constexpr (FAR) {
-                    async_copy<sizeof(A)>(d, coef + ((int64_t)Q.src * k + q) * r + c);
-                } else if constexpr (sizeof(S) == sizeof(A)) {
-                    async_copy<sizeof(A)>(d, ma.x + (Q.src + c) * ma.incx + (int64_t)q * ma.ldx);
-                } else {
-                    *d = (A)ma.x[(Q.src + c) * ma.incx + (int64_t)q * ma.ldx];
-                }
-            }
-            c1 = col + Q.width;
-        }
-        col += Q.width;
-    }
-    async_wait_all();
-    if (c0 < 0) {
-        if (FAR && !yfar) return;          // no far field on these rows
-        c0 = c1 = 0;
-    }
+    int c0, c1;
+    if (!seg_gather<S, A, FAR, KB>(ma, G, pieces, s, t, r, g, c0, c1) && FAR && !yfar) return;   // no far field
     __syncwarp();
-    const S *Pg = P + G.poff;
+    constexpr int NR = SegRows<S, KB>::per_lane;
+    A val[KB][NR];
+    seg_columns<S, A, KB>(P + G.poff, G.ld, g, c0, c1, val);
     // FAR with yfar: write the far-field rows to yfar (added to y later);
     // FAR without: add into y; near field: y (+)= per the caller's flag
     const bool acc_y = FAR ? (yfar == nullptr) : (ma.accumulate != 0);
-    constexpr int FOLD = 64;              // columns between compensated folds (KB > 1)
-    if constexpr (sizeof(S) == 4 && KB >= 4) {
-        // four or more right-hand sides: each value loaded feeds KB FMAs, so
-        // two rows per lane (float2) and every column in turn, which halves
-        // the accumulators of the four-row form (3 KB values per row) and lets
-        // twice as many warps hide the loads' latency
-        SegAcc<A, KB> a0, a1;
-        a0.zero(); a1.zero();
-        if (2 * lane < G.ld) {
-            const float2 *base = reinterpret_cast<const float2 *>(Pg + 2 * lane);
-            const int64_t ld2 = G.ld / 2;
-            for (int cb = c0; cb < c1; cb += FOLD) {
-                const int ce = min(c1, cb + FOLD);
-                int c = cb;
-                for (; c + 16 <= ce; c += 16) {      // 16 loads in flight per lane
-                    float2 p[16];
 #pragma unroll
-                    for (int u = 0; u < 16; ++u) p[u] = __ldcs(base + ld2 * (c + u));
+    for (int q = 0; q < KB; ++q) {
+        if (q >= ma.k) break;
 #pragma unroll
-                    for (int u = 0; u < 16; ++u) { a0.add(p[u].x, g + (c + u) * KB); a1.add(p[u].y, g + (c + u) * KB); }
-                }
-                for (; c + 8 <= ce; c += 8) {
-                    float2 p[8];
-#pragma unroll
-                    for (int u = 0; u < 8; ++u) p[u] = __ldcs(base + ld2 * (c + u));
-#pragma unroll
-                    for (int u = 0; u < 8; ++u) { a0.add(p[u].x, g + (c + u) * KB); a1.add(p[u].y, g + (c + u) * KB); }
-                }
-                for (; c + 4 <= ce; c += 4) {
-                    float2 p[4];
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) p[u] = __ldcs(base + ld2 * (c + u));
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) { a0.add(p[u].x, g + (c + u) * KB); a1.add(p[u].y, g + (c + u) * KB); }
-                }
-                for (; c < ce; ++c) {
-                    const float2 p0 = __ldcs(base + ld2 * c);
-                    a0.add(p0.x, g + c * KB); a1.add(p0.y, g + c * KB);
-                }
-                a0.fold(); a1.fold();
-            }
-        }
-#pragma unroll
-        for (int q = 0; q < KB; ++q) {
-            if (q >= k) break;
-            const A v2[2] = {a0.merged(q, 0, 0), a1.merged(q, 0, 0)};
-#pragma unroll
-            for (int j = 0; j < 2; ++j) {
-                const int row = 2 * lane + j;
-                if (row < G.nrows) {
-                    if (FAR && yfar) {
-                        yfar[(G.row0 + row) + (int64_t)q * ldf] = (S)v2[j];
-                    } else {
-                        S *yp = ma.y + (G.row0 + row) * ma.incy + (int64_t)q * ma.ldy;
-                        A v = v2[j];
-                        if (acc_y) v += (A)(*yp);
-                        *yp = (S)v;
-                    }
-                }
-            }
-        }
-    } else if (sizeof(S) == 4) {
-        const int rg = lane & 15, h = lane >> 4;
-        SegAcc<A, KB> acc[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[j].zero();
-        if (4 * rg < G.ld) {
-            const float4 *base = reinterpret_cast<const float4 *>(Pg + 4 * rg);
-            const int64_t ld4 = G.ld / 4;
-            for (int cb = c0; cb < c1; cb += FOLD) {
-                const int ce = min(c1, cb + FOLD);
-                int c = cb + ((h - cb) & 1);             // this half's columns have parity h
-                for (; c + 14 < ce; c += 16) {
-                    float4 p[8];
-#pragma unroll
-                    for (int u = 0; u < 8; ++u) p[u] = __ldcs(base + ld4 * (c + 2 * u));
-#pragma unroll
-                    for (int u = 0; u < 8; ++u) {
-                        const A *gu = g + (c + 2 * u) * KB;
-                        acc[0].add(p[u].x, gu); acc[1].add(p[u].y, gu); acc[2].add(p[u].z, gu); acc[3].add(p[u].w, gu);
-                    }
-                }
-                for (; c + 6 < ce; c += 8) {           // tails in batches: fewer dependent round trips
-                    float4 p[4];
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) p[u] = __ldcs(base + ld4 * (c + 2 * u));
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        const A *gu = g + (c + 2 * u) * KB;
-                        acc[0].add(p[u].x, gu); acc[1].add(p[u].y, gu); acc[2].add(p[u].z, gu); acc[3].add(p[u].w, gu);
-                    }
-                }
-                for (; c + 2 < ce; c += 4) {
-                    const float4 p0 = __ldcs(base + ld4 * c), p1 = __ldcs(base + ld4 * (c + 2));
-                    const A *g0 = g + c * KB, *g1 = g + (c + 2) * KB;
-                    acc[0].add(p0.x, g0); acc[1].add(p0.y, g0); acc[2].add(p0.z, g0); acc[3].add(p0.w, g0);
-                    acc[0].add(p1.x, g1); acc[1].add(p1.y, g1); acc[2].add(p1.z, g1); acc[3].add(p1.w, g1);
-                }
-                for (; c < ce; c += 2) {
-                    const float4 p0 = __ldcs(base + ld4 * c);
-                    const A *g0 = g + c * KB;
-                    acc[0].add(p0.x, g0); acc[1].add(p0.y, g0); acc[2].add(p0.z, g0); acc[3].add(p0.w, g0);
-                }
-#pragma unroll
-                for (int j = 0; j < 4; ++j) acc[j].fold();
-            }
-        }
-#pragma unroll
-        for (int q = 0; q < KB; ++q) {
-            if (q >= k) break;
-            A val[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const A so = __shfl_xor_sync(0xffffffffu, acc[j].hi(q), 16);
-                const A co = __shfl_xor_sync(0xffffffffu, acc[j].lo(q), 16);
-                val[j] = acc[j].merged(q, so, co);
-            }
-            if (h == 0) {
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const int row = 4 * rg + j;
-                    if (row < G.nrows) {
-                        if (FAR && yfar) {
-                            yfar[(G.row0 + row) + (int64_t)q * ldf] = (S)val[j];
-                        } else {
-                            S *yp = ma.y + (G.row0 + row) * ma.incy + (int64_t)q * ma.ldy;
-                            A v = val[j];
-                            if (acc_y) v += (A)(*yp);
-                            *yp = (S)v;
-                        }
-                    }
-                }
-            }
-        }
-    } else {
-        SegAcc<A, KB> a0, a1;
-        a0.zero(); a1.zero();
-        if (2 * lane < G.ld) {
-            const double2 *base = reinterpret_cast<const double2 *>(Pg + 2 * lane);
-            const int64_t ld2 = G.ld / 2;
-            for (int cb = c0; cb < c1; cb += FOLD) {
-                const int ce = min(c1, cb + FOLD);
-                int c = cb;
-                for (; c + 8 <= ce; c += 8) {
-                    double2 p[8];
-#pragma unroll
-                    for (int u = 0; u < 8; ++u) p[u] = __ldcs(base + ld2 * (c + u));
-#pragma unroll
-                    for (int u = 0; u < 8; ++u) { a0.add(p[u].x, g + (c + u) * KB); a1.add(p[u].y, g + (c + u) * KB); }
-                }
-                for (; c < ce; ++c) {
-                    const double2 p0 = __ldcs(base + ld2 * c);
-                    a0.add(p0.x, g + c * KB); a1.add(p0.y, g + c * KB);
-                }
-                a0.fold(); a1.fold();
-            }
-        }
-#pragma unroll
-        for (int q = 0; q < KB; ++q) {
-            if (q >= k) break;
-            const A v2[2] = {a0.merged(q, 0, 0), a1.merged(q, 0, 0)};
-#pragma unroll
-            for (int j = 0; j < 2; ++j) {
-                const int row = 2 * lane + j;
-                if (row < G.nrows) {
-                    if (FAR && yfar) {
-                        yfar[(G.row0 + row) + (int64_t)q * ldf] = (S)v2[j];
-                    } else {
-                        S *yp = ma.y + (G.row0 + row) * ma.incy + (int64_t)q * ma.ldy;
-                        A v = v2[j];
-                        if (acc_y) v += (A)(*yp);
-                        *yp = (S)v;
-                    }
-                }
+        for (int j = 0; j < NR; ++j) {
+            const int row = SegRows<S, KB>::row(j);
+            if (row >= G.nrows) continue;
+            if (FAR && yfar) {
+                yfar[(G.row0 + row) + (int64_t)q * ldf] = (S)val[q][j];
+            } else {
+                S *yp = ma.y + (G.row0 + row) * ma.incy + (int64_t)q * ma.ldy;
+                A v = val[q][j];
+                if (acc_y) v += (A)(*yp);
+                *yp = (S)v;
             }
         }
     }
@@ -1175,8 +992,14 @@ HM_INST_FAR(float, float, 4) HM_INST_FAR(float, float, 8) HM_INST_FAR(double, do
 HM_INST_FAR(double, double, 8)
 #define HM_INST_MV(S, A)                                                                             \
     template __global__ void leaf_up<S, A, 1>(MulArgs<S>, const hm_vpanel *, int, const S *, A *, int, int, int, LeafParts<A>); \
+    template __global__ void leaf_up<S, A, 2>(MulArgs<S>, const hm_vpanel *, int, const S *, A *, int, int, int, LeafParts<A>); \
+    template __global__ void leaf_up<S, A, 4>(MulArgs<S>, const hm_vpanel *, int, const S *, A *, int, int, int, LeafParts<A>); \
     template __global__ void leaf_up<S, A, 8>(MulArgs<S>, const hm_vpanel *, int, const S *, A *, int, int, int, LeafParts<A>); \
     template __global__ void m2l<S, A, 1>(const hm_m2l_row *, int, const hm_m2l_ent *, const S *, int,    \
+                                          const A *, A *, int, int);                                    \
+    template __global__ void m2l<S, A, 2>(const hm_m2l_row *, int, const hm_m2l_ent *, const S *, int,    \
+                                          const A *, A *, int, int);                                    \
+    template __global__ void m2l<S, A, 4>(const hm_m2l_row *, int, const hm_m2l_ent *, const S *, int,    \
                                           const A *, A *, int, int);                                    \
     template __global__ void m2l<S, A, 8>(const hm_m2l_row *, int, const hm_m2l_ent *, const S *, int,    \
                                           const A *, A *, int, int);                                    \
@@ -1188,17 +1011,33 @@ HM_INST_FAR(double, double, 8)
                                             const A *, const A *, int, int);                            \
     template __global__ void xfer_up_band<A, 1>(const hm_task *, const hm_step *, const hm_xfer *, const A *, \
                                                 A *, int, int);                                         \
+    template __global__ void xfer_up_band<A, 2>(const hm_task *, const hm_step *, const hm_xfer *, const A *, \
+                                                A *, int, int);                                         \
+    template __global__ void xfer_up_band<A, 4>(const hm_task *, const hm_step *, const hm_xfer *, const A *, \
+                                                A *, int, int);                                         \
     template __global__ void xfer_up_band<A, 8>(const hm_task *, const hm_step *, const hm_xfer *, const A *, \
                                                 A *, int, int);                                         \
     template __global__ void xfer_down_band<A, 1>(const hm_task *, const hm_step *, const hm_xfer *,        \
+                                                  const A *, A *, int, int);                            \
+    template __global__ void xfer_down_band<A, 2>(const hm_task *, const hm_step *, const hm_xfer *,        \
+                                                  const A *, A *, int, int);                            \
+    template __global__ void xfer_down_band<A, 4>(const hm_task *, const hm_step *, const hm_xfer *,        \
                                                   const A *, A *, int, int);                            \
     template __global__ void xfer_down_band<A, 8>(const hm_task *, const hm_step *, const hm_xfer *,        \
                                                   const A *, A *, int, int);                            \
     template __global__ void xfer_up_task<A, 1>(const hm_task *, const hm_step *, const hm_xfer *, const A *, \
                                                 A *, int, int, int);                                    \
+    template __global__ void xfer_up_task<A, 2>(const hm_task *, const hm_step *, const hm_xfer *, const A *, \
+                                                A *, int, int, int);                                    \
+    template __global__ void xfer_up_task<A, 4>(const hm_task *, const hm_step *, const hm_xfer *, const A *, \
+                                                A *, int, int, int);                                    \
     template __global__ void xfer_up_task<A, 8>(const hm_task *, const hm_step *, const hm_xfer *, const A *, \
                                                 A *, int, int, int);                                    \
     template __global__ void xfer_down_task<A, 1>(const hm_task *, const hm_step *, const hm_xfer *,        \
+                                                  const A *, A *, int, int, int);                       \
+    template __global__ void xfer_down_task<A, 2>(const hm_task *, const hm_step *, const hm_xfer *,        \
+                                                  const A *, A *, int, int, int);                       \
+    template __global__ void xfer_down_task<A, 4>(const hm_task *, const hm_step *, const hm_xfer *,        \
                                                   const A *, A *, int, int, int);                       \
     template __global__ void xfer_down_task<A, 8>(const hm_task *, const hm_step *, const hm_xfer *,        \
                                                   const A *, A *, int, int, int);

@@ -1,9 +1,9 @@
-// Device bodies of the tree passes and of a row segment's sums, shared by the
-// stage kernels (one launch per stage, hm_kernels.cu, hm_df.cu) and the fused
-// ones (hm_fused.cu).  Written for sm_103a.
+// Device bodies of the tree passes and of a row segment's sums, for the stage
+// kernels (one launch per stage, hm_kernels.cu, hm_df.cu).  Written for sm_103a.
 #pragma once
 #include "hm_async.cuh"
 #include "hm_kernels.cuh"
+#include "hm_plan.h"
 
 namespace hm {
 namespace {
@@ -217,9 +217,33 @@ __device__ __forceinline__ void leaf_panel(const MulArgs<S> &ma, const hm_vpanel
     }
 }
 
+// One band task's records in shared memory.  A level walk that reads its steps
+// and records from global memory pays two dependent L2 round trips per level,
+// more than the level's arithmetic; they are constant, so a kernel stages them
+// before it waits for its inputs.
+constexpr int kTaskRecs = (1 << kBandLevels) - 1;
+struct TaskRecs {
+    hm_xfer x[kTaskRecs];
+    hm_step step[kBandLevels];      // record ranges of the levels, relative to x
+    int nrec, nsteps;
+};
+// Fills R for one task by the CTA (a barrier is needed before it is read).
+__device__ __forceinline__ void load_task(const hm_task *task, const hm_step *steps, const hm_xfer *ents, TaskRecs &R)
+{
+    const hm_task tk = *task;
+    const int e0 = steps[tk.step0].e0, nrec = steps[tk.step1 - 1].e1 - e0, ns = tk.step1 - tk.step0;
+    const int tid = threadIdx.x;
+    if (tid < nrec) R.x[tid] = ents[e0 + tid];
+    if (tid < ns) {
+        const hm_step st = steps[tk.step0 + tid];
+        R.step[tid] = hm_step{st.e0 - e0, st.e1 - e0};
+    }
+    if (tid == 0) { R.nrec = nrec; R.nsteps = ns; }
+}
+
 // Band tasks with shared-memory-resident coefficients, one CTA per (task,
-// chunk of QC right-hand sides: blockIdx.y): the task's
-// external inputs (and T) are fetched once with cp.async, every level then
+// chunk of QC right-hand sides): the task's external inputs (and T) are fetched
+// once with cp.async, every level then
 // reads and writes shared memory only, with a CTA barrier between levels;
 // each coefficient the task produces is also written to global memory.
 // Task-local numbering (records' pad, set by the planner): upward, record i
@@ -228,19 +252,17 @@ __device__ __forceinline__ void leaf_panel(const MulArgs<S> &ma, const hm_vpanel
 // Upward, L holds r x QC values per local, right-hand side fastest
 // (L[local][m][qq]); downward QC x r (L[local][qq][m]).
 template <typename A, int QC>
-__device__ __forceinline__ void xfer_up_fetch(const hm_task &tk, const hm_step *steps, const hm_xfer *ents, const A *t,
-                                        A *L, int r, int k, int q0)
+__device__ __forceinline__ void xfer_up_fetch(const TaskRecs &R, const A *t, A *L, int r, int k, int q0)
 {
-    const int e0 = steps[tk.step0].e0, e1 = steps[tk.step1 - 1].e1, nrec = e1 - e0;
     const int qc = min(QC, k - q0);
     // external children: warps take records, lanes coefficients
-    for (int rec = threadIdx.x >> 5; rec < nrec; rec += blockDim.x >> 5) {
-        const hm_xfer X = ents[e0 + rec];
+    for (int rec = threadIdx.x >> 5; rec < R.nrec; rec += blockDim.x >> 5) {
+        const hm_xfer X = R.x[rec];
         const int ln = threadIdx.x & 31;
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
             const int lc = c ? (X.pad >> 16) : (X.pad & 0xffff);
-            if (lc < nrec || ln >= r) continue;           // produced by an earlier level of this task
+            if (lc < R.nrec || ln >= r) continue;         // produced by an earlier level of this task
             const A *src = t + ((int64_t)(c ? X.c1 : X.c0) * k + q0) * r + ln;
             A *d = L + (int64_t)lc * QC * r + ln * QC;
 #pragma unroll
@@ -257,42 +279,44 @@ __device__ __forceinline__ void xfer_up_fetch(const hm_task &tk, const hm_step *
 // inner loops unrolled their shared-memory loads issue ahead of the FMAs that
 // use them: the level walks are latency bound (a 100,003 x 77,777 FP32 matrix
 // with 3 right-hand sides 84.6 -> 74.6 us per product, n = 2^20 with one 233 ->
-// 226 us; FP64 708 -> 684 us, where the upward step's two FMAs per term
-// replace a multiply, an FMA and an add on the FP64 pipe).
+// 226 us).
 template <typename A, int QC, int RC>
-__device__ __forceinline__ void xfer_up_levels(const hm_task &tk, const hm_step *steps, const hm_xfer *ents,
-                                               const A *Ts, A *t, A *L, int rr, int k, int q0)
+__device__ __forceinline__ void xfer_up_levels(const TaskRecs &R, const A *Ts, A *t, A *L, int rr, int k, int q0)
 {
     const int r = RC ? RC : rr;
-    const int e0 = steps[tk.step0].e0;
     const int qc = min(QC, k - q0);
     const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    for (int st = tk.step0; st < tk.step1; ++st) {
-        const hm_step S = steps[st];
-        for (int w = threadIdx.x >> 5; w < S.e1 - S.e0; w += nw) {
-            const int e = S.e0 + w;
-            const hm_xfer X = ents[e];
+    for (int st = 0; st < R.nsteps; ++st) {
+        const hm_step S = R.step[st];
+        for (int e = S.e0 + (threadIdx.x >> 5); e < S.e1; e += nw) {
+            const hm_xfer X = R.x[e];
             const A *c0 = L + (int64_t)(X.pad & 0xffff) * QC * r;
             const A *c1 = L + (int64_t)(X.pad >> 16) * QC * r;
-            A *out = L + (int64_t)(e - e0) * QC * r;
+            A *out = L + (int64_t)e * QC * r;
             if (lane < r) {
-                A acc[QC];
+                // one sum per child: an FMA per term (a0 v0 + a1 v1 in one expression
+                // is three operations), and neither sum is rounded more often than
+                // when the pair was added first
+                A s0[QC], s1[QC];
 #pragma unroll
-                for (int qq = 0; qq < QC; ++qq) acc[qq] = 0;
+                for (int qq = 0; qq < QC; ++qq) s0[qq] = s1[qq] = 0;
 #pragma unroll(RC ? RC : 4)
                 for (int mp = 0; mp < r; ++mp) {
                     const A a0 = Ts[mp * r + lane], a1 = Ts[r * r + mp * r + lane];
                     A v0[QC], v1[QC];
                     ld_vec<QC>(c0 + mp * QC, v0);
                     ld_vec<QC>(c1 + mp * QC, v1);
-                    // two FMAs (a0 v0 + a1 v1 added to acc would be three operations)
 #pragma unroll
-                    for (int qq = 0; qq < QC; ++qq) acc[qq] = fma(a1, v1[qq], fma(a0, v0[qq], acc[qq]));
+                    for (int qq = 0; qq < QC; ++qq) {
+                        s0[qq] = fma(a0, v0[qq], s0[qq]);
+                        s1[qq] = fma(a1, v1[qq], s1[qq]);
+                    }
                 }
 #pragma unroll
                 for (int qq = 0; qq < QC; ++qq) {
-                    out[lane * QC + qq] = acc[qq];
-                    if (qq < qc) t[((int64_t)X.slot * k + q0 + qq) * r + lane] = acc[qq];
+                    const A sum = s0[qq] + s1[qq];
+                    out[lane * QC + qq] = sum;
+                    if (qq < qc) t[((int64_t)X.slot * k + q0 + qq) * r + lane] = sum;
                 }
             }
         }
@@ -301,15 +325,13 @@ __device__ __forceinline__ void xfer_up_levels(const hm_task &tk, const hm_step 
 }
 
 template <typename A, int QC>
-__device__ __forceinline__ void xfer_down_fetch(const hm_task &tk, const hm_step *steps, const hm_xfer *ents, const A *s,
-                                        A *L, int r, int k, int q0)
+__device__ __forceinline__ void xfer_down_fetch(const TaskRecs &R, const A *s, A *L, int r, int k, int q0)
 {
-    const int e0 = steps[tk.step0].e0, e1 = steps[tk.step1 - 1].e1, nrec = e1 - e0;
     const int qc = min(QC, k - q0);
     // children start from their far-field (m2l) coefficients; external parents as computed
     // warps take records, lanes coefficients
-    for (int rec = threadIdx.x >> 5; rec < nrec; rec += blockDim.x >> 5) {
-        const hm_xfer X = ents[e0 + rec];
+    for (int rec = threadIdx.x >> 5; rec < R.nrec; rec += blockDim.x >> 5) {
+        const hm_xfer X = R.x[rec];
         const int ln = threadIdx.x & 31;
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
@@ -320,7 +342,7 @@ __device__ __forceinline__ void xfer_down_fetch(const hm_task &tk, const hm_step
             } else {
                 lc = X.pad;
                 slot = X.slot;
-                if (lc < 2 * nrec) continue;              // a child of an earlier level of this task
+                if (lc < 2 * R.nrec) continue;            // a child of an earlier level of this task
             }
             if (ln >= r) continue;
             const A *src = s + ((int64_t)slot * k + q0) * r + ln;
@@ -335,33 +357,51 @@ __device__ __forceinline__ void xfer_down_fetch(const hm_task &tk, const hm_step
 }
 
 template <typename A, int QC, int RC>
-__device__ __forceinline__ void xfer_down_levels(const hm_task &tk, const hm_step *steps, const hm_xfer *ents,
-                                                 const A *Ts, A *s, A *L, int rr, int k, int q0)
+__device__ __forceinline__ void xfer_down_levels(const TaskRecs &R, const A *Ts, A *s, A *L, int rr, int k, int q0)
 {
     const int r = RC ? RC : rr;
-    const int e0 = steps[tk.step0].e0;
     const int qc = min(QC, k - q0);
     const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    for (int st = tk.step0; st < tk.step1; ++st) {
-        const hm_step S = steps[st];
-        for (int w = threadIdx.x >> 5; w < S.e1 - S.e0; w += nw) {
-            const int e = S.e0 + w;
-            const hm_xfer X = ents[e];
+    for (int st = 0; st < R.nsteps; ++st) {
+        const hm_step S = R.step[st];
+        for (int e = S.e0 + (threadIdx.x >> 5); e < S.e1; e += nw) {
+            const hm_xfer X = R.x[e];
             const A *p = L + (int64_t)X.pad * QC * r;
-            A *o0 = L + (int64_t)(2 * (e - e0)) * QC * r;
+            A *o0 = L + (int64_t)(2 * e) * QC * r;
             A *o1 = o0 + QC * r;
             if (lane < r) {
                 A a0[QC], a1[QC];
 #pragma unroll
                 for (int qq = 0; qq < QC; ++qq) { a0[qq] = 0; a1[qq] = 0; }
-#pragma unroll(RC ? RC : 4)
-                for (int m = 0; m < r; ++m) {
-                    const A t0 = Ts[lane * r + m], t1 = Ts[r * r + lane * r + m];
+                const A *Tl = Ts + lane * r, *Tr = Tl + r * r;
+                if constexpr (RC % 4 == 0 && RC > 0) {
+                    // rows of T and of the parent in 16-byte loads
 #pragma unroll
-                    for (int qq = 0; qq < QC; ++qq) {
-                        const A v = p[qq * r + m];
-                        a0[qq] += t0 * v;
-                        a1[qq] += t1 * v;
+                    for (int m = 0; m < RC; m += 4) {
+                        A t0[4], t1[4];
+                        ld_vec<4>(Tl + m, t0);
+                        ld_vec<4>(Tr + m, t1);
+#pragma unroll
+                        for (int qq = 0; qq < QC; ++qq) {
+                            A v[4];
+                            ld_vec<4>(p + qq * RC + m, v);
+#pragma unroll
+                            for (int u = 0; u < 4; ++u) {
+                                a0[qq] += t0[u] * v[u];
+                                a1[qq] += t1[u] * v[u];
+                            }
+                        }
+                    }
+                } else {
+#pragma unroll 4
+                    for (int m = 0; m < r; ++m) {
+                        const A t0 = Tl[m], t1 = Tr[m];
+#pragma unroll
+                        for (int qq = 0; qq < QC; ++qq) {
+                            const A v = p[qq * r + m];
+                            a0[qq] += t0 * v;
+                            a1[qq] += t1 * v;
+                        }
                     }
                 }
 #pragma unroll
@@ -386,7 +426,21 @@ __device__ __forceinline__ void xfer_down_levels(const hm_task &tk, const hm_ste
 // row and the column coefficients they multiply are double-buffered in
 // shared memory with cp.async: block e + 1 is in flight while block e is
 // used for every right-hand side of the chunk.  Lane m accumulates row m.
-// smem: m2l_warp_bytes of this warp.
+// smem: m2l_warp_bytes of this warp.  m2l_first copies the first block, which
+// does not depend on the upward pass: a kernel calls it before it waits.
+template <typename S>
+__device__ __forceinline__ void m2l_block(const S *F, int fstride, int64_t foff, S *dst)
+{
+    const char *src = reinterpret_cast<const char *>(F + foff);
+    for (int i = threadIdx.x & 31; i < (int)(fstride * sizeof(S) / 16); i += 32)
+        async_copy16(reinterpret_cast<char *>(dst) + 16 * i, src + 16 * i);
+}
+template <typename S>
+__device__ __forceinline__ void m2l_first(const hm_m2l_row &R, const hm_m2l_ent *ents, const S *F, int fstride,
+                                          unsigned char *smem)
+{
+    if (R.begin < R.end) m2l_block(F, fstride, ents[R.begin].foff, reinterpret_cast<S *>(smem));
+}
 template <typename S, typename A, int QC, int RC>
 __device__ __forceinline__ void m2l_row(const hm_m2l_row &R, int q0, const hm_m2l_ent *ents, const S *F, int fstride,
                                         const A *t, A *s, int rr, int k, unsigned char *smem)
@@ -399,9 +453,7 @@ __device__ __forceinline__ void m2l_row(const hm_m2l_row &R, int q0, const hm_m2
     const int qc = min(QC, k - q0);
     auto fetch = [&](int e, int buf) {
         const hm_m2l_ent E = ents[e];
-        const char *src = reinterpret_cast<const char *>(F + E.foff);
-        char *dst = reinterpret_cast<char *>(Fb + buf * fstride);
-        for (int i = lane; i < (int)(fstride * sizeof(S) / 16); i += 32) async_copy16(dst + 16 * i, src + 16 * i);
+        if (e > R.begin) m2l_block(F, fstride, E.foff, Fb + buf * fstride);      // the first: m2l_first
         A *tb = Tb + buf * QC * HM_RMAX;
         if (lane < r) {
             const A *src = t + ((int64_t)E.yslot * k + q0) * r + lane;
@@ -491,6 +543,193 @@ struct SegAcc {
         return t + (((h[q] - (t - bp)) + (so - bp)) + (l[q] + co));
     }
 };
+
+
+// The rows of a segment (<= 64) a lane sums: with one or two FP32 right-hand
+// sides lanes 0-15 and 16-31 take alternate columns, each lane four
+// consecutive rows (one 16-byte load per column; lanes 0-15 hold the sums);
+// otherwise every lane two rows.
+template <typename S, int KB>
+struct SegRows {
+    static constexpr bool quad = sizeof(S) == 4 && KB < 4;
+    static constexpr int per_lane = quad ? 4 : 2;
+    // row j of this lane, or past every segment where the lane holds no sums
+    static __device__ __forceinline__ int row(int j)
+    {
+        const int lane = threadIdx.x & 31;
+        if constexpr (quad) return lane < 16 ? 4 * lane + j : 1 << 20;
+        else return 2 * lane + j;
+    }
+};
+
+// Gathers the right-hand sides of a segment's near-field (FAR = false) or
+// far-field columns into shared memory (g[c * KB + q]) and waits for this
+// lane's copies.  The part's pieces are one contiguous column run [c0, c1) of
+// the panel; false (and an empty run) when there are none.
+template <typename S, typename A, bool FAR, int KB>
+__device__ __forceinline__ bool seg_gather(const MulArgs<S> &ma, const hm_seg &G, const hm_piece *pieces, const A *s,
+                                           const A *t, int r, A *g, int &c0, int &c1)
+{
+    const int lane = threadIdx.x & 31, k = ma.k;
+    int col = 0;
+    c0 = -1;
+    c1 = 0;
+    for (int pc = 0; pc < G.npieces; ++pc) {
+        const hm_piece Q = pieces[G.piece0 + pc];
+        const bool take = FAR ? (Q.kind != HM_PIECE_X) : (Q.kind == HM_PIECE_X);
+        if (take) {
+            if (c0 < 0) c0 = col;
+            const A *coef = Q.kind == HM_PIECE_TCOEF ? t : s;
+            // fire-and-forget copies into shared memory for every piece, one
+            // wait after the loop (no load-to-store round trip per piece)
+            const int n = Q.width * KB;
+            for (int i = lane; i < n; i += 32) {
+                const int c = i / KB, q = i % KB;
+                A *d = g + (col + c) * KB + q;
+                if (q >= k) {
+                    *d = A(0);
+                } else if constexpr (FAR) {
+                    async_copy<sizeof(A)>(d, coef + ((int64_t)Q.src * k + q) * r + c);
+                } else if constexpr (sizeof(S) == sizeof(A)) {
+                    async_copy<sizeof(A)>(d, ma.x + (Q.src + c) * ma.incx + (int64_t)q * ma.ldx);
+                } else {
+                    *d = (A)ma.x[(Q.src + c) * ma.incx + (int64_t)q * ma.ldx];
+                }
+            }
+            c1 = col + Q.width;
+        }
+        col += Q.width;
+    }
+    async_wait_all();
+    if (c0 >= 0) return true;
+    c0 = c1 = 0;
+    return false;
+}
+
+// val[q][j] = sum over columns [c0, c1) of P[row j][c] g[c * KB + q] for this
+// lane's rows (SegRows), FMA partial sums folded with TwoSum every 64 columns.
+template <typename S, typename A, int KB>
+__device__ __forceinline__ void seg_columns(const S *Pg, int ld, const A *g, int c0, int c1,
+                                            A (&val)[KB][SegRows<S, KB>::per_lane])
+{
+    const int lane = threadIdx.x & 31;
+    constexpr int FOLD = 64;              // columns between compensated folds (KB > 1)
+    if constexpr (sizeof(S) == 4 && KB >= 4) {
+        // four or more right-hand sides: each value loaded feeds KB FMAs, so
+        // two rows per lane (float2) and every column in turn, which halves
+        // the accumulators of the four-row form (3 KB values per row) and lets
+        // twice as many warps hide the loads' latency
+        SegAcc<A, KB> a0, a1;
+        a0.zero(); a1.zero();
+        if (2 * lane < ld) {
+            const float2 *base = reinterpret_cast<const float2 *>(Pg + 2 * lane);
+            const int64_t ld2 = ld / 2;
+            for (int cb = c0; cb < c1; cb += FOLD) {
+                const int ce = min(c1, cb + FOLD);
+                int c = cb;
+                for (; c + 16 <= ce; c += 16) {      // 16 loads in flight per lane
+                    float2 p[16];
+#pragma unroll
+                    for (int u = 0; u < 16; ++u) p[u] = __ldcs(base + ld2 * (c + u));
+#pragma unroll
+                    for (int u = 0; u < 16; ++u) { a0.add(p[u].x, g + (c + u) * KB); a1.add(p[u].y, g + (c + u) * KB); }
+                }
+                for (; c + 8 <= ce; c += 8) {
+                    float2 p[8];
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) p[u] = __ldcs(base + ld2 * (c + u));
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) { a0.add(p[u].x, g + (c + u) * KB); a1.add(p[u].y, g + (c + u) * KB); }
+                }
+                for (; c + 4 <= ce; c += 4) {
+                    float2 p[4];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) p[u] = __ldcs(base + ld2 * (c + u));
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) { a0.add(p[u].x, g + (c + u) * KB); a1.add(p[u].y, g + (c + u) * KB); }
+                }
+                for (; c < ce; ++c) {
+                    const float2 p0 = __ldcs(base + ld2 * c);
+                    a0.add(p0.x, g + c * KB); a1.add(p0.y, g + c * KB);
+                }
+                a0.fold(); a1.fold();
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < KB; ++q) { val[q][0] = a0.merged(q, 0, 0); val[q][1] = a1.merged(q, 0, 0); }
+    } else if constexpr (sizeof(S) == 4) {
+        const int rg = lane & 15, h = lane >> 4;
+        SegAcc<A, KB> acc[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[j].zero();
+        if (4 * rg < ld) {
+            const float4 *base = reinterpret_cast<const float4 *>(Pg + 4 * rg);
+            const int64_t ld4 = ld / 4;
+            auto add4 = [&](const float4 &p, const A *gu) {
+                acc[0].add(p.x, gu); acc[1].add(p.y, gu); acc[2].add(p.z, gu); acc[3].add(p.w, gu);
+            };
+            for (int cb = c0; cb < c1; cb += FOLD) {
+                const int ce = min(c1, cb + FOLD);
+                int c = cb + ((h - cb) & 1);             // this half's columns have parity h
+                for (; c + 14 < ce; c += 16) {
+                    float4 p[8];
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) p[u] = __ldcs(base + ld4 * (c + 2 * u));
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) add4(p[u], g + (c + 2 * u) * KB);
+                }
+                for (; c + 6 < ce; c += 8) {           // tails in batches: fewer dependent round trips
+                    float4 p[4];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) p[u] = __ldcs(base + ld4 * (c + 2 * u));
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) add4(p[u], g + (c + 2 * u) * KB);
+                }
+                for (; c + 2 < ce; c += 4) {
+                    const float4 p0 = __ldcs(base + ld4 * c), p1 = __ldcs(base + ld4 * (c + 2));
+                    add4(p0, g + c * KB);
+                    add4(p1, g + (c + 2) * KB);
+                }
+                for (; c < ce; c += 2) add4(__ldcs(base + ld4 * c), g + c * KB);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) acc[j].fold();
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < KB; ++q)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const A so = __shfl_xor_sync(0xffffffffu, acc[j].hi(q), 16);
+                const A co = __shfl_xor_sync(0xffffffffu, acc[j].lo(q), 16);
+                val[q][j] = acc[j].merged(q, so, co);
+            }
+    } else {
+        SegAcc<A, KB> a0, a1;
+        a0.zero(); a1.zero();
+        if (2 * lane < ld) {
+            const double2 *base = reinterpret_cast<const double2 *>(Pg + 2 * lane);
+            const int64_t ld2 = ld / 2;
+            for (int cb = c0; cb < c1; cb += FOLD) {
+                const int ce = min(c1, cb + FOLD);
+                int c = cb;
+                for (; c + 8 <= ce; c += 8) {
+                    double2 p[8];
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) p[u] = __ldcs(base + ld2 * (c + u));
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) { a0.add(p[u].x, g + (c + u) * KB); a1.add(p[u].y, g + (c + u) * KB); }
+                }
+                for (; c < ce; ++c) {
+                    const double2 p0 = __ldcs(base + ld2 * c);
+                    a0.add(p0.x, g + c * KB); a1.add(p0.y, g + c * KB);
+                }
+                a0.fold(); a1.fold();
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < KB; ++q) { val[q][0] = a0.merged(q, 0, 0); val[q][1] = a1.merged(q, 0, 0); }
+    }
+}
 
 }  // namespace
 }  // namespace hm

@@ -20,6 +20,7 @@
 // xfer_task_w per CTA the two transfer matrices and the task's local vectors.
 #include "hm_kernels.cuh"
 #include "hm_async.cuh"
+#include "hm_tree.cuh"
 
 namespace hm {
 
@@ -284,8 +285,7 @@ __global__ void __launch_bounds__(kWideTaskThreads)
     A *Ts = reinterpret_cast<A *>(wide_smem);
     A *L = Ts + 2 * R * R;
     constexpr int LV = QL * R;                                 // values of one local vector
-    const hm_task tk = tasks[blockIdx.x];
-    const int e0 = steps[tk.step0].e0, e1 = steps[tk.step1 - 1].e1, nrec = e1 - e0;
+    __shared__ TaskRecs recs;
     const int q0 = blockIdx.y * QL, qc = min(QL, k - q0);
     const int lane0 = threadIdx.x & 31, warp = threadIdx.x >> 5;
     // group (warp, g) of QL lanes takes records warp * G + g, + nw * G, ...
@@ -300,10 +300,13 @@ __global__ void __launch_bounds__(kWideTaskThreads)
             async_copy<sizeof(A)>(Ts + i, T + c * R * R + mp * R + m);
         }
     }
+    load_task(tasks + blockIdx.x, steps, ents, recs);
+    __syncthreads();
+    const int nrec = recs.nrec;
     pdl_wait();                                                // inputs of the band are ready
     // external inputs: groups take records, a group copies a QL x R block
     for (int rec = gw; rec < nrec; rec += nw) {
-        const hm_xfer X = ents[e0 + rec];
+        const hm_xfer X = recs.x[rec];
 #pragma unroll
         for (int c = 0; c < (UP ? 2 : 3); ++c) {
             int lc, slot;
@@ -325,11 +328,10 @@ __global__ void __launch_bounds__(kWideTaskThreads)
     }
     async_wait_all();
     __syncthreads();
-    for (int st = tk.step0; st < tk.step1; ++st) {
-        const hm_step S = steps[st];
-        for (int w = gw; w < S.e1 - S.e0; w += nw) {
-            const int e = S.e0 + w;
-            const hm_xfer X = ents[e];
+    for (int st = 0; st < recs.nsteps; ++st) {
+        const hm_step S = recs.step[st];
+        for (int e = S.e0 + gw; e < S.e1; e += nw) {
+            const hm_xfer X = recs.x[e];
             if (UP) {
                 const A *c0 = L + (int64_t)(X.pad & 0xffff) * LV + lane * R;
                 const A *c1 = L + (int64_t)(X.pad >> 16) * LV + lane * R;
@@ -353,7 +355,7 @@ __global__ void __launch_bounds__(kWideTaskThreads)
                         }
                     }
                 }
-                A *out = L + (int64_t)(e - e0) * LV + lane * R;
+                A *out = L + (int64_t)e * LV + lane * R;
 #pragma unroll
                 for (int m = 0; m < R; m += 4) st4<A>(out + m, acc + m);
                 if (lane < qc) {
@@ -363,7 +365,7 @@ __global__ void __launch_bounds__(kWideTaskThreads)
                 }
             } else {
                 const A *p = L + (int64_t)X.pad * LV + lane * R;
-                A *o0 = L + (int64_t)(2 * (e - e0)) * LV + lane * R;
+                A *o0 = L + (int64_t)(2 * e) * LV + lane * R;
                 A *o1 = o0 + LV;
                 A a0[R], a1[R];
 #pragma unroll
