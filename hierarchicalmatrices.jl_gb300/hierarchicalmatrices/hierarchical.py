@@ -422,13 +422,19 @@ class AbstractHierarchical:
         import torch
         from .kernelmatrix import _stream_ptr
         h = self.handle(_np_dtype(x))
+        # the results are overwritten (accumulate 0): no zero fill
         if x.dim() == 1:
-            y = torch.zeros(self.shape[0], dtype=x.dtype, device=x.device)
-            return self.mul(y, x.contiguous())
+            m, n = self.shape
+            if x.shape[0] < n:
+                raise IndexError(f"index out of bounds: x has {x.shape[0]} entries, needs {n}")
+            x = x.contiguous()
+            y = torch.empty(m, dtype=x.dtype, device=x.device)
+            check(lib.hm_mul(h, x.data_ptr(), n, y.data_ptr(), m, 1, 0, _stream_ptr(None)))
+            return y
         X = x if x.stride(0) == 1 else x.t().contiguous().t()
-        Y = torch.zeros((x.shape[1], self.shape[0]), dtype=x.dtype, device=x.device).t()
+        Y = torch.empty((x.shape[1], self.shape[0]), dtype=x.dtype, device=x.device).t()
         check(lib.hm_mul(h, X.data_ptr(), max(X.stride(1), self.shape[1]), Y.data_ptr(), max(Y.stride(1), self.shape[0]),
-                         x.shape[1], 1, _stream_ptr(None)))
+                         x.shape[1], 0, _stream_ptr(None)))
         return Y
 
     def __del__(self):

@@ -309,7 +309,7 @@ class KernelMatrix:
             import torch
             if isinstance(v, torch.Tensor):
                 shape = (self.shape[0],) if v.dim() == 1 else (v.shape[1], self.shape[0])
-                u = torch.zeros(shape, dtype=v.dtype, device=v.device)
+                u = torch.empty(shape, dtype=v.dtype, device=v.device)       # overwritten (accumulate=False)
                 if v.dim() == 2:
                     u = u.t()                        # column-major view
                 return self.mul(u, v, accumulate=False)
