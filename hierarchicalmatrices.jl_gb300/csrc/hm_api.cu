@@ -16,6 +16,7 @@
 #include <type_traits>
 #include <vector>
 
+#include "hm_fused.cuh"
 #include "hm_kernels.cuh"
 #include "hm_plan.h"
 #include "hmgpu.h"
@@ -1356,6 +1357,213 @@ int launch_expand_k(hm_handle *h, const MulArgs<S> &ma, const A *s, const A *t, 
     return HM_OK;
 }
 
+// ---- the fused schedule (hm_fused.cu) ----------------------------------------
+
+// Whether the tree passes are more than one stage of leaf bases.
+bool has_transfers(const hm_handle *h)
+{
+    return h->n_m2l_rows > 0 || last_band(h->up_band_ptr) >= 0 || last_band(h->down_band_ptr) >= 0;
+}
+
+constexpr size_t kFusedSmemTarget = 96 * 1024;   // leaves room for expand_both beside tree_fused on an SM
+
+// Shared memory and warps of one tree_fused launch.
+struct FusedPlan {
+    size_t smem;
+    int leaf_warps, m2l_warps;
+};
+
+template <typename S, typename A, int QC, bool DF>
+bool fused_plan(const hm_handle *h, bool split, FusedPlan &fp)
+{
+    const size_t es = DF ? sizeof(float2) : sizeof(A);
+    const size_t ts = 2 * (size_t)HM_RMAX * HM_RMAX * es;
+    const int cap = split ? kPartRows : h->vp_cap;
+    const size_t lb = DF ? (size_t)cap * sizeof(float2) : leaf_up_warp_bytes<S, A, QC>(cap, h->vp_wcap);
+    const size_t mb = DF ? (size_t)(kM2lDfStages * 400 + 32) * sizeof(float2) : m2l_warp_bytes<S, A, QC>(h->fstride);
+    auto warps = [&](size_t b) {
+        return (int)std::max<size_t>(1, std::min<size_t>(kFusedThreads / 32, (kFusedSmemTarget - ts) / std::max<size_t>(b, 1)));
+    };
+    fp.leaf_warps = warps(lb);
+    fp.m2l_warps = warps(mb);
+    const size_t lv = (size_t)(DF ? 1 : QC) * h->r * es;
+    fp.smem = ts + std::max(std::max(h->n_vp ? fp.leaf_warps * lb : 0, h->n_m2l_rows ? fp.m2l_warps * mb : 0),
+                            (size_t)std::max(h->band_locals[0], h->band_locals[1]) * lv);
+    return fp.smem <= kTaskSmemMax;
+}
+
+template <typename S, typename A>
+bool fused_plan_k(const hm_handle *h, int k, bool split, FusedPlan &fp)
+{
+    const int qc = tree_chunk(k);
+    return qc == 1   ? fused_plan<S, A, 1, false>(h, split, fp)
+           : qc == 2 ? fused_plan<S, A, 2, false>(h, split, fp)
+           : qc == 4 ? fused_plan<S, A, 4, false>(h, split, fp)
+                     : fused_plan<S, A, 8, false>(h, split, fp);
+}
+
+// Whether a product takes the fused schedule: the default stream schedule
+// (HM_OPT_OVERLAP 2) with the default panel kernels, ordinary device vectors, no
+// stage timing, and a tree small enough.
+template <typename S, typename A>
+bool fused_ok(const hm_handle *h, const MulArgs<S> &ma, const Sched &sc)
+{
+    if (sc.overlap != 2 || sc.near_kernel != 0 || ma.xin || ma.yout || (h->profile_mask & 0xfu)) return false;
+    if (!(h->n_vp || h->n_m2l_rows) || !h->n_segs || !h->stream_ctas) return false;
+    if (ma.k > 2 && h->part_width[1] > 64) return false;
+    const bool df = h->storage == HM_DF64;
+    if (df && h->n_m2l_rows && h->r != 20) return false;
+    if (h->up_band_ptr.size() > kFusedBands + 1 || h->down_band_ptr.size() > kFusedBands + 1) return false;
+    const bool split = h->d_vparts != nullptr;
+    FusedPlan fp;
+    bool fits;
+    if constexpr (std::is_same<S, double>::value)
+        fits = df ? fused_plan<S, A, 1, true>(h, split, fp) : fused_plan_k<S, A>(h, ma.k, split, fp);
+    else
+        fits = fused_plan_k<S, A>(h, ma.k, split, fp);
+    // expand_both gathers whole segments; wider ones keep the streaming kernels
+    const size_t kb = ma.k > kPartMaxK ? 0 : ma.k > 4 ? 8 : ma.k > 2 ? 4 : 2;
+    if (!fits || kWarpsPerCta * (size_t)h->max_width * kb * (df ? sizeof(float2) : sizeof(A)) > 100 * 1024) return false;
+    // The lines, in coefficient slots (about n / 30), where the cluster's 16 SMs
+    // take as long as the stage kernels on all of them (us, fused against stages):
+    // FP32, 1 right-hand side: 21.7 / 30.8 at 144, 24.9 / 30.5 at 272, 38.3 / 33.1
+    // at 578; 8: 33.7 / 41.3 at 144, 42.0 / 41.8 at 272; 16: 41.4 / 43.9 at 60, 54.7
+    // / 51.7 at 144.  FP64, 1: 47.5 / 64.5 at 144, 61.9 / 67.1 at 272, 101 / 83 at 578;
+    // 2: 76 / 88 at 144, 99 / 90 at 272; 8: 256 / 263 at 144.  HM_DF64, 1: 49.8 /
+    // 57.5 at 144, 80.6 / 72.6 at 578; 2: 82 / 85 at 272; 4: 47.6 / 72.2 at 60, 86 / 81 at
+    // 144; 8: 88 / 130 at 60.  Matrices without transfers or far-field blocks
+    // (low-rank factors only) run their one tree stage on all SMs at any size.
+    const int slots = std::max(h->n_xslots, h->n_yslots), k = ma.k;
+    if (!has_transfers(h)) return k <= kPartMaxK;
+    if (df) return slots <= (k <= 2 ? 288 : k <= 8 ? 80 : 0);
+    if (sizeof(S) == 8) return slots <= (k == 1 ? 320 : k <= 8 ? 160 : 0);
+    return slots <= (k <= 4 ? 320 : k <= 8 ? 160 : k <= 16 ? 64 : 0);
+}
+
+// Clusters of kFusedCtas (beyond the portable 8) for `kernel`, set once per device.
+std::set<std::pair<int, const void *>> g_cluster_set;
+template <typename K>
+int allow_cluster(K kernel)
+{
+    int dev = 0;
+    HM_CK(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> lk(g_smem_mu);
+    if (!g_cluster_set.insert({dev, reinterpret_cast<const void *>(kernel)}).second) return HM_OK;
+    HM_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    return HM_OK;
+}
+
+template <typename S, typename A, int QC, bool DF>
+int launch_tree_fused(hm_handle *h, const MulArgs<S> &ma, cudaStream_t st, A *t, A *s, const LeafParts<A> &lp, int *sync)
+{
+    TreeArgs<S, A> a;
+    a.ma = ma;
+    a.vp = lp.rec ? h->d_vp_split : h->d_vp;
+    a.n_vp = lp.rec ? h->n_vp_split : h->n_vp;
+    a.cap = lp.rec ? kPartRows : h->vp_cap;
+    a.wcap = h->vp_wcap;
+    a.V = h->d_V; a.T = h->d_T; a.F = h->d_F;
+    a.lp = lp;
+    a.up_tasks = h->d_up_tasks; a.up_steps = h->d_up_steps; a.up_ents = h->d_up_ents;
+    a.down_tasks = h->d_down_tasks; a.down_steps = h->d_down_steps; a.down_ents = h->d_down_ents;
+    a.rows = h->d_m2l_rows; a.n_rows = h->n_m2l_rows; a.ents = h->d_m2l_ents; a.fstride = h->fstride;
+    a.t = t; a.s = s;
+    a.r = h->r;
+    auto bands = [&](const std::vector<int> &ptr, int *out) {
+        int n = 0;
+        out[0] = ptr.empty() ? 0 : ptr[0];
+        for (size_t b = 0; b + 1 < ptr.size(); ++b) {
+            if (ptr[b + 1] == ptr[b]) continue;
+            out[++n] = ptr[b + 1];
+        }
+        return n;
+    };
+    a.n_up = bands(h->up_band_ptr, a.up_band);
+    a.n_down = bands(h->down_band_ptr, a.down_band);
+    FusedPlan fp;
+    fused_plan<S, A, QC, DF>(h, lp.rec != nullptr, fp);
+    a.leaf_warps = fp.leaf_warps;
+    a.m2l_warps = fp.m2l_warps;
+    auto kern = tree_fused<S, A, QC, DF>;
+    HM_TRY(ensure_smem(kern, fp.smem));
+    HM_TRY(allow_cluster(kern));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(kFusedCtas);
+    cfg.blockDim = dim3(kFusedThreads);
+    cfg.dynamicSmemBytes = fp.smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = kFusedCtas;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cuda_status(cudaLaunchKernelEx(&cfg, kern, a), "tree_fused");
+}
+
+template <typename S, typename A, int KB>
+int launch_both(hm_handle *h, const MulArgs<S> &ma, cudaStream_t st, const A *t, const A *s, const void *panels, bool pdl)
+{
+    const int maxw = std::max(h->max_width, 1);
+    if constexpr (std::is_same<S, double>::value) {
+        if (h->storage == HM_DF64) {
+            const size_t smem = (size_t)kWarpsPerCta * maxw * KB * sizeof(float2);
+            HM_TRY(ensure_smem(expand_both_df<KB>, smem));
+            return launch_k("expand_both_df", expand_both_df<KB>, dim3(warp_ctas(h->n_segs)), dim3(32 * kWarpsPerCta),
+                            smem, st, pdl, ma, h->d_segs, h->n_segs, h->d_pieces, static_cast<const float2 *>(panels),
+                            s, t, h->r, maxw);
+        }
+    }
+    const size_t smem = (size_t)kWarpsPerCta * maxw * KB * sizeof(A);
+    HM_TRY((ensure_smem(expand_both<S, A, KB>, smem)));
+    const int tile = cur_sched(h).tile;
+    return launch_k("expand_both", expand_both<S, A, KB>, dim3(warp_ctas(h->n_segs)), dim3(32 * kWarpsPerCta), smem, st,
+                    pdl, ma, h->d_segs, h->n_segs, h->d_pieces, static_cast<const S *>(panels), s, t, h->r, maxw,
+                    kRingTile[tile >= 0 && tile < kRingTiles ? tile : 0].pf);
+}
+
+template <typename S, typename A>
+int launch_fused(hm_handle *h, const MulArgs<S> &ma, cudaStream_t st, void *scratch, int *sync, const void *panels)
+{
+    const int k = ma.k;
+    const ScratchLayout L = scratch_layout<A>(h, k);
+    A *t = reinterpret_cast<A *>(static_cast<char *>(scratch) + L.t_off);
+    A *s = reinterpret_cast<A *>(static_cast<char *>(scratch) + L.s_off);
+    LeafParts<A> lp;
+    if (h->d_vparts) {
+        lp.rec = h->d_vparts;
+        lp.sums = reinterpret_cast<A *>(static_cast<char *>(scratch) + parts_off<A>(h, k));
+        lp.count = sync;
+    }
+    StageTimer whole(h, 4, st);
+    bool done = false;             // the tree passes are launched
+    if (!has_transfers(h)) {
+        done = true;
+        HM_TRY((launch_tree<S, A>(h, ma, st, t, s, false, nullptr, 0, nullptr, lp)));
+    }
+    if constexpr (std::is_same<S, double>::value) {
+        if (!done && h->storage == HM_DF64) {
+            done = true;
+            HM_TRY((launch_tree_fused<S, A, 1, true>(h, ma, st, t, s, lp, sync)));
+        }
+    }
+    if (!done) {
+        const int qc = tree_chunk(k);
+        HM_TRY((qc == 1   ? launch_tree_fused<S, A, 1, false>(h, ma, st, t, s, lp, sync)
+                : qc == 2 ? launch_tree_fused<S, A, 2, false>(h, ma, st, t, s, lp, sync)
+                : qc == 4 ? launch_tree_fused<S, A, 4, false>(h, ma, st, t, s, lp, sync)
+                          : launch_tree_fused<S, A, 8, false>(h, ma, st, t, s, lp, sync)));
+    }
+    if (k > kPartMaxK) return launch_expand_k<S, A>(h, ma, s, t, panels, st);
+    const bool pdl = h->pdl != 0;
+    if constexpr (sizeof(S) == 8) {
+        if (k == 1) return launch_both<S, A, 1>(h, ma, st, t, s, panels, pdl);
+    }
+    if (k <= 2) return launch_both<S, A, 2>(h, ma, st, t, s, panels, pdl);
+    if (k <= 4) return launch_both<S, A, 4>(h, ma, st, t, s, panels, pdl);
+    return launch_both<S, A, 8>(h, ma, st, t, s, panels, pdl);
+}
+
 // One product.  With a side stream the tree passes and the far-field rows
 // (U s, into the scratch vector yfar) run there, concurrently with the
 // near-field panels on the caller's stream; yfar is added to y after the join.
@@ -1441,6 +1649,7 @@ int run_mul(hm_handle *h, MulArgs<S> ma, cudaStream_t st, const void *panels = n
     SchedScope scope(&sched);
     hm_handle::StreamCtx *sc = nullptr;
     HM_TRY(stream_ctx(h, st, stream_scratch_bytes<A>(h, ma.k), &sc));
+    if (fused_ok<S, A>(h, ma, sched)) return launch_fused<S, A>(h, ma, st, sc->p, sc->sync, panels ? panels : h->d_P);
     StageTimer whole(h, 4, st);
     return launch_pipeline<S, A>(h, ma, st, sched.overlap ? sc->side : st, sc->fork, sc->join, sc->p, true, panels,
                                  sched.overlap >= 2 ? sc->mid : nullptr, sc->sync);
