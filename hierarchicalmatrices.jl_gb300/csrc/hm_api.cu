@@ -280,6 +280,7 @@ struct hm_handle {
     unsigned long long wait_ns = 2000000000ull;
     int test_stall = 0;
     bool tc_ok = false;             // segments fit the tensor-core panel kernel
+    bool quad_pieces = false;       // every piece starts at a multiple of 4 columns, X pieces of 4 rows of x too
     bool tensor_cores = true;       // use it for FP32 products with many right-hand sides
 
     std::mutex mu;
@@ -394,9 +395,22 @@ int prepare_streaming(hm_handle *h, const std::vector<hm_seg> &segs, const std::
     HM_CK(cudaMemsetAsync(h->d_status, 0, sizeof(int), st));
     h->stream_ctas = 0;
     if (segs.empty()) return HM_OK;
+    int dev = 0, sms = 0;
+    HM_CK(cudaGetDevice(&dev));
+    HM_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    h->sms = sms;
     h->tc_ok = true;
-    for (const hm_seg &g : segs)
+    h->quad_pieces = h->r % 4 == 0;
+    for (const hm_seg &g : segs) {
         if (g.ld % 4 || g.poff % 32 || g.nrows > 64 || g.ld > 64) h->tc_ok = false;
+        int col = 0;
+        for (int i = 0; i < g.npieces; ++i) {
+            const hm_piece &q = pieces[g.piece0 + i];
+            if (col % 4 || (q.kind == HM_PIECE_X && q.src % 4) || (q.width % 4 && i + 1 < g.npieces)) h->quad_pieces = false;
+            col += q.width;
+        }
+        if (col % 4) h->quad_pieces = false;
+    }
     for (const hm_seg &g : segs) {
         int nfar = 0;
         bool seen_x = false;
@@ -411,10 +425,6 @@ int prepare_streaming(hm_handle *h, const std::vector<hm_seg> &segs, const std::
         h->part_width[0] = std::max(h->part_width[0], g.width - g.nfar);
         h->part_width[1] = std::max(h->part_width[1], g.nfar);
     }
-    int dev = 0, sms = 0;
-    HM_CK(cudaGetDevice(&dev));
-    HM_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    h->sms = sms;
     double near_bytes = 0;
     for (const hm_seg &g : segs) near_bytes += (double)(g.width - g.nfar) * g.ld * 4.0;
     const int64_t want = std::max<int64_t>((int64_t)kStreamCtasPerSm * sms, (int64_t)(near_bytes / kStreamCtaBytes));
@@ -1337,12 +1347,19 @@ int launch_expand_k(hm_handle *h, const MulArgs<S> &ma, const A *s, const A *t, 
     if constexpr (sizeof(S) == 4 && sizeof(A) == 4) {
         if (cur_sched(h).tensor_cores && h->tc_ok && ma.k >= kTensorCoreMinK) {
             const int maxw = std::max(h->max_width, 1);
-            const size_t smem = expand_tc_smem_bytes(maxw);
-            HM_TRY(ensure_smem(expand_tc, smem));
-            // right-hand-side chunks of a segment run next to each other (its panel is re-read from L2)
-            const dim3 grid((unsigned)((ma.k + 127) / 128), (unsigned)h->n_segs);
-            expand_tc<<<grid, 256, smem, st>>>(ma, h->d_segs, h->d_pieces, static_cast<const float *>(panels), s, t,
-                                               h->r, maxw, h->d_status, h->wait_ns, h->test_stall);
+            const TcPlan plan = expand_tc_plan(ma.k, maxw);
+            if (!plan.stages) { set_error("panels of %d columns do not fit in shared memory", maxw); return HM_ERR_UNSUPPORTED; }
+            const bool vec = h->quad_pieces && ma.incx == 1 && ma.ldx % 4 == 0 &&
+                             reinterpret_cast<uintptr_t>(ma.x) % 16 == 0;
+            auto kern = ma.k <= 32   ? (vec ? expand_tc<true, 2> : expand_tc<false, 2>)
+                        : ma.k <= 64 ? (vec ? expand_tc<true, 4> : expand_tc<false, 4>)
+                                     : (vec ? expand_tc<true, 8> : expand_tc<false, 8>);
+            HM_TRY(ensure_smem(kern, plan.smem));
+            // a segment's chunks of 128 right-hand sides run at the same time (its panel comes from L2)
+            const int64_t items = (int64_t)h->n_segs * ((ma.k + 127) / 128);
+            kern<<<(unsigned)std::min<int64_t>(items, h->sms), TC_THREADS, plan.smem, st>>>(
+                ma, h->d_segs, h->n_segs, h->d_pieces, static_cast<const float *>(panels), s, t, h->r, maxw, plan,
+                h->d_status, h->wait_ns, h->test_stall);
             HM_CK_LAUNCH("expand_tc");
             return HM_OK;
         }

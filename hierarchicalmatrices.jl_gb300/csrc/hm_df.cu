@@ -274,8 +274,9 @@ __global__ void xfer_df(const hm_task *tasks, const hm_step *steps, const hm_xfe
     float2 *L = Ts + 2 * HM_RMAX * HM_RMAX;                    // r pairs per local
     const int q = blockIdx.y;
     if (early) pdl_trigger();
-    for (int i = threadIdx.x; i < 2 * r * r; i += blockDim.x) Ts[i] = T[i];
+    for (int i = threadIdx.x; i < 2 * r * r; i += blockDim.x) async_copy<8>(Ts + i, T + i);
     load_task(tasks + blockIdx.x, steps, ents, recs);
+    async_wait_all();
     __syncthreads();
     pdl_wait();                                                // inputs of the band are ready
     xfer_df_fetch<UP>(recs, coef, L, r, k, q);

@@ -30,7 +30,7 @@ __device__ __forceinline__ void df_fma(float &sh, float &sl, float ph, float pl,
 }
 
 // One basis panel by one warp (leaf_up_df); xs: cap pairs of this warp.
-__device__ __forceinline__ void leaf_panel_df(const MulArgs<double> &ma, const hm_vpanel &P, const float2 *V, double *t,
+__device__ __forceinline__ void leaf_panel_df(const MulArgs<double> &ma, const hm_vpanel P, const float2 *V, double *t,
                                               int r, int cap, float2 *xs)
 {
     const int lane = threadIdx.x & 31;
@@ -75,7 +75,7 @@ __device__ __forceinline__ void leaf_panel_df(const MulArgs<double> &ma, const h
 // One row slot's far field by one warp (m2l_df_ring, rank 20); ring: NS blocks
 // and ts: 32 pairs of this warp.
 template <int NS>
-__device__ __forceinline__ void m2l_row_df(const hm_m2l_row &R, const hm_m2l_ent *ents, const float2 *F,
+__device__ __forceinline__ void m2l_row_df(const hm_m2l_row R, const hm_m2l_ent *ents, const float2 *F,
                                            const double *t, double *s, int k, float2 *ring, float2 *ts)
 {
     constexpr int R20 = 20, BLK = R20 * R20;
@@ -170,7 +170,7 @@ __device__ __forceinline__ void xfer_df_levels(const TaskRecs &R, const float2 *
             if (UP) {
                 const float2 *c0 = L + (X.pad & 0xffff) * r, *c1 = L + (X.pad >> 16) * r;
                 float sh = 0.f, sl = 0.f;
-#pragma unroll(RC ? RC : 4)
+#pragma unroll 4
                 for (int mp = 0; mp < r; ++mp) {
                     const float2 a0 = Ts[mp * r + lane], a1 = Ts[r * r + mp * r + lane];
                     df_fma(sh, sl, a0.x, a0.y, c0[mp].x, c0[mp].y);
@@ -182,7 +182,7 @@ __device__ __forceinline__ void xfer_df_levels(const TaskRecs &R, const float2 *
                 const float2 *p = L + X.pad * r;
                 float2 *o0 = L + (2 * e) * r, *o1 = o0 + r;
                 float h0 = o0[lane].x, l0 = o0[lane].y, h1 = o1[lane].x, l1 = o1[lane].y;
-#pragma unroll(RC ? RC : 4)
+#pragma unroll 4
                 for (int m = 0; m < r; ++m) {
                     const float2 t0 = Ts[lane * r + m], t1 = Ts[r * r + lane * r + m];
                     df_fma(h0, l0, t0.x, t0.y, p[m].x, p[m].y);

@@ -332,15 +332,25 @@ template <int PART, int KB>
 __global__ void expand_df(MulArgs<double> ma, const hm_seg *segs, int nsegs, const hm_piece *pieces, const float2 *P,
                           const double *s, const double *t, int r, int maxw, double *yfar, int64_t ldf, int q0);
 
-// Tensor-core panels for many right-hand sides (FP32 storage): grid
-// (ceil(k / 128), segments), 256 threads, expand_tc_smem_bytes(maxw) of shared
-// memory; needs segments of <= 64 rows, ld % 4 == 0, poff % 32 == 0.
-// Waits on the tensor core give up after wait_ns (HM_DEV_WAIT_TIMEOUT in
-// *status); stall != 0 makes each CTA's first wait run out (test hook).
-size_t expand_tc_smem_bytes(int maxw);
-__global__ void expand_tc(MulArgs<float> ma, const hm_seg *segs, const hm_piece *pieces, const float *P,
-                          const float *s, const float *t, int r, int maxw, int *status, unsigned long long wait_ns,
-                          int stall);
+// Tensor-core panels for many right-hand sides (FP32 storage): persistent, at
+// most one CTA of TC_THREADS threads per SM, shared memory and stages by
+// expand_tc_plan; needs segments of <= 64 rows, ld % 4 == 0, poff % 32 == 0.
+// Waits give up after wait_ns (HM_DEV_WAIT_TIMEOUT in *status); stall != 0 makes
+// each CTA's first wait for operands run out (test hook).
+constexpr int TC_THREADS = 704;
+struct TcPlan {
+    int groups;          // 8-row groups of live right-hand sides in an operand stage
+    int tables, stages;
+    size_t smem;
+};
+TcPlan expand_tc_plan(int k, int maxw);
+// VEC: every four panel columns from a multiple of 4 on belong to one piece and
+// start on a 16-byte boundary of its source.  NJ: at most 16 NJ right-hand sides
+// at a time (2, 4, 8).
+template <bool VEC, int NJ>
+__global__ void expand_tc(MulArgs<float> ma, const hm_seg *segs, int nsegs, const hm_piece *pieces, const float *P,
+                          const float *s, const float *t, int r, int maxw, TcPlan plan, int *status,
+                          unsigned long long wait_ns, int stall);
 
 template <typename S, typename A>
 __global__ void expand_k(MulArgs<S> ma, const hm_seg *segs, const hm_piece *pieces, const S *P, const A *s,

@@ -86,7 +86,7 @@ __device__ __forceinline__ bool last_arrival(int *count, int n, int lane)
 // apart per right-hand side.
 // smem: leaf_up_warp_bytes of this warp.
 template <typename S, typename A, int QC>
-__device__ __forceinline__ void leaf_panel(const MulArgs<S> &ma, const hm_vpanel &P, const hm_vpart &part, const S *V,
+__device__ __forceinline__ void leaf_panel(const MulArgs<S> &ma, const hm_vpanel P, const hm_vpart part, const S *V,
                                            A *t, int r, int cap, int wcap, unsigned char *smem,
                                            const LeafParts<A> &lp)
 {
@@ -436,13 +436,13 @@ __device__ __forceinline__ void m2l_block(const S *F, int fstride, int64_t foff,
         async_copy16(reinterpret_cast<char *>(dst) + 16 * i, src + 16 * i);
 }
 template <typename S>
-__device__ __forceinline__ void m2l_first(const hm_m2l_row &R, const hm_m2l_ent *ents, const S *F, int fstride,
+__device__ __forceinline__ void m2l_first(const hm_m2l_row R, const hm_m2l_ent *ents, const S *F, int fstride,
                                           unsigned char *smem)
 {
     if (R.begin < R.end) m2l_block(F, fstride, ents[R.begin].foff, reinterpret_cast<S *>(smem));
 }
 template <typename S, typename A, int QC, int RC>
-__device__ __forceinline__ void m2l_row(const hm_m2l_row &R, int q0, const hm_m2l_ent *ents, const S *F, int fstride,
+__device__ __forceinline__ void m2l_row(const hm_m2l_row R, int q0, const hm_m2l_ent *ents, const S *F, int fstride,
                                         const A *t, A *s, int rr, int k, unsigned char *smem)
 {
     const int r = RC ? RC : rr;
