@@ -225,12 +225,14 @@ TcPlan expand_tc_plan(int k, int maxw)
     TcPlan p;
     p.groups = ((k < TC_M ? k : TC_M) + 7) / 8;
     const size_t table = ((size_t)maxw * sizeof(const float *) + 127) / 128 * 128, stage = tc_stage_bytes(p.groups);
-    for (p.tables = TC_MAX_TABLES; p.tables >= 1; --p.tables) {
-        const size_t used = tc_fixed_bytes() + p.tables * table + 1024;        // the ring starts on a 1,024-byte boundary
-        const size_t fit = used < kMax ? (kMax - used) / stage : 0;
-        p.stages = (int)(fit < TC_MAX_STAGES ? fit : TC_MAX_STAGES);
-        p.smem = used + p.stages * stage;
-        if (p.stages >= 2) return p;
+    for (int least = 2; least >= 1; --least) {             // one stage only for panels of thousands of columns
+        for (p.tables = TC_MAX_TABLES; p.tables >= 1; --p.tables) {
+            const size_t used = tc_fixed_bytes() + p.tables * table + 1024;    // the ring starts on a 1,024-byte boundary
+            const size_t fit = used < kMax ? (kMax - used) / stage : 0;
+            p.stages = (int)(fit < TC_MAX_STAGES ? fit : TC_MAX_STAGES);
+            p.smem = used + p.stages * stage;
+            if (p.stages >= least) return p;
+        }
     }
     p.stages = 0;
     return p;
