@@ -315,7 +315,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
         uint32_t tab_phase = 0, phase = 0;
         TcItem it{};
         const float *const *cols = nullptr;
-        bool have = false, ok = true;                          // have: the item's table is open
+        bool have = false, ok = true, again = false;           // have: the item's table is open
         for (; stage >= plan.stages; stage -= plan.stages) phase ^= 1;
         while (ok) {
             // this group's next chunk, through the tables of the items it has no chunk of
@@ -378,6 +378,11 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
                     }
                 }
             }
+            // the stage's last fill read.  A parity tells a phase from its neighbours only:
+            // with two or more stages this group's previous chunk was let in after the
+            // fill before that one was read; on a single stage that is waited for first
+            if (plan.stages == 1 && again && !tc_wait<20>(&S.empty[0], phase, wait_ns, &S.abort)) break;
+            again = true;
             if (!tc_wait<20>(&S.empty[stage], phase ^ 1, wait_ns, &S.abort)) break;
             unsigned char *sg = ring + (size_t)stage * stage_bytes, *sp = sg + 3 * gpiece;
             // columns up to the last step of 16 the MMAs take
