@@ -250,6 +250,10 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     const int table_bytes = (int)(((size_t)maxw * sizeof(const float *) + 127) / 128 * 128);
     unsigned char *ring = tables + (size_t)plan.tables * table_bytes;
     ring += (1024u - (smem_addr(ring) & 1023u)) & 1023u;
+    // A parity tells a barrier's neighbouring phases apart only: two groups need two
+    // stages (a group's previous chunk was then let in after the fill two before
+    // its next one was read); on a single stage one group works.
+    const int ngroups = plan.stages > 1 ? TC_GROUPS : 1;
     const int gpiece = plan.groups * 1024, stage_bytes = tc_stage_bytes(plan.groups);
     const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     // items in order: segment, then chunk of right-hand sides; a CTA takes every
@@ -280,7 +284,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
         }
         for (int i = 0; i < plan.tables; ++i) {
             mbar_init(&S.tab_full[i], 1);
-            mbar_init(&S.tab_empty[i], TC_PRODUCERS);
+            mbar_init(&S.tab_empty[i], ngroups * TC_GROUP);
         }
         for (int i = 0; i < 2; ++i) {
             mbar_init(&S.acc_full[i], 1);
@@ -315,7 +319,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
         uint32_t tab_phase = 0, phase = 0;
         TcItem it{};
         const float *const *cols = nullptr;
-        bool have = false, ok = true, again = false;           // have: the item's table is open
+        bool have = false, ok = grp < ngroups;               // have: the item's table is open
         for (; stage >= plan.stages; stage -= plan.stages) phase ^= 1;
         while (ok) {
             // this group's next chunk, through the tables of the items it has no chunk of
@@ -378,11 +382,6 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
                     }
                 }
             }
-            // the stage's last fill read.  A parity tells a phase from its neighbours only:
-            // with two or more stages this group's previous chunk was let in after the
-            // fill before that one was read; on a single stage that is waited for first
-            if (plan.stages == 1 && again && !tc_wait<20>(&S.empty[0], phase, wait_ns, &S.abort)) break;
-            again = true;
             if (!tc_wait<20>(&S.empty[stage], phase ^ 1, wait_ns, &S.abort)) break;
             unsigned char *sg = ring + (size_t)stage * stage_bytes, *sp = sg + 3 * gpiece;
             // columns up to the last step of 16 the MMAs take
@@ -397,8 +396,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");               // visible to the tensor core
             __syncwarp();
             if (lane == 0) mbar_arrive(&S.full[stage]);
-            ch += TC_GROUPS;
-            for (stage += TC_GROUPS; stage >= plan.stages; stage -= plan.stages) phase ^= 1;
+            ch += ngroups;
+            for (stage += ngroups; stage >= plan.stages; stage -= plan.stages) phase ^= 1;
         }
     } else if (warp == 5) {
         // ---- column tables: the address of each column's right-hand side q0 (bit 0 set
