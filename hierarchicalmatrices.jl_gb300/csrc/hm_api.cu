@@ -194,7 +194,7 @@ void transfer_matrices(int r, const std::vector<double> &x, const std::vector<do
 struct Sched {
     int overlap, near_kernel, near_stages, tensor_cores, pdl;
     int tile = 0;      // per-warp ring tile (kRingTile index) for 3-8 FP32 right-hand sides
-    int wide = 1;      // tree passes on the lane-per-right-hand-side kernels: 0 never, 1 from 32, 2 from 2 RHS
+    int wide = 1;      // tree passes on the lane-per-right-hand-side kernels: 0 never, 1 by wide_tree_ok's rule, 2 from 2 RHS
 };
 
 // Right-hand-side buckets of the autotuned schedules: 1, 2, 3-4, 5-8, 9-16,
@@ -241,7 +241,7 @@ struct hm_handle {
     int vp_cap = 64, vp_wcap = HM_RMAX;   // leaf_up's shared-memory panel: rows (multiple of 32) x columns
     bool vp_covers_x = false;             // the leaf panels' rows partition [0, ny): leaf_up reads every x once
     bool vp_wide = false;                 // every leaf panel row-major with ld == width == 20 (leaf_up_w)
-    int wide_tree = 1;                    // lane-per-RHS tree kernels: 0 never, 1 from 32 RHS, 2 from 2 (HM_OPT_WIDE_TREE)
+    int wide_tree = 1;                    // lane-per-RHS tree kernels: 0 never, 1 by rule, 2 from 2 (HM_OPT_WIDE_TREE)
     int ring_tile = 0;                    // per-warp ring tile (HM_OPT_RING_TILE)
     // the panels with those of more than kPartRows rows split by rows (leaf_up's
     // parts), or none when no panel is that tall
@@ -868,6 +868,8 @@ inline unsigned warp_ctas(int64_t warps) { return (unsigned)((warps + kWarpsPerC
 
 constexpr size_t kTaskSmemMax = 200 * 1024;     // shared memory of a band task kernel
 constexpr int kWideMinK = 32;                    // right-hand sides from which the lane-per-RHS tree kernels run
+constexpr int kWideMinK32 = 5;                   // ... of FP32 storage, from kWideSlots32 coefficient slots on
+constexpr int kWideSlots32 = 2048;
 
 // Index of the last non-empty band of a band pointer array, or -1.
 inline int last_band(const std::vector<int> &ptr)
@@ -1067,12 +1069,19 @@ int launch_tree_qc(hm_handle *h, const MulArgs<S> &ma, cudaStream_t st, A *t, A 
 inline int wide_groups(int k) { return k <= 8 ? 4 : k <= 16 ? 2 : 1; }
 
 // Whether the tree passes of a product with k right-hand sides run on those
-// kernels under the schedule's `wide` (0 never, 1 from kWideMinK, 2 from 2 on):
+// kernels under the schedule's `wide` (0 never, 1 by the rule, 2 from 2 on):
 // rank 20, panels of the stored layout, band tasks within shared memory.
+// The rule: from 32 right-hand sides, and FP32 from 5 on where the tree fills the
+// chip (slots: about n / 30).  FP32, us per product on random points, chunks of 8
+// against lane per right-hand side: 8 right-hand sides 49.2 / 48.0 at n = 2^15, 66.6
+// / 59.8 at 2^16, 285 / 269 at 2^19; 16: 72.9 / 72.4, 108 / 100, 535 / 463; 24: 81 /
+// 83 at 2^15, 335 / 306 at 2^18; but 4: 188 / 218 at 2^19.  FP64 (8: 3.56 / 3.69 ms at
+// 2^19) is bound by its pipe, which idle lanes fill as live ones do.
 template <typename S, typename A>
 bool wide_tree_ok(const hm_handle *h, const MulArgs<S> &ma, int wide)
 {
-    const int kmin = wide >= 2 ? 2 : wide == 1 ? kWideMinK : INT32_MAX;
+    const bool big32 = sizeof(S) == 4 && std::max(h->n_xslots, h->n_yslots) >= kWideSlots32;
+    const int kmin = wide >= 2 ? 2 : wide == 1 ? (big32 ? kWideMinK32 : kWideMinK) : INT32_MAX;
     if (!(std::is_same<S, A>::value && ma.k >= kmin && h->r == 20 && h->vp_wide && !ma.xin && h->fstride % 4 == 0 &&
           h->storage != HM_DF64))
         return false;
@@ -1581,6 +1590,31 @@ int launch_fused(hm_handle *h, const MulArgs<S> &ma, cudaStream_t st, void *scra
     return launch_both<S, A, 8>(h, ma, st, t, s, panels, pdl);
 }
 
+// The stage of the tree passes that the near field starts after under the default
+// schedule (the result keeps its bits wherever it starts); HM_OPT_OVERLAP's values:
+// 1 none, 2 the upward pass, 4 the leaf stage.  Right-hand sides in host memory
+// (MulArgs::xin) are brought in by the leaf stage, so the near field waits for it.
+// Measured, us per product, start after 2 / 4 / 1 (random points unless a grid):
+//   FP32, 1: n = 2^17 56 / 59 / 62, 2^19 152 / 145 / 134, grid 2^19 121 / 114 / 124,
+//   grid 2^20 217 / 211 / 211, 2^22 774 / 769 / 807;  3: 2^13 (k = 5) 40.1 / 38.2 /
+//   36.7, 2^17 82 / 73 / 66, 2^19 208 / 182 / 186, 2^21 671 / 616 / 634;  8 (with the
+//   lane-per-right-hand-side tree kernels): 2^18 164 / 145 / 151, 2^19 330 / 286 / 269,
+//   128 instances 1,009 / 927 / 833.
+//   HM_DF64, 1: n = 2^15 108 / 84 / 86, 2^19 354 / 345 / 357, grid 2^19 288 / 264 /
+//   287; 2: 2^17 190 / 196 / 191.  FP64 (2^20 884 / 865 / 877, grid 672 / 676 / 672;
+//   k = 3, 2^17 590 / 634 / 629) has no line.
+template <typename S>
+int near_start(const hm_handle *h, const MulArgs<S> &ma, int overlap)
+{
+    if (overlap != 2 || ma.k > kPartMaxK) return overlap;
+    const int slots = std::max(h->n_xslots, h->n_yslots), k = ma.k;
+    int m = 2;
+    if (h->storage == HM_DF64) m = k == 1 ? 4 : 2;
+    else if (sizeof(S) == 4) m = k <= 2 ? (slots >= 8192 ? 4 : 2) : k <= 4 ? (slots >= 8192 ? 4 : 1)
+                                 : (slots >= 2048 && slots < 16384 ? 4 : 1);
+    return m == 1 && ma.xin ? 4 : m;
+}
+
 // One product.  With a side stream the tree passes and the far-field rows
 // (U s, into the scratch vector yfar) run there, concurrently with the
 // near-field panels on the caller's stream; yfar is added to y after the join.
@@ -1668,8 +1702,12 @@ int run_mul(hm_handle *h, MulArgs<S> ma, cudaStream_t st, const void *panels = n
     HM_TRY(stream_ctx(h, st, stream_scratch_bytes<A>(h, ma.k), &sc));
     if (fused_ok<S, A>(h, ma, sched)) return launch_fused<S, A>(h, ma, st, sc->p, sc->sync, panels ? panels : h->d_P);
     StageTimer whole(h, 4, st);
-    return launch_pipeline<S, A>(h, ma, st, sched.overlap ? sc->side : st, sc->fork, sc->join, sc->p, true, panels,
-                                 sched.overlap >= 2 ? sc->mid : nullptr, sc->sync);
+    Sched run = sched;
+    run.overlap = near_start(h, ma, sched.overlap);
+    SchedScope staged(&run);
+    // above kPartMaxK one panel kernel follows the tree passes: nothing waits for mid
+    return launch_pipeline<S, A>(h, ma, st, run.overlap ? sc->side : st, sc->fork, sc->join, sc->p, true, panels,
+                                 run.overlap >= 2 && ma.k <= kPartMaxK ? sc->mid : nullptr, sc->sync);
 }
 
 // Row-derivative panels (same layout as the panels), filled once.
@@ -1779,9 +1817,10 @@ std::vector<Sched> sched_candidates(const hm_handle *h, int k, bool fp32)
     // the lane-per-right-hand-side tree kernels on and off (32+, unless the
     // option turned them off)
     const bool ring = fp32 && k >= 3 && k <= kPartMaxK && h->stream_ctas > 0 && h->n_segs;
-    // (from 32 right-hand sides: on or off; from 2 to 31: the chunk-of-8 kernels or the grouped ones)
+    // (where the rule takes them: on or off; below: the chunk kernels or the grouped ones)
     std::vector<int> wides{base.wide};
-    if (tree && h->wide_tree && k >= kWideMinK) wides = {1, 0};
+    const int wide_from = fp32 && std::max(h->n_xslots, h->n_yslots) >= kWideSlots32 ? kWideMinK32 : kWideMinK;
+    if (tree && h->wide_tree && k >= wide_from) wides = {1, 0};
     else if (tree && h->wide_tree && k >= 2) wides = {1, 2};
     std::vector<Sched> c{base};       // the configured schedule first, timed for comparison
     auto add = [&c](Sched s) {

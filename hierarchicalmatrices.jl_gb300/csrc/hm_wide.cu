@@ -335,9 +335,11 @@ __global__ void __launch_bounds__(kWideTaskThreads)
             if (UP) {
                 const A *c0 = L + (int64_t)(X.pad & 0xffff) * LV + lane * R;
                 const A *c1 = L + (int64_t)(X.pad >> 16) * LV + lane * R;
-                A acc[R];
+                // one sum per child, added at the end: as a single chain of 2 R terms
+                // the FP32 log-kernel products were off by 15% more
+                A acc[R], acc1[R];
 #pragma unroll
-                for (int m = 0; m < R; ++m) acc[m] = A(0);
+                for (int m = 0; m < R; ++m) acc[m] = acc1[m] = A(0);
 #pragma unroll
                 for (int mp = 0; mp < R; mp += 4) {
                     A a[4], b[4];
@@ -351,10 +353,12 @@ __global__ void __launch_bounds__(kWideTaskThreads)
                             ld4(Ts + (mp + u) * R + m, t0);
                             ld4(Ts + R * R + (mp + u) * R + m, t1);
                             axpy4(t0, a[u], acc + m);
-                            axpy4(t1, b[u], acc + m);
+                            axpy4(t1, b[u], acc1 + m);
                         }
                     }
                 }
+#pragma unroll
+                for (int m = 0; m < R; ++m) acc[m] += acc1[m];
                 A *out = L + (int64_t)e * LV + lane * R;
 #pragma unroll
                 for (int m = 0; m < R; m += 4) st4<A>(out + m, acc + m);
@@ -369,10 +373,7 @@ __global__ void __launch_bounds__(kWideTaskThreads)
                 A *o1 = o0 + LV;
                 A a0[R], a1[R];
 #pragma unroll
-                for (int m = 0; m < R; m += 4) {
-                    ld4(o0 + m, a0 + m);
-                    ld4(o1 + m, a1 + m);
-                }
+                for (int m = 0; m < R; ++m) a0[m] = a1[m] = A(0);
 #pragma unroll
                 for (int m = 0; m < R; m += 4) {
                     A pv[4];
@@ -387,6 +388,17 @@ __global__ void __launch_bounds__(kWideTaskThreads)
                             axpy4(t0, pv[u], a0 + mq);
                             axpy4(t1, pv[u], a1 + mq);
                         }
+                    }
+                }
+#pragma unroll
+                for (int m = 0; m < R; m += 4) {               // the far-field values join the whole sums
+                    A f0[4], f1[4];
+                    ld4(o0 + m, f0);
+                    ld4(o1 + m, f1);
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        a0[m + u] += f0[u];
+                        a1[m + u] += f1[u];
                     }
                 }
 #pragma unroll

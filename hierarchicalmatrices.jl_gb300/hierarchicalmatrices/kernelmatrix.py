@@ -169,8 +169,8 @@ class KernelMatrix:
 
     def set_wide_tree(self, enable=True):
         """Tree passes on the lane-per-right-hand-side kernels: True (the
-        default) from 32 right-hand sides, "all" from 2, False never (the
-        kernels for chunks of 8)."""
+        default) from 32 right-hand sides and FP32 from 5 on large trees,
+        "all" from 2, False never (the kernels for chunks of up to 8)."""
         code = 2 if enable == "all" else (1 if enable else 0)
         check(lib.hm_configure(self._h, _lib.HM_OPT_WIDE_TREE, code))
 
@@ -333,9 +333,10 @@ class KernelMatrix:
 
     def set_overlap(self, enable=True):
         """Tree passes on a side stream beside the near-field panels: the near
-        field from the start (1), after the upward pass (2; True, the
-        default), after the far-field stage (3) or after the leaf-basis
-        stage (4); or every stage in order (False or 0)."""
+        field from the start (1), after the far-field stage (3), after the
+        leaf-basis stage (4) or where size and right-hand sides make it
+        fastest, a small matrix's product in two kernels (2; True, the
+        default); or every stage in order (False or 0)."""
         mode = int(enable) if not isinstance(enable, bool) else (2 if enable else 0)
         check(lib.hm_configure(self._h, _lib.HM_OPT_OVERLAP, mode))
 

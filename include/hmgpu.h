@@ -233,9 +233,11 @@ int hm_direct_rows(hm_handle *h, const double *b, const int64_t *rows, int64_t n
 
 /* Handle options.  HM_OPT_OVERLAP (default 2): 1 runs the tree passes of
    hm_mul on a side stream concurrently with the near-field panels from the
-   start, 2 starts the near field after the upward pass, 3 after the
-   far-field (M2L) stage, 4 after the leaf-basis stage of the upward pass; 0
-   runs every stage in order on the caller's stream. */
+   start, 3 starts the near field after the far-field (M2L) stage, 4 after the
+   leaf-basis stage of the upward pass, 2 where storage, size and right-hand
+   sides make it fastest (after the upward pass, as 4 or as 1), with a small
+   matrix's product in two kernels; 0 runs every stage in order on the
+   caller's stream. */
 enum {
     HM_OPT_OVERLAP = 1,
     /* HM_OPT_NEAR_STAGES (default 4, 2..16): shared-memory stages (8 KB each)
@@ -278,14 +280,14 @@ enum {
        nothing arrives on, so it runs out after HM_OPT_WAIT_LIMIT_NS.  Keeps
        autotuned schedules.  No reference counterpart. */
     HM_OPT_TEST_STALL = 8,
-    /* HM_OPT_WIDE_TREE (default 1): products with 32 or more right-hand sides
-       (rank 20) run the tree passes (leaf bases, transfers, far-field blocks)
+    /* HM_OPT_WIDE_TREE (default 1): products with 32 or more right-hand sides,
+       and FP32 ones with 5 or more on large trees (rank 20), run the tree passes (leaf bases, transfers, far-field blocks)
        on kernels that give each lane one right-hand side and all 20
        coefficients of it (a warp of 32, or 2 or 4 groups of 16 or 8 lanes);
        2 uses them from 2 right-hand sides on; 0 keeps the kernels with the
        coefficients on the lanes and chunks of 8 right-hand sides.  Applies to
        the autotuned schedules too (it overrides their choice; the autotuner
-       tries 1 and 2 for 2-31 right-hand sides, 1 and 0 from 32).  No reference
+       tries 1 and 0 where 1 takes these kernels, 1 and 2 below).  No reference
        counterpart. */
     HM_OPT_WIDE_TREE = 9,
     /* HM_OPT_RING_TILE (default 0): the per-warp rings' tile for 3-8 FP32
@@ -305,7 +307,7 @@ int hm_configure(hm_handle *h, int option, int64_t value);
    (0..1 above 8 right-hand sides), HM_OPT_NEAR_KERNEL 0 (with each of the
    three ring tiles for 3-8 FP32 right-hand sides), 1 (FP32 with 3-8
    right-hand sides) or 2 with HM_OPT_NEAR_STAGES 3, 4 or 6 (up to 8
-   right-hand sides), HM_OPT_WIDE_TREE on or off (32 or more),
+   right-hand sides), HM_OPT_WIDE_TREE on or off,
    HM_OPT_TENSOR_CORES
    on or off (FP32, 16 or more), HM_OPT_PDL on or off.  Inputs are scratch vectors allocated on
    `stream` and freed before return; synchronous; not allowed while `stream`
