@@ -66,85 +66,26 @@ __device__ __forceinline__ const T *stack_col(const void *X1, int64_t ld1, int k
     return l < k1 ? static_cast<const T *>(X1) + ld1 * l : static_cast<const T *>(X2) + ld2 * (l - k1);
 }
 
-// Householder QR of the m x k panel A (ld m) in place, LAPACK xGEQR2
-// conventions: H_j = I - tau_j v v^T with v_j = 1 and v below the diagonal of
-// column j, beta = -sign(alpha) ||(alpha, x)||, R in the upper triangle.
-template <typename T>
-__device__ void house_qr(T *A, int64_t m, int k, T *tau)
-{
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int kk = (int)(m < k ? m : k);
-    for (int j = 0; j < kk; ++j) {
-        T *x = A + m * j;
-        if (warp == j % kWarps) {
-            T ss = 0;
-            for (int64_t i = j + 1 + lane; i < m; i += 32) ss = fma(x[i], x[i], ss);
-            ss = warp_sum(ss);
-            const T alpha = x[j];
-            T t = 0;
-            if (ss != T(0)) {
-                const T beta = -copysign(sqrt(fma(alpha, alpha, ss)), alpha);
-                t = (beta - alpha) / beta;
-                const T sc = T(1) / (alpha - beta);
-                for (int64_t i = j + 1 + lane; i < m; i += 32) x[i] *= sc;
-                __syncwarp();
-                if (lane == 0) x[j] = beta;
-            }
-            if (lane == 0) tau[j] = t;
-        }
-        __syncthreads();
-        const T tj = tau[j];
-        if (tj != T(0)) {
-            for (int c = warp; c < k; c += kWarps) {
-                if (c <= j) continue;
-                T *y = A + m * c;
-                const T yj = y[j];
-                T w = 0;
-                for (int64_t i = j + 1 + lane; i < m; i += 32) w = fma(x[i], y[i], w);
-                w = tj * (warp_sum(w) + yj);
-                __syncwarp();
-                if (lane == 0) y[j] = yj - w;
-                for (int64_t i = j + 1 + lane; i < m; i += 32) y[i] = fma(-w, x[i], y[i]);
-            }
-        }
-        __syncthreads();
-    }
-}
+// GB300 issues an FP64 warp instruction every 64 cycles per sub-partition, with one
+// lane live or 32, so the small factorisations below count FP64 instructions: the
+// library's divide and square root (some 20 each) are replaced by an FP32 estimate
+// refined in FP64, sums over few rows run several columns per warp, and values
+// move between the formats by their bits.
 
-// y <- Q y = H_0 H_1 ... H_{kk-1} y for one column y (length m) by one warp.
-template <typename T>
-__device__ void apply_q(const T *A, int64_t m, int kk, const T *tau, T *y)
-{
-    const int lane = threadIdx.x & 31;
-    for (int j = kk - 1; j >= 0; --j) {
-        const T tj = tau[j];
-        if (tj == T(0)) continue;
-        const T *x = A + m * j;
-        const T yj = y[j];
-        T w = 0;
-        for (int64_t i = j + 1 + lane; i < m; i += 32) w = fma(x[i], y[i], w);
-        w = tj * (warp_sum(w) + yj);
-        __syncwarp();
-        if (lane == 0) y[j] = yj - w;
-        for (int64_t i = j + 1 + lane; i < m; i += 32) y[i] = fma(-w, x[i], y[i]);
-        __syncwarp();
-    }
-}
-
-// The Jacobi rotation of lr_svd: t = tan(theta) is the smaller root of
-// t^2 + 2 zeta t - 1 = 0, zeta = (be - al) / (2 ga), i.e.
-// |t| = |g| / (|a| + sqrt(a^2 + g^2)) with a = be - al, g = 2 ga and the sign
-// of a g.  t is formed in FP32 (FP64 issue time is scarce on GB300): from a
-// and g scaled by a common power of two when |g| >= 2^-30 |a|, else as
-// t = g / (2a) from the two mantissas with the exponents applied apart
-// (strongly graded columns give angles far below FP32's range).  Its
-// relative error, about 1e-7, only leaves an inner product of that relative
-// size for the next sweep.  c = (1 + t^2)^(-1/2) is then refined in T from
-// the FP32 estimate, so c^2 + s^2 = 1 to T's rounding and
-// every rotation is orthogonal in T (c by one Halley step from the FP32
-// estimate).  Returns false when t underflows.
+// exponent (unbiased; zero and subnormal -1023) and signed mantissa, +-[1, 2)
 __device__ __forceinline__ int exponent_of(double x) { return ((__double2hiint(x) >> 20) & 0x7ff) - 1023; }
 __device__ __forceinline__ int exponent_of(float x) { return ((__float_as_int(x) >> 23) & 0xff) - 127; }
+__device__ __forceinline__ float mantissa_of(double x)
+{
+    const int hi = __double2hiint(x);
+    return __int_as_float((hi & 0x80000000) | (127 << 23) | ((hi & 0xfffff) << 3) | ((unsigned)__double2loint(x) >> 29));
+}
+// x 2^e for a normal float x and a result in double's normal range
+__device__ __forceinline__ double widen(float x, int e)
+{
+    const int b = __float_as_int(x);
+    return __hiloint2double((b & 0x80000000) | ((((b >> 23) & 0xff) - 127 + 1023 + e) << 20) | ((b >> 3) & 0xfffff), b << 29);
+}
 template <typename T> __device__ __forceinline__ T pow2(int e);
 template <> __device__ __forceinline__ double pow2<double>(int e)
 {
@@ -157,29 +98,13 @@ template <> __device__ __forceinline__ float pow2<float>(int e)
     return __int_as_float((127 + e) << 23);
 }
 
-template <typename T>
-__device__ __forceinline__ bool jacobi_tangent(T al, T be, T ga, T &t)
-{
-    const T a = be - al, g = ga + ga;
-    const int ea = a == T(0) ? -100000 : exponent_of(a), eg = exponent_of(g);
-    if (eg < ea - 30) {
-        const float am = (float)(a * pow2<T>(-ea)), gm = (float)(g * pow2<T>(-eg));
-        if (eg - ea < (sizeof(T) == 8 ? -1000 : -120)) return false;     // t below T's normal range
-        t = (T)(gm / (am + am)) * pow2<T>(eg - ea);
-    } else {
-        const int e = ea > eg ? ea : eg;
-        const T sc = pow2<T>(-e);
-        const float af = (float)(a * sc), gf = (float)(g * sc);
-        float t32 = fabsf(gf) / (fabsf(af) + sqrtf(fmaf(af, af, gf * gf)));
-        if ((af < 0.f) != (gf < 0.f)) t32 = -t32;
-        t = (T)t32;
-    }
-    return t != T(0);
-}
+// x != 0 without the FP64 pipe (a compare there costs as much as an FMA)
+__device__ __forceinline__ bool nonzero(double x) { return ((__double2hiint(x) & 0x7fffffff) | __double2loint(x)) != 0; }
+__device__ __forceinline__ bool nonzero(float x) { return x != 0.f; }
 
 // d^(-1/2) for d > 0 from the FP32 estimate refined by Halley's iteration;
 // d outside FP32's range is first scaled to m in [1, 4) by an even power of
-// two.  (Subnormal d: the library square root.)
+// two.  (d near double's smallest: the library square root.)
 __device__ __forceinline__ double rsqrt_halley(double d, double y0)
 {
     // one step of Halley's iteration for d^(-1/2): with e = 1 - d y0^2,
@@ -190,12 +115,14 @@ __device__ __forceinline__ double rsqrt_halley(double d, double y0)
 }
 __device__ __forceinline__ double rsqrt_pos(double d)
 {
-    if (d > 1e-30 && d < 1e30) return rsqrt_halley(d, (double)rsqrtf((float)d));
-    if (d < 1e-300) return 1.0 / sqrt(d);
     int e = exponent_of(d);
-    e -= e & 1;
-    const double m = d * pow2<double>(-e);
-    return rsqrt_halley(m, (double)rsqrtf((float)m)) * pow2<double>(-e / 2);
+    if (e < -1000) return 1.0 / sqrt(d);
+    const float m = mantissa_of(d);
+    if (e > -100 && e < 100) return rsqrt_halley(d, widen(rsqrtf(m * pow2<float>(e)), 0));
+    const int odd = e & 1;
+    e -= odd;
+    const double md = d * pow2<double>(-e);
+    return rsqrt_halley(md, widen(rsqrtf(odd ? m + m : m), 0)) * pow2<double>(-e / 2);
 }
 __device__ __forceinline__ float rsqrt_pos(float d)
 {
@@ -204,23 +131,296 @@ __device__ __forceinline__ float rsqrt_pos(float d)
     return y * fmaf(-0.5f * d, y * y, 1.5f);
 }
 
-template <typename T>
-__device__ __forceinline__ bool jacobi_rotation(T al, T be, T ga, T &c, T &s)
+// s = d^(1/2) and y = d^(-1/2) for d > 0: the estimate's residual corrects s
+__device__ __forceinline__ void sqrt_both(double d, double &s, double &y)
 {
-    T t;
-    if (!jacobi_tangent(al, be, ga, t)) return false;
-    const float tf = (float)t;
-    const T u = fma(t, t, T(1));
-    const T c0 = (T)rsqrtf(fmaf(tf, tf, 1.f));
-    T cc;
-    if constexpr (sizeof(T) == 8) {
-        cc = rsqrt_halley(u, c0);
-    } else {
-        cc = c0 * fmaf(-0.5f * u, c0 * c0, 1.5f);
+    if (exponent_of(d) == 1024) {                              // inf, NaN
+        s = sqrt(d);
+        y = 1.0 / s;
+        return;
     }
-    c = cc;
-    s = cc * t;
+    y = rsqrt_pos(d);
+    const double s0 = d * y;
+    s = fma(0.5 * y, fma(-s0, s0, d), s0);
+}
+__device__ __forceinline__ void sqrt_both(float d, float &s, float &y)
+{
+    s = sqrtf(d);
+    y = 1.f / s;
+}
+
+// 1 / d: the FP32 reciprocal of d's mantissa and one step of the third-order
+// (Householder) iteration, y = y0 (1 + e + e^2), e = 1 - d y0, which leaves e^3 <
+// 2^-66.  Exponents near the ends of double's range: the division.
+__device__ __forceinline__ double recip(double d)
+{
+    const int e = exponent_of(d);
+    if (e < -1000 || e > 1000) return 1.0 / d;
+    const double y0 = widen(1.f / mantissa_of(d), -e);
+    const double r = fma(-d, y0, 1.0);
+    return fma(y0, fma(r, r, r), y0);
+}
+__device__ __forceinline__ float recip(float d) { return 1.f / d; }
+
+// Sum over the aligned group of G lanes.
+template <typename T>
+__device__ __forceinline__ T group_sum(T v, int G)
+{
+    for (int o = G >> 1; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+__device__ __forceinline__ void warps_barrier(int id, int nw)
+{
+    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nw * 32) : "memory");
+}
+
+// sum of x[i] y[i], i = i0, i0 + G, ... < m, in four chains (a dependent FP64 FMA
+// takes about 100 cycles)
+template <typename T>
+__device__ __forceinline__ T strided_dot(const T *x, const T *y, int64_t i0, int64_t m, int G)
+{
+    T a0 = 0, a1 = 0, a2 = 0, a3 = 0;
+    int64_t i = i0;
+    for (; i + 3 * G < m; i += 4 * G) {
+        a0 = fma(x[i], y[i], a0);
+        a1 = fma(x[i + G], y[i + G], a1);
+        a2 = fma(x[i + 2 * G], y[i + 2 * G], a2);
+        a3 = fma(x[i + 3 * G], y[i + 3 * G], a3);
+    }
+    if (i < m) a0 = fma(x[i], y[i], a0);
+    if (i + G < m) a1 = fma(x[i + G], y[i + G], a1);
+    if (i + 2 * G < m) a2 = fma(x[i + 2 * G], y[i + 2 * G], a2);
+    return (a0 + a1) + (a2 + a3);
+}
+
+// Householder QR of the m x k panel A (ld) in place by nw warps, this one
+// `warp` of them (barrier `bar`; ss: a shared value of theirs), LAPACK xGEQR2 conventions: H_j = I -
+// tau_j v v^T with v_j = 1 and v below the diagonal of column j, beta = -sign(alpha)
+// ||(alpha, x)||, R in the upper triangle.  tau: 2 k values (the scales of v after
+// the taus).  A column belongs to a group of G lanes.  Bound by the chain of dependent
+// FP64 operations of a step, so the products x . y_c and x . x run side by side on the
+// unscaled x (v = x / (alpha - beta)), every warp with columns forms the reflector's
+// scalars itself, and the columns are scaled at the end.  64 x 10 and 64 x 10 at once
+// 63 -> 15 us (one after the other, reflector by one warp, in global memory, with the
+// library's divide and square root).
+template <typename T>
+__device__ void house_qr(T *A, int64_t ld, int64_t m, int k, T *tau, T *ss, int warp, int nw, int bar, bool local)
+{
+    const int lane = threadIdx.x & 31;
+    const int kk = (int)(m < k ? m : k);
+    const int G = local ? 8 : 32;
+    const int lg = lane & (G - 1), grp = lane / G, cpw = 32 / G;
+    for (int j = 0; j < kk; ++j) {
+        T *x = A + ld * j;
+        const int cb = j + warp * cpw;                     // this warp's first columns, column j among them
+        const bool busy = cb < k;
+        T alpha = 0, w = 0;
+        if (busy) {
+            const int c = cb + grp < k ? cb + grp : j;
+            alpha = x[j];
+            w = group_sum(strided_dot(x, A + ld * c, j + 1 + lg, m, G), G);
+            if (cb == j && lane == 0) *ss = w;
+        }
+        warps_barrier(bar, nw);
+        if (busy) {
+            const T sq = *ss;
+            T t = 0, sc = 1, beta = alpha;
+            if (nonzero(sq)) {
+                T nrm, inv;
+                sqrt_both(fma(alpha, alpha, sq), nrm, inv);
+                beta = -copysign(nrm, alpha);
+                t = (alpha - beta) * copysign(inv, alpha);              // (beta - alpha) / beta
+                sc = recip(alpha - beta);
+            }
+            if (cb == j && lane == 0) {
+                x[j] = beta;
+                tau[j] = t;
+                tau[k + j] = sc;
+            }
+            if (nonzero(t)) {
+                for (int b = cb; b < k; b += nw * cpw) {               // warp-uniform
+                    const int c = b + grp;
+                    const bool live = c < k && c > j;
+                    T *y = A + ld * (c < k ? c : k - 1);
+                    if (b != cb) w = group_sum(strided_dot(x, y, j + 1 + lg, m, G), G);
+                    if (live) {
+                        const T yj = y[j], f = t * fma(w, sc, yj), fs = f * sc;
+                        __syncwarp(__activemask());
+                        if (lg == 0) y[j] = yj - f;
+                        for (int64_t i = j + 1 + lg; i < m; i += G) y[i] = fma(-fs, x[i], y[i]);
+                    }
+                    __syncwarp();
+                }
+            }
+        }
+        warps_barrier(bar, nw);
+    }
+    for (int j = warp; j < kk; j += nw) {
+        const T sc = tau[k + j];
+        for (int64_t i = j + 1 + lane; i < m; i += 32) A[i + ld * j] *= sc;
+    }
+    warps_barrier(bar, nw);
+}
+
+// y <- Q y = H_0 H_1 ... H_{kk-1} y for one column y (length m) by one warp.
+template <typename T>
+__device__ void apply_q(const T *A, int64_t ld, int64_t m, int kk, const T *tau, T *y)
+{
+    const int lane = threadIdx.x & 31;
+    for (int j = kk - 1; j >= 0; --j) {
+        const T tj = tau[j];
+        if (!nonzero(tj)) continue;
+        const T *x = A + ld * j;
+        const T yj = y[j];
+        T w = 0;
+        for (int64_t i = j + 1 + lane; i < m; i += 32) w = fma(x[i], y[i], w);
+        w = tj * (warp_sum(w) + yj);
+        __syncwarp();
+        if (lane == 0) y[j] = yj - w;
+        for (int64_t i = j + 1 + lane; i < m; i += 32) y[i] = fma(-w, x[i], y[i]);
+        __syncwarp();
+    }
+}
+
+// The same for m <= G RPL rows in registers, a column per group of G lanes: lane
+// lg holds rows lg + G u.  Called by whole warps.
+template <typename T, int RPL>
+__device__ __forceinline__ void apply_q_regs(const T *A, int64_t ld, int m, int kk, const T *tau, int G, int lg, T (&y)[RPL])
+{
+    for (int j = kk - 1; j >= 0; --j) {
+        const T tj = tau[j];
+        if (!nonzero(tj)) continue;
+        const T *x = A + ld * j;
+        T v[RPL], w = 0;
+#pragma unroll
+        for (int u = 0; u < RPL; ++u) {
+            const int i = lg + G * u;
+            v[u] = i > j && i < m ? x[i] : (i == j ? T(1) : T(0));
+            w = fma(v[u], y[u], w);
+        }
+        w = tj * group_sum(w, G);
+#pragma unroll
+        for (int u = 0; u < RPL; ++u) y[u] = fma(-w, v[u], y[u]);
+    }
+}
+
+// Columns c0, c0 + 32 / G cstep's worth ... of out = Q in: `in(c, i)` is row i of
+// column c before, `out(c, i, v)` takes row i after; ncol columns over nw warps.
+template <typename T, int RPL, typename In, typename Out>
+__device__ void apply_q_cols(const T *A, int64_t ld, int m, int kk, const T *tau, int G, int ncol, int warp, int nw,
+                             In in, Out out)
+{
+    const int lane = threadIdx.x & 31, lg = lane & (G - 1), grp = lane / G, cpw = 32 / G;
+    for (int cb = warp * cpw; cb < ncol; cb += nw * cpw) {
+        const int c = cb + grp;
+        const bool live = c < ncol;
+        T y[RPL];
+#pragma unroll
+        for (int u = 0; u < RPL; ++u) {
+            const int i = lg + G * u;
+            y[u] = live && i < m ? in(c, i) : T(0);
+        }
+        apply_q_regs<T, RPL>(A, ld, m, kk, tau, G, lg, y);
+#pragma unroll
+        for (int u = 0; u < RPL; ++u) {
+            const int i = lg + G * u;
+            if (live && i < m) out(c, i, y[u]);
+        }
+    }
+}
+constexpr int kRegRows = 256;          // rows apply_q_any keeps in registers (8 a lane)
+template <typename T, typename In, typename Out>
+__device__ void apply_q_any(const T *A, int64_t ld, int m, int kk, const T *tau, int ncol, int warp, int nw, In in, Out out)
+{
+    if (m <= 16) apply_q_cols<T, 2>(A, ld, m, kk, tau, 8, ncol, warp, nw, in, out);
+    else if (m <= 32) apply_q_cols<T, 4>(A, ld, m, kk, tau, 8, ncol, warp, nw, in, out);
+    else apply_q_cols<T, 8>(A, ld, m, kk, tau, m <= 64 ? 8 : m <= 128 ? 16 : 32, ncol, warp, nw, in, out);
+}
+
+// The Jacobi rotation of lr_svd: t = tan(theta) is the smaller root of
+// t^2 + 2 zeta t - 1 = 0, zeta = (be - al) / (2 ga), i.e.
+// |t| = |g| / (|a| + sqrt(a^2 + g^2)) with a = be - al, g = 2 ga and the sign
+// of a g.  t is formed in FP32: from a
+// and g scaled by a common power of two when |g| >= 2^-30 |a|, else as
+// t = g / (2a) from the two mantissas with the exponents applied apart
+// (strongly graded columns give angles far below FP32's range).  Its
+// relative error, about 1e-7, only leaves an inner product of that relative
+// size for the next sweep.  c = (1 + t^2)^(-1/2) is then refined in T from
+// the FP32 estimate, so c^2 + s^2 = 1 to T's rounding and
+// every rotation is orthogonal in T (c by one Halley step from the FP32
+// estimate).  Returns false when t underflows.
+// Columns whose cosine is below T's rounding are not rotated; that test, too, works on
+// exponents and FP32 mantissas.
+__device__ __forceinline__ bool jacobi_rotation(double al, double be, double ga, double &c, double &s)
+{
+    const int ka = exponent_of(al), kb = exponent_of(be), kg = exponent_of(ga);
+    if (ka == -1023 || kb == -1023 || kg == -1023 || ka == 1024 || kb == 1024 || kg == 1024) return false;
+    const float mg = mantissa_of(ga);
+    // ga^2 > 2^-104 al be
+    const int d = 2 * kg - ka - kb + 104;
+    if (d < -2 || (d <= 2 && !(mg * mg * pow2<float>(d) > mantissa_of(al) * mantissa_of(be)))) return false;
+    const double a = be - al;
+    const int ea = exponent_of(a), eg = kg + 1;            // g = 2 ga
+    float am = mantissa_of(a), tf;
+    if (ea == -1023) am = 0.f;
+    double t;
+    if (am != 0.f && eg < ea - 30) {
+        if (eg - ea < -1000) return false;                 // t below the normal range
+        tf = mg / (am + am);
+        t = widen(tf, eg - ea);
+        tf = 0.f;                                          // c rounds to 1
+    } else {
+        const int e = am != 0.f && ea > eg ? ea : eg;
+        const float af = am != 0.f && ea - e > -120 ? am * pow2<float>(ea - e) : 0.f, gf = mg * pow2<float>(eg - e);
+        tf = fabsf(gf) / (fabsf(af) + sqrtf(fmaf(af, af, gf * gf)));
+        if ((af < 0.f) != (gf < 0.f)) tf = -tf;
+        t = widen(tf, 0);
+    }
+    const double u = fma(t, t, 1.0);
+    c = rsqrt_halley(u, widen(rsqrtf(fmaf(tf, tf, 1.f)), 0));
+    s = c * t;
     return true;
+}
+__device__ __forceinline__ bool jacobi_rotation(float al, float be, float ga, float &c, float &s)
+{
+    constexpr float eps2 = Lim<float>::eps * Lim<float>::eps;
+    if (al == 0.f || be == 0.f || !(ga * ga > eps2 * al * be)) return false;
+    const float a = be - al, g = ga + ga;
+    const int ea = a == 0.f ? -100000 : exponent_of(a), eg = exponent_of(g);
+    float t;
+    if (eg < ea - 30) {
+        const float am = a * pow2<float>(-ea), gm = g * pow2<float>(-eg);
+        if (eg - ea < -120) return false;                  // t below the normal range
+        t = gm / (am + am) * pow2<float>(eg - ea);
+    } else {
+        const int e = ea > eg ? ea : eg;
+        const float sc = pow2<float>(-e), af = a * sc, gf = g * sc;
+        t = fabsf(gf) / (fabsf(af) + sqrtf(fmaf(af, af, gf * gf)));
+        if ((af < 0.f) != (gf < 0.f)) t = -t;
+    }
+    if (t == 0.f) return false;
+    const float u = fmaf(t, t, 1.f), c0 = rsqrtf(u);
+    c = c0 * fmaf(-0.5f * u, c0 * c0, 1.5f);
+    s = c * t;
+    return true;
+}
+
+// The sums of al, be and ga over an aligned group of G (8 to 32) lanes, in every
+// lane: after one step the lanes hold al or be by turns, after two al, be, ga, ga,
+// so the three sums take log2 G + 1 additions instead of 3 log2 G.
+template <typename T>
+__device__ __forceinline__ void group_sum3(T &al, T &be, T &ga, int G, int lane)
+{
+    const bool b0 = lane & 1, b1 = lane & 2;
+    const T x = (b0 ? be : al) + __shfl_xor_sync(0xffffffffu, b0 ? al : be, 1);
+    const T g = ga + __shfl_xor_sync(0xffffffffu, ga, 1);
+    T r = (b1 ? g : x) + __shfl_xor_sync(0xffffffffu, b1 ? x : g, 2);
+    for (int o = 4; o < G; o <<= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
+    const int base = lane & ~(G - 1);
+    al = __shfl_sync(0xffffffffu, r, base);
+    be = __shfl_sync(0xffffffffu, r, base + 1);
+    ga = __shfl_sync(0xffffffffu, r, base + 2);
 }
 
 // One problem of lr_svd as the kernel reads it: the public descriptor and,
@@ -236,6 +436,16 @@ struct LrJob {
     int64_t ldm2;
 };
 
+// Rows between the columns of a panel in shared memory: four groups of 8 lanes
+// reading four columns then meet no bank twice (8 mod 16 doubles).
+__host__ __device__ inline int64_t lr_panel_ld(int64_t m) { return (m + 7) / 16 * 16 + 8; }
+// Values of a problem's panels and reflector scales there.
+__host__ __device__ inline int64_t lr_panel_vals(const hm_lr_problem &p)
+{
+    const int64_t a = p.a1 + p.a2, b = p.b1 + p.b2;
+    return (p.qr_left ? lr_panel_ld(p.m) * a : 0) + (p.qr_right ? lr_panel_ld(p.n) * b : 0) + 2 * (a + b);
+}
+
 // Core storage of lr_svd: D (p x q core, ld p), then J (q x q right
 // rotations, before that the staging area of the Xm^T Ym product), sigma (q)
 // and the sort order (q ints).  In shared memory (D takes d_elems values)
@@ -243,7 +453,7 @@ struct LrJob {
 template <typename T>
 __global__ void __launch_bounds__(kThreads) lr_svd_kernel(const LrJob *jobs, const int64_t *ws_off,
                                                           const int64_t *core_off, T *ws, int *ranks, int64_t d_elems,
-                                                          int64_t xoff)
+                                                          int64_t xoff, int64_t soff, int64_t scap)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const hm_lr_problem pr = jobs[blockIdx.x].p;
@@ -257,35 +467,47 @@ __global__ void __launch_bounds__(kThreads) lr_svd_kernel(const LrJob *jobs, con
     const bool tr = kb > ka;
     const int p = tr ? kb : ka, q = tr ? ka : kb;
     __shared__ int s_flag, s_rank;
-    __shared__ T s_scale, s_unscale;
+    __shared__ T s_scale, s_unscale, s_ss[2];
     if (q == 0) {
         if (tid == 0) ranks[blockIdx.x] = 0;
         return;
     }
-    T *WP = ws + ws_off[blockIdx.x];
-    T *WQ = WP + (pr.qr_left ? m * a : 0);
-    T *tauP = WQ + (pr.qr_right ? n * b : 0);
-    T *tauQ = tauP + a;
+    // the panels: in shared memory where they fit, else in the workspace
+    const bool local = (pr.qr_left || pr.qr_right) && lr_panel_vals(pr) <= scap;
+    const int64_t ldP = local ? lr_panel_ld(m) : m, ldQ = local ? lr_panel_ld(n) : n;
+    T *WP = local ? reinterpret_cast<T *>(smem_raw) + soff : ws + ws_off[blockIdx.x];
+    T *WQ = WP + (pr.qr_left ? ldP * a : 0);
+    T *tauP = WQ + (pr.qr_right ? ldQ * b : 0);
+    T *tauQ = tauP + 2 * a;
     const int64_t co = core_off[blockIdx.x];
     T *D = co < 0 ? reinterpret_cast<T *>(smem_raw) : ws + co;
     T *J = D + (co < 0 ? d_elems : (int64_t)p * q);
 
-    // 1. orthonormalise the factors that the operation orthonormalises
-    if (pr.qr_left) {
+    // 1. orthonormalise the factors that the operation orthonormalises: both at the
+    //    same time, by half of the warps each
+    if (pr.qr_left)
         for (int64_t e = tid; e < m * a; e += kThreads) {
             const int l = (int)(e / m);
-            WP[e] = stack_col<T>(pr.P1, pr.ldp1, pr.a1, pr.P2, pr.ldp2, l)[e - m * l];
+            const int64_t i = e - m * l;
+            WP[i + ldP * l] = stack_col<T>(pr.P1, pr.ldp1, pr.a1, pr.P2, pr.ldp2, l)[i];
         }
-        __syncthreads();
-        house_qr(WP, m, a, tauP);
-    }
-    if (pr.qr_right) {
+    if (pr.qr_right)
         for (int64_t e = tid; e < n * b; e += kThreads) {
             const int l = (int)(e / n);
-            WQ[e] = stack_col<T>(pr.Q1, pr.ldq1, pr.b1, pr.Q2, pr.ldq2, l)[e - n * l];
+            const int64_t i = e - n * l;
+            WQ[i + ldQ * l] = stack_col<T>(pr.Q1, pr.ldq1, pr.b1, pr.Q2, pr.ldq2, l)[i];
         }
+    __syncthreads();
+    if (pr.qr_left && pr.qr_right) {
+        // (warps 0, 1, 4, 5 and 2, 3, 6, 7: two sub-partitions each)
+        const int hw = (warp & 1) + (warp >> 2) * 2;
+        if (!(warp & 2)) house_qr(WP, ldP, m, a, tauP, s_ss, hw, kWarps / 2, 1, local);
+        else house_qr(WQ, ldQ, n, b, tauQ, s_ss + 1, hw, kWarps / 2, 2, local);
         __syncthreads();
-        house_qr(WQ, n, b, tauQ);
+    } else if (pr.qr_left) {
+        house_qr(WP, ldP, m, a, tauP, s_ss, warp, kWarps, 0, local);
+    } else if (pr.qr_right) {
+        house_qr(WQ, ldQ, n, b, tauQ, s_ss, warp, kWarps, 0, local);
     }
 
     // 2. the core C (ka x kb), stored as D = C (p = ka) or D = C^T (p = kb)
@@ -329,10 +551,10 @@ __global__ void __launch_bounds__(kThreads) lr_svd_kernel(const LrJob *jobs, con
             const int i = e % ka, l2 = e / ka;
             T acc = 0;
             if (l2 < pr.a1) {
-                if (l2 >= i) acc = WP[i + m * l2] * s1[l2];
+                if (l2 >= i) acc = WP[i + ldP * l2] * s1[l2];
             } else {
                 for (int l = i > pr.a1 ? i : pr.a1; l < a; ++l)
-                    acc = fma(WP[i + m * l], M2[(l - pr.a1) + ldm2 * (l2 - pr.a1)], acc);
+                    acc = fma(WP[i + ldP * l], M2[(l - pr.a1) + ldm2 * (l2 - pr.a1)], acc);
                 acc *= sign2;
             }
             Tm[e] = acc;
@@ -341,7 +563,7 @@ __global__ void __launch_bounds__(kThreads) lr_svd_kernel(const LrJob *jobs, con
         for (int e = tid; e < ka * kb; e += kThreads) {
             const int i = e % ka, j = e / ka;
             T acc = 0;
-            for (int l2 = j; l2 < b; ++l2) acc = fma(Tm[i + ka * l2], WQ[j + n * l2], acc);
+            for (int l2 = j; l2 < b; ++l2) acc = fma(Tm[i + ka * l2], WQ[j + ldQ * l2], acc);
             D[didx(i, j)] = acc;
         }
         __syncthreads();                                   // Tm is read before J is written
@@ -355,13 +577,13 @@ __global__ void __launch_bounds__(kThreads) lr_svd_kernel(const LrJob *jobs, con
             if (!pr.qr_left && !pr.qr_right) {
                 if (i == j) acc = i < pr.a1 ? s1[i] : sign2 * s2[i - pr.a1];
             } else if (!pr.qr_left) {                  // C(i, j) = sd_i R_Q(j, i)
-                if (i >= j) acc = (i < pr.a1 ? s1[i] : sign2 * s2[i - pr.a1]) * WQ[j + n * i];
+                if (i >= j) acc = (i < pr.a1 ? s1[i] : sign2 * s2[i - pr.a1]) * WQ[j + ldQ * i];
             } else if (!pr.qr_right) {                 // C(i, j) = R_P(i, j) sd_j
-                if (j >= i) acc = WP[i + m * j] * (j < pr.a1 ? s1[j] : sign2 * s2[j - pr.a1]);
+                if (j >= i) acc = WP[i + ldP * j] * (j < pr.a1 ? s1[j] : sign2 * s2[j - pr.a1]);
             } else {
                 for (int l = i > j ? i : j; l < a; ++l) {
                     const T sd = l < pr.a1 ? s1[l] : sign2 * s2[l - pr.a1];
-                    acc = fma(WP[i + m * l] * sd, WQ[j + n * l], acc);
+                    acc = fma(WP[i + ldP * l] * sd, WQ[j + ldQ * l], acc);
                 }
             }
             D[didx(i, j)] = acc;
@@ -409,8 +631,8 @@ __global__ void __launch_bounds__(kThreads) lr_svd_kernel(const LrJob *jobs, con
     if (pre) {
         Xs = reinterpret_cast<T *>(smem_raw) + xoff;   // q x q
         Lf = Xs + (int64_t)q * q;                      // p x q
-        tq = Lf + (int64_t)p * q;                      // q
-        house_qr(D, (int64_t)p, q, tq);
+        tq = Lf + (int64_t)p * q;                      // 2 q
+        house_qr(D, (int64_t)p, (int64_t)p, q, tq, s_ss, warp, kWarps, 0, true);
         for (int e = tid; e < q * q; e += kThreads) {
             const int i = e % q, j = e / q;
             Xs[e] = i >= j ? D[j + (int64_t)p * i] : T(0);
@@ -420,9 +642,9 @@ __global__ void __launch_bounds__(kThreads) lr_svd_kernel(const LrJob *jobs, con
     T *const Dj = pre ? Xs : D;
     const int pj = pre ? q : p;
     const int qq = (q + 1) & ~1, npairs = qq / 2;
-    const int G = pj <= 32 ? 8 : (pj <= 64 ? 16 : 32);
+    // (16 rows and fewer: 16 lanes, still at most one warp per sub-partition)
+    const int G = pj <= 16 ? 16 : pj <= 32 ? 8 : (pj <= 64 ? 16 : 32);
     const int gpw = 32 / G, lg = lane & (G - 1), grp = lane / G;
-    const T eps2 = Lim<T>::eps * Lim<T>::eps;
     for (int sweep = 0; sweep < kJacobiSweeps; ++sweep) {
         if (tid == 0) s_flag = 0;
         __syncthreads();
@@ -443,14 +665,9 @@ __global__ void __launch_bounds__(kThreads) lr_svd_kernel(const LrJob *jobs, con
                         const T u = di[r], v = dj[r];
                         al = fma(u, u, al); be = fma(v, v, be); ga = fma(u, v, ga);
                     }
-                for (int o = G >> 1; o; o >>= 1) {              // within the aligned group of G lanes
-                    al += __shfl_xor_sync(0xffffffffu, al, o);
-                    be += __shfl_xor_sync(0xffffffffu, be, o);
-                    ga += __shfl_xor_sync(0xffffffffu, ga, o);
-                }
-                if (!live || al == T(0) || be == T(0) || !(ga * ga > eps2 * al * be)) continue;
+                group_sum3(al, be, ga, G, lane);
                 T c, sn;
-                if (!jacobi_rotation(al, be, ga, c, sn)) continue;
+                if (!live || !jacobi_rotation(al, be, ga, c, sn)) continue;
                 for (int r = lg; r < pj; r += G) {
                     const T u = di[r], v = dj[r];
                     di[r] = c * u - sn * v;
@@ -473,41 +690,61 @@ __global__ void __launch_bounds__(kThreads) lr_svd_kernel(const LrJob *jobs, con
     if (pre) {
         // D's columns become Q [J_j; 0] sigma_j (sigma_j = |X_j|) and J's X_j / sigma_j,
         // the form the unpreconditioned sweeps leave
-        for (int j = warp; j < q; j += kWarps) {
-            const T *xj = Xs + (int64_t)q * j;
-            T ss = 0;
-            for (int r = lane; r < q; r += 32) ss = fma(xj[r], xj[r], ss);
-            const T sgm = sqrt(warp_sum(ss));
-            T *y = Lf + (int64_t)p * j;
-            T *jc = J + (int64_t)q * j;
-            for (int i = lane; i < p; i += 32) y[i] = i < q ? jc[i] : T(0);
-            __syncwarp();
-            apply_q(D, (int64_t)p, q, tq, y);
-            for (int i = lane; i < p; i += 32) y[i] *= sgm;
-            const T inv = sgm > T(0) ? T(1) / sgm : T(0);
-            for (int r = lane; r < q; r += 32) jc[r] = sgm > T(0) ? xj[r] * inv : (r == j ? T(1) : T(0));
-        }
+        const bool regs = p <= kRegRows;
+        if (regs)
+            apply_q_any<T>(D, (int64_t)p, p, q, tq, q, warp, kWarps,
+                           [&](int j, int i) { return i < q ? J[i + (int64_t)q * j] : T(0); },
+                           [&](int j, int i, T v) { Lf[i + (int64_t)p * j] = v; });
+        else
+            for (int j = warp; j < q; j += kWarps) {
+                T *y = Lf + (int64_t)p * j;
+                for (int i = lane; i < p; i += 32) y[i] = i < q ? J[i + (int64_t)q * j] : T(0);
+                __syncwarp();
+                apply_q(D, (int64_t)p, (int64_t)p, q, tq, y);
+            }
         __syncthreads();
-        for (int e = tid; e < p * q; e += kThreads) D[e] = Lf[e];
+        for (int jb = warp * 4; jb < q; jb += kWarps * 4) {        // 8 lanes a column
+            const int j = jb + (lane >> 3), l8 = lane & 7;
+            const bool live = j < q;
+            const T *xj = Xs + (int64_t)q * (live ? j : jb);
+            T ss = 0;
+            for (int r = l8; r < q; r += 8) ss = fma(xj[r], xj[r], ss);
+            ss = group_sum(ss, 8);
+            T sgm = 0, inv = 0;
+            if (ss > T(0)) sqrt_both(ss, sgm, inv);
+            else sgm = ss;                                         // 0, or NaN as it came
+            if (live) {
+                T *y = Lf + (int64_t)p * j, *jc = J + (int64_t)q * j;
+                for (int i = l8; i < p; i += 8) y[i] *= sgm;
+                for (int r = l8; r < q; r += 8) jc[r] = sgm > T(0) ? xj[r] * inv : (r == j ? T(1) : T(0));
+            }
+        }
+        D = Lf;
         __syncthreads();
     }
 
     // 4. singular values, descending order, getrank
     T *sig = J + (int64_t)q * q;
     int *perm = reinterpret_cast<int *>(sig + q);
-    for (int j = warp; j < q; j += kWarps) {
-        T *dj = D + (int64_t)p * j, *jj = J + (int64_t)q * j;
+    for (int jb = warp * 4; jb < q; jb += kWarps * 4) {            // 8 lanes a column
+        const int j = jb + (lane >> 3), l8 = lane & 7;
+        const bool live = j < q;
+        T *dj = D + (int64_t)p * (live ? j : jb), *jj = J + (int64_t)q * (live ? j : jb);
         T ss = 0, sj = 0;
-        for (int r = lane; r < p; r += 32) ss = fma(dj[r], dj[r], ss);
-        for (int r = lane; r < q; r += 32) sj = fma(jj[r], jj[r], sj);
-        const T sv = sqrt(warp_sum(ss)), nj = sqrt(warp_sum(sj));
-        if (sv > T(0)) {
-            const T inv = T(1) / sv;
-            for (int r = lane; r < p; r += 32) dj[r] *= inv;
+        for (int r = l8; r < p; r += 8) ss = fma(dj[r], dj[r], ss);
+        for (int r = l8; r < q; r += 8) sj = fma(jj[r], jj[r], sj);
+        ss = group_sum(ss, 8);
+        sj = group_sum(sj, 8);
+        T sv = ss, inv = 0, nj, invj;
+        if (ss > T(0)) sqrt_both(ss, sv, inv);
+        sqrt_both(sj, nj, invj);
+        __syncwarp();
+        if (live) {
+            if (sv > T(0))
+                for (int r = l8; r < p; r += 8) dj[r] *= inv;
+            for (int r = l8; r < q; r += 8) jj[r] *= invj;
+            if (l8 == 0) sig[j] = sv * invj * s_unscale;
         }
-        const T invj = T(1) / nj;
-        for (int r = lane; r < q; r += 32) jj[r] *= invj;
-        if (lane == 0) sig[j] = sv * invj * s_unscale;
     }
     __syncthreads();
     // descending order, ties by index; a NaN ranks below everything (its key
@@ -534,15 +771,30 @@ __global__ void __launch_bounds__(kThreads) lr_svd_kernel(const LrJob *jobs, con
 
     // 5. outputs: U = (Q_P or P) W, V = (Q_Q or Q) Z for the kept columns
     T *U = static_cast<T *>(pr.U), *V = static_cast<T *>(pr.V), *so = static_cast<T *>(pr.s);
+    // w_k, length ka, and z_k, length kb
+    auto wcol = [&](int k) -> const T * { return tr ? J + (int64_t)q * perm[k] : D + (int64_t)p * perm[k]; };
+    auto zcol = [&](int k) -> const T * { return tr ? D + (int64_t)p * perm[k] : J + (int64_t)q * perm[k]; };
+    for (int k = tid; k < rk; k += kThreads) so[k] = sig[perm[k]];
+    const bool fastU = pr.qr_left && m <= kRegRows, fastV = pr.qr_right && n <= kRegRows;
+    // with both sides in registers the two halves of the warps take one each
+    const int nu = fastU && fastV ? kWarps / 2 : kWarps;
+    if (fastU && warp < nu)
+        apply_q_any<T>(WP, ldP, (int)m, ka, tauP, rk, warp, nu,
+                       [&](int k, int i) { return i < ka ? wcol(k)[i] : T(0); },
+                       [&](int k, int i, T v) { U[i + m * k] = v; });
+    if (fastV && (nu == kWarps || warp >= nu))
+        apply_q_any<T>(WQ, ldQ, (int)n, kb, tauQ, rk, nu == kWarps ? warp : warp - nu, nu,
+                       [&](int k, int i) { return i < kb ? zcol(k)[i] : T(0); },
+                       [&](int k, int i, T v) { V[i + n * k] = v; });
+    if (fastU && fastV) return;
     for (int k = warp; k < rk; k += kWarps) {
-        const int j = perm[k];
-        const T *wv = tr ? J + (int64_t)q * j : D + (int64_t)p * j;     // length ka
-        const T *zv = tr ? D + (int64_t)p * j : J + (int64_t)q * j;     // length kb
+        const T *wv = wcol(k), *zv = zcol(k);
         T *u = U + m * k;
-        if (pr.qr_left) {
+        if (fastU) {
+        } else if (pr.qr_left) {
             for (int64_t i = lane; i < m; i += 32) u[i] = i < ka ? wv[i] : T(0);
             __syncwarp();
-            apply_q(WP, m, ka, tauP, u);
+            apply_q(WP, ldP, m, ka, tauP, u);
         } else {
             for (int64_t i = lane; i < m; i += 32) {
                 T acc = 0;
@@ -552,10 +804,11 @@ __global__ void __launch_bounds__(kThreads) lr_svd_kernel(const LrJob *jobs, con
             }
         }
         T *v = V + n * k;
-        if (pr.qr_right) {
+        if (fastV) {
+        } else if (pr.qr_right) {
             for (int64_t i = lane; i < n; i += 32) v[i] = i < kb ? zv[i] : T(0);
             __syncwarp();
-            apply_q(WQ, n, kb, tauQ, v);
+            apply_q(WQ, ldQ, n, kb, tauQ, v);
         } else if (!pr.Q1) {
             for (int64_t i = lane; i < n; i += 32) v[i] = zv[i];
         } else {
@@ -566,7 +819,6 @@ __global__ void __launch_bounds__(kThreads) lr_svd_kernel(const LrJob *jobs, con
                 v[i] = acc;
             }
         }
-        if (lane == 0) so[k] = sig[j];
     }
 }
 
@@ -769,9 +1021,10 @@ __device__ __forceinline__ void upper_pair(int p, int &i, int &j)
 // Right-looking with lookahead: warp 0 applies step j to row j + 1 and forms
 // pivot j + 1 (a Halley reciprocal square root; the dependent FP64 chain is
 // the kernel's critical path on GB300, 64 cycles per operation) while the
-// other warps apply step j to the rows below, its entries spread evenly over
-// them (an FP64 warp instruction costs the same with idle lanes); one barrier
-// per step.  L is what the forward substitutions of the solves read (its
+// warps of the other three sub-partitions apply step j to the rows below, its
+// entries spread evenly over them (an FP64 warp instruction costs the same with
+// idle lanes; a fourth warp's would stand before warp 0's); one barrier per step.
+// L is what the forward substitutions of the solves read (its
 // columns contiguous).
 struct LeafChol {
     int64_t n;
@@ -788,10 +1041,9 @@ int64_t leaf_chol_max()
     return n;
 }
 template <typename T>
-__global__ void __launch_bounds__(kThreads) leaf_chol(const LeafChol *probs, int *info)
+__global__ void __launch_bounds__(kThreads) leaf_chol(const LeafChol g, int *info)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const LeafChol g = probs[blockIdx.x];
     const int n = (int)g.n, ls = n + 1, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     T *S = reinterpret_cast<T *>(smem_raw);            // n x n, ld n + 1
     __shared__ int s_fail;
@@ -822,9 +1074,9 @@ __global__ void __launch_bounds__(kThreads) leaf_chol(const LeafChol *probs, int
                 __syncwarp();
                 pivot(j + 1);
             }
-        } else {
+        } else if (warp & 3) {
             const int m = n - j - 2, tj = m > 0 ? m * (m + 1) / 2 : 0;
-            for (int p = tid - 32; p < tj; p += kThreads - 32) {
+            for (int p = tid - 32 - (warp > 4 ? 32 : 0); p < tj; p += kThreads - 64) {
                 int i, l;
                 upper_pair(p, i, l);
                 i += j + 2;
@@ -834,7 +1086,7 @@ __global__ void __launch_bounds__(kThreads) leaf_chol(const LeafChol *probs, int
         }
         __syncthreads();
     }
-    if (tid == 0) info[blockIdx.x] = s_fail;
+    if (tid == 0) *info = s_fail;
     // R and L are written also after a failed pivot (the partial factor, as
     // potrf_batched leaves it): what follows reads finite values
     T *R = static_cast<T *>(g.R), *Lo = static_cast<T *>(g.L);
@@ -843,6 +1095,21 @@ __global__ void __launch_bounds__(kThreads) leaf_chol(const LeafChol *probs, int
         R[i + g.ldr * j] = S[i + ls * j];
         Lo[i + g.ldl * j] = i >= j ? S[j + ls * i] : T(0);
     }
+}
+
+// X = U, sk = s, Vk = V (n1 x r, r, n2 x r): the block that a node's solve starts
+// from, in one launch (three copies cost three launches of the factorisation's
+// serial chain).
+template <typename T>
+__global__ void __launch_bounds__(kThreads) hchol_block(const T *U, int64_t ldu, int64_t n1, const T *s, const T *V, int64_t ldv,
+                                                         int64_t n2, int r, T *X, T *sk, T *Vk)
+{
+    const int c = blockIdx.y;
+    for (int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x; i < n1 + n2; i += (int64_t)gridDim.x * kThreads) {
+        if (i < n1) X[i + n1 * c] = U[i + ldu * c];
+        else Vk[i - n1 + n2 * c] = V[i - n1 + ldv * c];
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) sk[c] = s[c];
 }
 
 // H = diag(s) X^T X diag(s) for a tall X (rows x r, r <= kGramMax) by
@@ -1188,9 +1455,13 @@ constexpr size_t kPreconSmemBytes = 224 * 1024;
 // Workspace layout and shared memory of one lr_svd launch.
 struct LrPlan {
     std::vector<int64_t> off, coff;
-    int64_t ws = 0, dmax = 1, xoff = -1;
+    int64_t ws = 0, dmax = 1, xoff = -1, soff = 0, scap = 0;
     size_t smem = 0;
 };
+// Shared memory up to which panels are staged: whole SMs while a launch has an SM
+// per problem, a third of one for larger batches (whose CTAs share the SMs).
+constexpr size_t kPanelSmemBytes = 224 * 1024, kPanelSmemBytesMany = 72 * 1024;
+constexpr int kPanelFew = 152;
 
 template <typename T>
 int lr_svd_plan(int nprob, const LrJob *jobs, LrPlan &pl)
@@ -1238,7 +1509,7 @@ int lr_svd_plan(int nprob, const LrJob *jobs, LrPlan &pl)
         const int64_t q = std::min(ka, kb), pp = std::max(ka, kb);
         if (q > 0 && (!p.U || !p.s || !p.V)) { set_last_error("problem %d: NULL output", i); return HM_ERR_INVALID_ARG; }
         pl.off[i] = ws;
-        ws += (p.qr_left ? p.m * a : 0) + (p.qr_right ? p.n * b : 0) + a + b;
+        ws += (p.qr_left ? p.m * a : 0) + (p.qr_right ? p.n * b : 0) + 2 * (a + b);
         ws = (ws + 31) / 32 * 32;
         const int64_t jn = std::max({q * q, p.Xm ? (int64_t)32 * (a + b) : 0, full2 ? ka * b : 0});
         const size_t need = (size_t)(pp * q + jn + q) * sizeof(T) + (size_t)q * sizeof(int) + 64;
@@ -1246,7 +1517,7 @@ int lr_svd_plan(int nprob, const LrJob *jobs, LrPlan &pl)
             dmax = std::max(dmax, pp * q);
             jmax = std::max(jmax, jn);
             qmax = std::max<int>(qmax, (int)q);
-            xmax = std::max(xmax, q * q + pp * q + q);
+            xmax = std::max(xmax, q * q + pp * q + 2 * q);
         } else {
             pl.coff[i] = ws;
             ws += pp * q + jn + 2 * q;          // sigma (q values) and the order (q ints) after J
@@ -1263,6 +1534,14 @@ int lr_svd_plan(int nprob, const LrJob *jobs, LrPlan &pl)
         pl.xoff = xoff;
         pl.smem = (size_t)(xoff + xmax) * sizeof(T);
     }
+    pl.soff = (int64_t)((pl.smem + 15) / 16 * 16 / sizeof(T));
+    const size_t most = nprob <= kPanelFew ? kPanelSmemBytes : kPanelSmemBytesMany;
+    for (int i = 0; i < nprob; ++i) {
+        const hm_lr_problem &p = jobs[i].p;
+        const int64_t v = p.qr_left || p.qr_right ? lr_panel_vals(p) : 0;
+        if ((size_t)(pl.soff + v) * sizeof(T) <= most) pl.scap = std::max(pl.scap, v);
+    }
+    if (pl.scap) pl.smem = (size_t)(pl.soff + pl.scap) * sizeof(T);
     return set_smem(lr_svd_kernel<T>, pl.smem);
 }
 
@@ -1284,7 +1563,8 @@ int lr_svd_run(int nprob, const hm_lr_problem *probs, int32_t *ranks, cudaStream
     ALG_TRY(S.put(pl.coff.data(), pl.coff.size(), &d_coff));
     ALG_TRY(S.zeros((size_t)pl.ws, &d_ws));
     ALG_TRY(S.zeros((size_t)nprob, &d_ranks));
-    lr_svd_kernel<T><<<nprob, kThreads, pl.smem, st>>>(d_jobs, d_off, d_coff, d_ws, d_ranks, pl.dmax, pl.xoff);
+    lr_svd_kernel<T><<<nprob, kThreads, pl.smem, st>>>(d_jobs, d_off, d_coff, d_ws, d_ranks, pl.dmax, pl.xoff,
+                                                     pl.soff, pl.scap);
     ALG_CK(cudaGetLastError());
     std::vector<int> hr(nprob);
     ALG_CK(cudaMemcpyAsync(hr.data(), d_ranks, nprob * sizeof(int), cudaMemcpyDeviceToHost, st));
@@ -1834,9 +2114,7 @@ struct HChol {
             const LeafChol lc{g.n, N.D, N.ldd, o.R, o.ldr, lts[i], g.n};
             const size_t smem = (size_t)(g.n * (g.n + 1)) * sizeof(T);
             ALG_TRY(set_smem(leaf_chol<T>, smem));
-            LeafChol *dl = nullptr;
-            ALG_TRY(S.put(&lc, 1, &dl));
-            leaf_chol<T><<<1, kThreads, smem, st>>>(dl, d_info + N.leaf);
+            leaf_chol<T><<<1, kThreads, smem, st>>>(lc, d_info + N.leaf);
             ALG_CK(cudaGetLastError());
             return inverse(i);
         }
@@ -2048,14 +2326,21 @@ struct HChol {
         T *dws = nullptr;
         int *dr = nullptr;
         S.st = sx;
-        int rc = S.put(jobs.data(), (size_t)np, &dj);
-        if (!rc) rc = S.put(pl.off.data(), pl.off.size(), &doff);
-        if (!rc) rc = S.put(pl.coff.data(), pl.coff.size(), &dcoff);
+        // jobs, workspace offsets and core offsets in one copy
+        std::vector<char> desc((size_t)np * (sizeof(LrJob) + 2 * sizeof(int64_t)));
+        char *dd = nullptr;
+        std::memcpy(desc.data(), jobs.data(), np * sizeof(LrJob));
+        std::memcpy(desc.data() + np * sizeof(LrJob), pl.off.data(), np * sizeof(int64_t));
+        std::memcpy(desc.data() + np * (sizeof(LrJob) + sizeof(int64_t)), pl.coff.data(), np * sizeof(int64_t));
+        const int rc = S.put(desc.data(), desc.size(), &dd);
+        dj = reinterpret_cast<LrJob *>(dd);
+        doff = reinterpret_cast<int64_t *>(dd + np * sizeof(LrJob));
+        dcoff = doff + np;
         S.st = st;
         ALG_TRY(rc);
         ALG_TRY(S.zeros((size_t)pl.ws, &dws));
         ALG_TRY(S.zeros((size_t)np, &dr));
-        lr_svd_kernel<T><<<np, kThreads, pl.smem, sx>>>(dj, doff, dcoff, dws, dr, pl.dmax, pl.xoff);
+        lr_svd_kernel<T><<<np, kThreads, pl.smem, sx>>>(dj, doff, dcoff, dws, dr, pl.dmax, pl.xoff, pl.soff, pl.scap);
         ALG_CK(cudaGetLastError());
         int32_t *slot = nullptr;
         ALG_TRY(pinned_words(np, &slot));
@@ -2082,11 +2367,9 @@ struct HChol {
         ALG_TRY(res->keep.get((size_t)r, &sk));
         ALG_TRY(res->keep.get((size_t)(n2 * r), &Vk));
         if (r > 0) {
-            ALG_CK(cudaMemcpy2DAsync(X, n1 * sizeof(T), N.U, N.ldu * sizeof(T), n1 * sizeof(T), r,
-                                     cudaMemcpyDeviceToDevice, st));
-            ALG_CK(cudaMemcpyAsync(sk, N.s, r * sizeof(T), cudaMemcpyDeviceToDevice, st));
-            ALG_CK(cudaMemcpy2DAsync(Vk, n2 * sizeof(T), N.V, N.ldv * sizeof(T), n2 * sizeof(T), r,
-                                     cudaMemcpyDeviceToDevice, st));
+            const unsigned bx = (unsigned)std::min<int64_t>((n1 + n2 + kThreads - 1) / kThreads, 64);
+            hchol_block<T><<<dim3(bx, r), kThreads, 0, st>>>(N.U, N.ldu, n1, N.s, N.V, N.ldv, n2, r, X, sk, Vk);
+            ALG_CK(cudaGetLastError());
             const Node &L = nd[g.left];
             hm_solve_op *dops = nullptr;
             ALG_TRY(schedule(g.left, &dops));
