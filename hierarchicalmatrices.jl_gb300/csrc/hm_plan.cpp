@@ -18,6 +18,7 @@
 #include "hm_plan.h"
 
 #include <algorithm>
+#include <cstdint>
 
 namespace hm {
 
@@ -131,40 +132,54 @@ void assign_basis(Tree &T, int id, bool above)
     }
 }
 
-// Slots in (level, lo) order; returns the slot count.
-int assign_slots(Tree &T)
+// Slots in (level, lo) order; `ids` receives the node of each slot.  Returns the
+// slot count.
+int assign_slots(Tree &T, std::vector<int> &ids)
 {
-    std::vector<int> ids;
+    // bucketed by level, each level sorted by (lo, node)
+    std::vector<int> start;
+    for (const Node &n : T.nodes)
+        if (n.kind) {
+            if (n.level + 2 > (int)start.size()) start.resize(n.level + 2, 0);
+            ++start[n.level + 1];
+        }
+    for (size_t k = 1; k < start.size(); ++k) start[k] += start[k - 1];
+    const int count = start.empty() ? 0 : start.back();
+    std::vector<std::pair<int64_t, int>> keys(count);
+    std::vector<int> at(start);
     for (size_t i = 0; i < T.nodes.size(); ++i)
-        if (T.nodes[i].kind) ids.push_back((int)i);
-    std::sort(ids.begin(), ids.end(), [&](int u, int v) {
-        if (T.nodes[u].level != T.nodes[v].level) return T.nodes[u].level < T.nodes[v].level;
-        if (T.nodes[u].lo != T.nodes[v].lo) return T.nodes[u].lo < T.nodes[v].lo;
-        return u < v;
-    });
-    for (size_t k = 0; k < ids.size(); ++k) T.nodes[ids[k]].slot = (int)k;
-    return (int)ids.size();
+        if (T.nodes[i].kind) keys[at[T.nodes[i].level]++] = {T.nodes[i].lo, (int)i};
+    for (size_t k = 0; k + 1 < start.size(); ++k)
+        if (!std::is_sorted(keys.begin() + start[k], keys.begin() + start[k + 1]))
+            std::sort(keys.begin() + start[k], keys.begin() + start[k + 1]);
+    ids.resize(count);
+    for (int k = 0; k < count; ++k) {
+        ids[k] = keys[k].second;
+        T.nodes[ids[k]].slot = k;
+    }
+    return count;
 }
 
-// Transfer steps for the internal basis nodes, grouped by level.
-void transfer_steps(const Tree &T, bool deepest_first, std::vector<hm_xfer> &out,
+// Transfer steps for the internal basis nodes, grouped by level (slots are in
+// level order, so a level's nodes follow one another in `ids`).
+void transfer_steps(const Tree &T, const std::vector<int> &ids, bool deepest_first, std::vector<hm_xfer> &out,
                     std::vector<int> &ptr)
 {
-    int maxlev = 0;
-    for (const Node &n : T.nodes) if (n.kind == 1) maxlev = std::max(maxlev, n.level);
-    std::vector<std::vector<hm_xfer>> by(maxlev + 1);
-    for (const Node &n : T.nodes)
-        if (n.kind == 1)
-            by[n.level].push_back({n.slot, T.nodes[n.child[0]].slot, T.nodes[n.child[1]].slot, 0});
     out.clear(); ptr.clear();
     ptr.push_back(0);
-    for (int k = 0; k <= maxlev; ++k) {
-        int lev = deepest_first ? maxlev - k : k;
-        auto &v = by[lev];
-        if (v.empty()) continue;
-        std::sort(v.begin(), v.end(), [](const hm_xfer &p, const hm_xfer &q) { return p.slot < q.slot; });
-        out.insert(out.end(), v.begin(), v.end());
-        ptr.push_back((int)out.size());
+    auto level = [&](size_t b, size_t e) {
+        for (size_t k = b; k < e; ++k) {
+            const Node &n = T.nodes[ids[k]];
+            if (n.kind == 1) out.push_back({n.slot, T.nodes[n.child[0]].slot, T.nodes[n.child[1]].slot, 0});
+        }
+        if ((int)out.size() > ptr.back()) ptr.push_back((int)out.size());
+    };
+    std::vector<size_t> bounds;
+    for (size_t k = 0; k <= ids.size(); ++k)
+        if (k == 0 || k == ids.size() || T.nodes[ids[k]].level != T.nodes[ids[k - 1]].level) bounds.push_back(k);
+    for (size_t k = 0; k + 1 < bounds.size(); ++k) {
+        const size_t l = deepest_first ? bounds.size() - 2 - k : k;
+        level(bounds[l], bounds[l + 1]);
     }
 }
 
@@ -174,36 +189,40 @@ inline int64_t round_up(int64_t v, int64_t m) { return (v + m - 1) / m * m; }
 // from the deepest internal level).  Within a band, a task is the set of
 // nodes sharing the same topmost in-band ancestor; its steps are its levels,
 // deepest first for the upward pass, topmost first for the downward pass.
-void band_transfers(const Tree &T, bool upward, std::vector<hm_xfer> &ents, std::vector<hm_step> &steps,
-                    std::vector<hm_task> &tasks, std::vector<int> &band_ptr)
+void band_transfers(const Tree &T, const std::vector<int> &ids, bool upward, std::vector<hm_xfer> &ents,
+                    std::vector<hm_step> &steps, std::vector<hm_task> &tasks, std::vector<int> &band_ptr)
 {
     ents.clear(); steps.clear(); tasks.clear(); band_ptr.clear();
     int maxlev = -1;
-    for (const Node &n : T.nodes) if (n.kind == 1) maxlev = std::max(maxlev, n.level);
+    for (int id : ids) if (T.nodes[id].kind == 1) maxlev = std::max(maxlev, T.nodes[id].level);
     band_ptr.push_back(0);
     if (maxlev < 0) return;
     const int nbands = maxlev / kBandLevels + 1;
     auto band_of = [&](int level) { return (maxlev - level) / kBandLevels; };
-    // task root of every internal node: climb while the parent is internal and in the same band
-    std::vector<std::vector<std::pair<int, int>>> members(nbands);   // (root id, node id)
-    for (size_t i = 0; i < T.nodes.size(); ++i) {
-        if (T.nodes[i].kind != 1) continue;
-        int root = (int)i;
-        const int b = band_of(T.nodes[i].level);
-        while (T.nodes[root].parent >= 0 && T.nodes[T.nodes[root].parent].kind == 1 &&
-               band_of(T.nodes[T.nodes[root].parent].level) == b)
-            root = T.nodes[root].parent;
-        members[b].push_back({root, (int)i});
+    // task root of every internal node: its parent's where the parent is internal and in
+    // the same band (parents have lower slots), else itself
+    std::vector<int> root(ids.size(), -1);
+    // records in (root, level in launch order, slot) order, one key each
+    static_assert(kBandLevels <= 4, "two bits of the key");
+    std::vector<std::vector<uint64_t>> members(nbands);
+    for (size_t k = 0; k < ids.size(); ++k) {
+        const Node &n = T.nodes[ids[k]];
+        if (n.kind != 1) continue;
+        const int b = band_of(n.level);
+        root[k] = (int)k;
+        if (n.parent >= 0) {
+            const Node &q = T.nodes[n.parent];
+            if (q.kind == 1 && band_of(q.level) == b) root[k] = root[q.slot];
+        }
+        const uint64_t below = (maxlev - n.level) % kBandLevels;       // 0: the band's deepest level
+        members[b].push_back((uint64_t)root[k] << 33 | (upward ? below : kBandLevels - 1 - below) << 31 | (uint64_t)k);
     }
     for (int k = 0; k < nbands; ++k) {
         const int b = upward ? k : nbands - 1 - k;
-        auto &mem = members[b];
-        std::sort(mem.begin(), mem.end(), [&](const std::pair<int, int> &p, const std::pair<int, int> &q) {
-            if (p.first != q.first) return T.nodes[p.first].slot < T.nodes[q.first].slot;
-            const int lp = T.nodes[p.second].level, lq = T.nodes[q.second].level;
-            if (lp != lq) return upward ? lp > lq : lp < lq;
-            return T.nodes[p.second].slot < T.nodes[q.second].slot;
-        });
+        std::vector<std::pair<int, int>> mem;                          // (root slot, node)
+        std::sort(members[b].begin(), members[b].end());
+        mem.reserve(members[b].size());
+        for (uint64_t key : members[b]) mem.push_back({(int)(key >> 33), ids[(size_t)(key & 0x7fffffffu)]});
         for (size_t i = 0; i < mem.size(); ++i) {
             const Node &n = T.nodes[mem[i].second];
             const bool new_task = i == 0 || mem[i].first != mem[i - 1].first;
@@ -224,10 +243,11 @@ void band_transfers(const Tree &T, bool upward, std::vector<hm_xfer> &ents, std:
     // pad = local(c0) | local(c1) << 16.  Downward, record i's children are
     // locals 2i and 2i + 1 and its parent is an earlier child or external
     // (numbered after the children); pad = local(parent).
+    std::vector<std::pair<int32_t, int32_t>> made;         // (slot, local), small per task
     for (const hm_task &tk : tasks) {
         const int e0 = steps[tk.step0].e0, e1 = steps[tk.step1 - 1].e1;
         const int nrec = e1 - e0;
-        std::vector<std::pair<int32_t, int32_t>> made;     // (slot, local), small per task
+        made.clear();
         auto find = [&](int32_t slot) {
             for (auto &m : made) if (m.first == slot) return m.second;
             return -1;
@@ -270,21 +290,18 @@ int build_plan(const double *x, int64_t nx, const double *y, int64_t ny, double 
     mark_sub_used(P.Y);
     assign_basis(P.X, 0, false);
     assign_basis(P.Y, 0, false);
-    P.n_xslots = assign_slots(P.X);
-    P.n_yslots = assign_slots(P.Y);
-    transfer_steps(P.Y, true, P.up, P.up_level_ptr);
-    transfer_steps(P.X, false, P.down, P.down_level_ptr);
+    std::vector<int> xids, yids;                           // the node of each slot
+    P.n_xslots = assign_slots(P.X, xids);
+    P.n_yslots = assign_slots(P.Y, yids);
+    transfer_steps(P.Y, yids, true, P.up, P.up_level_ptr);
+    transfer_steps(P.X, xids, false, P.down, P.down_level_ptr);
 
     // Explicit column bases at the deepest basis nodes of the column tree.
     {
-        std::vector<int> leaves;
-        for (size_t i = 0; i < P.Y.nodes.size(); ++i)
-            if (P.Y.nodes[i].kind == 2) leaves.push_back((int)i);
-        std::sort(leaves.begin(), leaves.end(),
-                  [&](int u, int v) { return P.Y.nodes[u].slot < P.Y.nodes[v].slot; });
         int64_t off = 0;
-        for (int id : leaves) {
+        for (int id : yids) {                              // slot order
             const Node &n = P.Y.nodes[id];
+            if (n.kind != 2) continue;
             hm_vpanel vp;
             vp.row0 = n.lo;
             vp.nrows = (int32_t)(n.hi - n.lo);
@@ -301,61 +318,88 @@ int build_plan(const double *x, int64_t nx, const double *y, int64_t ny, double 
         P.vstore_elems = off;
     }
 
-    band_transfers(P.Y, true, P.up_ents, P.up_steps, P.up_tasks, P.up_band_ptr);
-    band_transfers(P.X, false, P.down_ents, P.down_steps, P.down_tasks, P.down_band_ptr);
+    band_transfers(P.Y, yids, true, P.up_ents, P.up_steps, P.up_tasks, P.up_band_ptr);
+    band_transfers(P.X, xids, false, P.down_ents, P.down_steps, P.down_tasks, P.down_band_ptr);
 
     // M2L rows: barycentric blocks grouped by row cluster.
     P.fstride = (int)round_up((int64_t)r * r, 4);
     {
-        std::vector<std::pair<int, int>> bs;   // (xslot, index into bary)
-        for (size_t i = 0; i < P.bary.size(); ++i)
-            bs.push_back({P.X.nodes[P.bary[i].first].slot, (int)i});
-        std::sort(bs.begin(), bs.end(), [&](const std::pair<int, int> &p, const std::pair<int, int> &q) {
-            if (p.first != q.first) return p.first < q.first;
-            return P.Y.nodes[P.bary[p.second].second].slot < P.Y.nodes[P.bary[q.second].second].slot;
-        });
         // One row per row-basis slot (slots without blocks get empty ranges, so
-        // the far-field pass writes every coefficient).
-        for (int sl = 0; sl < P.n_xslots; ++sl) P.m2l_rows.push_back({sl, 0, 0, 0});
+        // the far-field pass writes every coefficient); a row's blocks by column slot.
+        std::vector<int32_t> at(P.n_xslots + 1, 0);
+        for (auto &e : P.bary) ++at[P.X.nodes[e.first].slot + 1];
+        for (int sl = 0; sl < P.n_xslots; ++sl) at[sl + 1] += at[sl];
+        P.m2l_rows.reserve(P.n_xslots);
+        for (int sl = 0; sl < P.n_xslots; ++sl)
+            P.m2l_rows.push_back({sl, at[sl + 1] > at[sl] ? at[sl] : 0, at[sl + 1] > at[sl] ? at[sl + 1] : 0, 0});
+        std::vector<uint64_t> bs(P.bary.size());           // column slot, index into bary
+        for (size_t i = 0; i < P.bary.size(); ++i)
+            bs[at[P.X.nodes[P.bary[i].first].slot]++] = (uint64_t)P.Y.nodes[P.bary[i].second].slot << 32 | (uint64_t)i;
+        for (const hm_m2l_row &row : P.m2l_rows) std::sort(bs.begin() + row.begin, bs.begin() + row.end);
+        P.m2l_ents.resize(bs.size());
+        P.f_fill.resize(bs.size());
         for (size_t k = 0; k < bs.size(); ++k) {
-            const int xn = P.bary[bs[k].second].first, yn = P.bary[bs[k].second].second;
-            hm_m2l_row &row = P.m2l_rows[bs[k].first];
-            if (row.end == 0) row.begin = (int32_t)k;
-            row.end = (int32_t)(k + 1);
-            hm_m2l_ent e;
-            e.foff = (int64_t)k * P.fstride;
-            e.yslot = P.Y.nodes[yn].slot;
-            e.pad = 0;
-            P.m2l_ents.push_back(e);
-            P.f_fill.push_back({P.X.nodes[xn].a, P.X.nodes[xn].b, P.Y.nodes[yn].a, P.Y.nodes[yn].b});
+            const auto &blk = P.bary[(size_t)(bs[k] & 0xffffffffu)];
+            const Node &xn = P.X.nodes[blk.first], &yn = P.Y.nodes[blk.second];
+            P.m2l_ents[k] = hm_m2l_ent{};
+            P.m2l_ents[k].foff = (int64_t)k * P.fstride;
+            P.m2l_ents[k].yslot = yn.slot;
+            P.f_fill[k] = {xn.a, xn.b, yn.a, yn.b};
         }
         P.fstore_elems = (int64_t)bs.size() * P.fstride;
     }
 
     // Row segments: elementary row intervals of {row-basis leaves, dense rows}.
     {
+        std::vector<std::pair<int64_t, int>> xl;           // (lo, node) of the row-basis leaves
+        std::vector<char> dense_x(P.X.nodes.size(), 0);
+        for (int id : xids)
+            if (P.X.nodes[id].kind == 2 && P.X.size(id) > 0) xl.push_back({P.X.nodes[id].lo, id});
+        std::sort(xl.begin(), xl.end());
         std::vector<int> xleaves;
-        for (size_t i = 0; i < P.X.nodes.size(); ++i)
-            if (P.X.nodes[i].kind == 2 && P.X.size((int)i) > 0) xleaves.push_back((int)i);
-        std::sort(xleaves.begin(), xleaves.end(),
-                  [&](int u, int v) { return P.X.nodes[u].lo < P.X.nodes[v].lo; });
-        std::vector<int64_t> cuts = {0, nx};
-        for (int id : xleaves) { cuts.push_back(P.X.nodes[id].lo); cuts.push_back(P.X.nodes[id].hi); }
-        for (auto &e : P.dense) {
-            if (P.X.size(e.first) == 0 || P.Y.size(e.second) == 0) continue;
-            cuts.push_back(P.X.nodes[e.first].lo);
-            cuts.push_back(P.X.nodes[e.first].hi);
+        xleaves.reserve(xl.size());
+        for (auto &e : xl) xleaves.push_back(e.second);
+        for (auto &e : P.dense)
+            if (P.X.size(e.first) > 0 && P.Y.size(e.second) > 0) dense_x[e.first] = 1;
+        // the cuts as bits over 0 .. nx: their order and a cut's index come from counting
+        // bits (sorting four values per block took a quarter of the whole plan)
+        const size_t words = (size_t)(nx / 64 + 1);
+        std::vector<uint64_t> bits(words, 0);
+        auto cut = [&](int64_t i) { bits[(size_t)(i >> 6)] |= uint64_t(1) << (i & 63); };
+        cut(0);
+        cut(nx);
+        for (size_t i = 0; i < P.X.nodes.size(); ++i) {
+            const Node &n = P.X.nodes[i];
+            if (!dense_x[i] && !(n.kind == 2 && n.hi > n.lo)) continue;
+            cut(n.lo);
+            cut(n.hi);
         }
-        std::sort(cuts.begin(), cuts.end());
-        cuts.erase(std::unique(cuts.begin(), cuts.end()), cuts.end());
+        std::vector<uint32_t> before(words);
+        std::vector<int64_t> cuts;
+        for (size_t w = 0; w < words; ++w) {
+            before[w] = (uint32_t)cuts.size();
+            for (uint64_t b = bits[w]; b; b &= b - 1) cuts.push_back((int64_t)w * 64 + __builtin_ctzll(b));
+        }
+        auto index_of = [&](int64_t i) {
+            const uint64_t below = bits[(size_t)(i >> 6)] & ((uint64_t(1) << (i & 63)) - 1);
+            return (size_t)before[(size_t)(i >> 6)] + (size_t)__builtin_popcountll(below);
+        };
         const size_t nint = cuts.size() - 1;
-        std::vector<std::vector<int>> dl(nint);
-        for (size_t k = 0; k < P.dense.size(); ++k) {
-            const Node &xn = P.X.nodes[P.dense[k].first];
-            if (xn.hi <= xn.lo || P.Y.size(P.dense[k].second) == 0) continue;
-            size_t i0 = std::lower_bound(cuts.begin(), cuts.end(), xn.lo) - cuts.begin();
-            size_t i1 = std::lower_bound(cuts.begin(), cuts.end(), xn.hi) - cuts.begin();
-            for (size_t i = i0; i < i1; ++i) dl[i].push_back((int)k);
+        // the dense blocks of each interval, by first column
+        std::vector<int32_t> dptr(nint + 1, 0);
+        auto intervals = [&](const std::pair<int, int> &e, auto &&visit) {
+            if (!dense_x[e.first] || P.Y.size(e.second) == 0) return;
+            const Node &xn = P.X.nodes[e.first];
+            const size_t i1 = index_of(xn.hi);
+            for (size_t i = index_of(xn.lo); i < i1; ++i) visit(i);
+        };
+        for (auto &e : P.dense) intervals(e, [&](size_t i) { ++dptr[i + 1]; });
+        for (size_t i = 0; i < nint; ++i) dptr[i + 1] += dptr[i];
+        std::vector<std::pair<int64_t, int>> dl(dptr[nint]);           // (first column, column node)
+        {
+            std::vector<int32_t> at(dptr.begin(), dptr.end() - 1);
+            for (auto &e : P.dense)
+                intervals(e, [&](size_t i) { dl[at[i]++] = {P.Y.nodes[e.second].lo, e.second}; });
         }
         size_t lp = 0;
         int64_t poff = 0;
@@ -365,10 +409,8 @@ int build_plan(const double *x, int64_t nx, const double *y, int64_t ny, double 
             while (lp < xleaves.size() && P.X.nodes[xleaves[lp]].hi <= p) ++lp;
             int leafid = -1;
             if (lp < xleaves.size() && P.X.nodes[xleaves[lp]].lo <= p) leafid = xleaves[lp];
-            auto &ds = dl[iv];
-            std::sort(ds.begin(), ds.end(), [&](int u, int v) {
-                return P.Y.nodes[P.dense[u].second].lo < P.Y.nodes[P.dense[v].second].lo;
-            });
+            const auto d0 = dl.begin() + dptr[iv], d1 = dl.begin() + dptr[iv + 1];
+            std::sort(d0, d1);
             for (int64_t r0 = p; r0 < q; r0 += seg_rows) {
                 hm_seg s;
                 s.row0 = r0;
@@ -386,8 +428,8 @@ int build_plan(const double *x, int64_t nx, const double *y, int64_t ny, double 
                     f.has_basis = 1; f.basis_w = r;
                     f.a = P.X.nodes[leafid].a; f.b = P.X.nodes[leafid].b;
                 }
-                for (int k : ds) {
-                    const Node &yn = P.Y.nodes[P.dense[k].second];
+                for (auto d = d0; d != d1; ++d) {
+                    const Node &yn = P.Y.nodes[d->second];
                     hm_piece pc;
                     pc.kind = HM_PIECE_X; pc.src = yn.lo; pc.width = (int32_t)(yn.hi - yn.lo);
                     P.pieces.push_back(pc);
