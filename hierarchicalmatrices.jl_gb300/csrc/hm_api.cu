@@ -11,6 +11,7 @@
 #include <map>
 #include <set>
 #include <thread>
+#include <tuple>
 #include <mutex>
 #include <string>
 #include <type_traits>
@@ -777,6 +778,23 @@ int prefer_shared(K kernel)
     return HM_OK;
 }
 
+// CTAs of `kernel` that fit on an SM (asked once per device, kernel and shared memory).
+std::map<std::tuple<int, const void *, size_t>, int> g_ctas_per_sm;
+template <typename K>
+int ctas_per_sm(K kernel, int threads, size_t smem, int *out)
+{
+    int dev = 0;
+    HM_CK(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> lk(g_smem_mu);
+    int &n = g_ctas_per_sm[std::make_tuple(dev, reinterpret_cast<const void *>(kernel), smem)];
+    if (n == 0) {
+        HM_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, threads, smem));
+        n = std::max(n, 1);
+    }
+    *out = n;
+    return HM_OK;
+}
+
 // Per-call scratch: coefficients t (column slots) then s (row slots).
 struct ScratchLayout {
     size_t t_off, s_off, yfar_off, bytes;
@@ -1298,11 +1316,16 @@ int launch_part_kb(hm_handle *h, const MulArgs<S> &ma, const A *s, const A *t, c
             const size_t smem = ring_smem_bytes(KB, tl.pf, tl.ns);
             HM_TRY(ensure_smem(kern, smem));
             HM_TRY(prefer_shared(kern));
-            // about kRingSegsPerWarp segments per warp: CTAs retire through the
-            // product and hand their slots to the tree passes on the side stream;
-            // fewer per warp where that would leave SMs short of 16 warps each
-            const int64_t spw = std::max<int64_t>(
-                1, std::min<int64_t>(kRingSegsPerWarp, h->n_segs / ((int64_t)16 * std::max(h->sms, 1))));
+            // the same number of segments for every warp, about kRingWaves waves of the CTAs
+            // that fit on the chip: CTAs retire through the product and hand their slots to
+            // the tree passes on the side stream.  With few waves the last, partial one
+            // cost a whole one: 8 right-hand sides, near field alone, us, 1.1 waves
+            // against 3 to 6: 128 instances 529 / 386, n = 2^19 random points 169 / 140, grid
+            // 133 / 102; 1.3 segments per warp took 284 us per product where 1 took 261.
+            int per_sm = 0;
+            HM_TRY(ctas_per_sm(kern, 32 * kRingWarps, smem, &per_sm));
+            const int64_t most = (int64_t)kRingWaves * per_sm * kRingWarps * std::max(h->sms, 1);
+            const int64_t spw = std::min<int64_t>(kRingSegsPerWarp, (h->n_segs + most - 1) / most);
             const int64_t warps = (h->n_segs + spw - 1) / spw;
             const unsigned grid = (unsigned)((warps + kRingWarps - 1) / kRingWarps);
             HM_TRY(launch_k(FAR ? "ring_far" : "ring_near", kern, dim3(grid), dim3(32 * kRingWarps), smem, st,

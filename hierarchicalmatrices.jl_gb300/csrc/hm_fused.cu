@@ -167,7 +167,8 @@ namespace {
 
 // The near-field sums of 3 to 8 FP32 right-hand sides in ring_part's order:
 // chunks of at most 32 columns and pf panel values, the partial sums folded
-// before a chunk that would take them past 64 columns.
+// before a chunk that would take them past 64 columns, a chunk's columns dealt out to
+// the lane groups of a low segment.
 template <int KB>
 __device__ __forceinline__ void seg_columns_ring(const float *Pg, int ld, const float *g, int c0, int c1, int pf,
                                                  float (&val)[KB][2])
@@ -175,10 +176,39 @@ __device__ __forceinline__ void seg_columns_ring(const float *Pg, int ld, const 
     const int lane = threadIdx.x & 31;
     SegAcc<float, KB> a0, a1;
     a0.zero(); a1.zero();
-    if (2 * lane < ld) {
+    const int64_t ld2 = ld / 2;
+    const int cc = min(kRingCols, pf / max(ld, 4)), cg = ring_groups(ld);
+    if (cg > 1) {
+        const int lr = lane & (32 / cg - 1);
+        const float2 *base = reinterpret_cast<const float2 *>(Pg + 2 * lr);
+        int nfold = 0;
+        for (int c = c0; c < c1; c += cc) {
+            const int n = min(cc, c1 - c);
+            if (nfold + n > 64) {
+                a0.fold(); a1.fold();
+                nfold = 0;
+            }
+            nfold += n;
+            if (2 * lr >= ld) continue;
+            for (int u = lane / (32 / cg); u < n; u += 4 * cg) {
+                float2 p[4];
+#pragma unroll
+                for (int v = 0; v < 4; ++v)
+                    if (u + v * cg < n) p[v] = __ldcs(base + ld2 * (c + u + v * cg));
+#pragma unroll
+                for (int v = 0; v < 4; ++v)
+                    if (u + v * cg < n) {
+                        float gv[KB];
+                        ld_vec<KB>(g + (c + u + v * cg) * KB, gv);
+                        a0.add(p[v].x, gv); a1.add(p[v].y, gv);
+                    }
+            }
+        }
+        a0.fold(); a1.fold();
+        ring_combine<KB>(32 / cg, [&](int i, int q) -> float & { return i ? a1.h[q] : a0.h[q]; },
+                         [&](int i, int q) -> float & { return i ? a1.l[q] : a0.l[q]; });
+    } else if (2 * lane < ld) {
         const float2 *base = reinterpret_cast<const float2 *>(Pg + 2 * lane);
-        const int64_t ld2 = ld / 2;
-        const int cc = min(kRingCols, pf / max(ld, 4));
         int left = 0, nfold = 0;
         auto use = [&](const float2 &p, int c) {
             if (left == 0) {

@@ -255,7 +255,8 @@ __global__ void stream_part(MulArgs<S> ma, const hm_seg *segs, const int *cta_se
 // poff % 4 == 0.  Grid: a whole number of CTAs of kRingWarps warps, shared
 // memory ring_smem_bytes(KB, PF, NS).
 constexpr int kRingWarps = 2;
-constexpr int kRingSegsPerWarp = 24;      // segments per warp (the launch's grid follows from it)
+constexpr int kRingSegsPerWarp = 24;      // segments per warp at most
+constexpr int kRingWaves = 6;              // waves of CTAs aimed at
 constexpr int kRingCols = 32;              // columns per chunk at most (lane c gathers column c)
 // The compiled tiles: panel values per stage (at most) and stages.
 struct RingTile { int pf, ns; };

@@ -15,24 +15,32 @@
 // 2l+1 of the current segment (8-byte reads of the staged columns) and
 // accumulates KB right-hand sides with FMA, folding the partial sums into
 // compensated (TwoSum) pairs at most every 64 columns, as the per-segment warp
-// kernel does.  Only cp.async groups of the warp's own lanes are waited on
+// kernel does; each two adjacent right-hand sides go out as one packed FP32x2 FMA.
+// Segments of 32, 16 or 8 rows and fewer (random points: clusters of 64 to 79 points
+// leave a segment of 1 to 15 behind one of 64) take 2, 4 or 8 columns at once, a group
+// of lanes each (ring_groups), combined with TwoSum at the segment's end.  Only cp.async groups of the warp's own lanes are waited on
 // (cp.async.wait_group, then __syncwarp): no barrier spans warps or kernels.
 #include "hm_kernels.cuh"
 #include "hm_async.cuh"
+#include "hm_tree.cuh"
 
 namespace hm {
 
 namespace {
 
 template <int KB>
-struct RingAcc {     // two rows x KB right-hand sides: FMA partials folded into (hi, lo) pairs
-    float part[2][KB], hi[2][KB], lo[2][KB];
+struct RingAcc {     // two rows x KB right-hand sides: FMA partials (pairs of right-hand sides) folded into (hi, lo) pairs
+    float2 part[2][KB / 2];
+    float hi[2][KB], lo[2][KB];
     __device__ __forceinline__ void zero()
     {
 #pragma unroll
         for (int i = 0; i < 2; ++i)
 #pragma unroll
-            for (int q = 0; q < KB; ++q) part[i][q] = hi[i][q] = lo[i][q] = 0.f;
+            for (int q = 0; q < KB; ++q) {
+                hi[i][q] = lo[i][q] = 0.f;
+                part[i][q / 2] = make_float2(0.f, 0.f);
+            }
     }
     __device__ __forceinline__ void fold()
     {
@@ -40,9 +48,23 @@ struct RingAcc {     // two rows x KB right-hand sides: FMA partials folded into
         for (int i = 0; i < 2; ++i)
 #pragma unroll
             for (int q = 0; q < KB; ++q) {
-                hm::fold(hi[i][q], lo[i][q], part[i][q]);
-                part[i][q] = 0.f;
+                hm::fold(hi[i][q], lo[i][q], q & 1 ? part[i][q / 2].y : part[i][q / 2].x);
+                if (q & 1) part[i][q / 2] = make_float2(0.f, 0.f);
             }
+    }
+    // one column: rows (p.x, p.y), right-hand sides g[0 .. KB)
+    __device__ __forceinline__ void add(const float2 &p, const float4 *g)
+    {
+        const float2 px = make_float2(p.x, p.x), py = make_float2(p.y, p.y);
+#pragma unroll
+        for (int v = 0; v < KB / 4; ++v) {
+            const float4 g4 = g[v];
+            const float2 a = make_float2(g4.x, g4.y), b = make_float2(g4.z, g4.w);
+            part[0][2 * v] = __ffma2_rn(px, a, part[0][2 * v]);
+            part[0][2 * v + 1] = __ffma2_rn(px, b, part[0][2 * v + 1]);
+            part[1][2 * v] = __ffma2_rn(py, a, part[1][2 * v]);
+            part[1][2 * v + 1] = __ffma2_rn(py, b, part[1][2 * v + 1]);
+        }
     }
 };
 
@@ -163,6 +185,8 @@ __global__ void __launch_bounds__(kRingWarps * 32)
     };
     auto finish = [&]() {
         acc.fold();
+        ring_combine<KB>(32 / ring_groups(cld), [&](int i, int q) -> float & { return acc.hi[i][q]; },
+                         [&](int i, int q) -> float & { return acc.lo[i][q]; });
 #pragma unroll
         for (int q = 0; q < KB; ++q) {
             if (q >= k) break;
@@ -209,29 +233,28 @@ __global__ void __launch_bounds__(kRingWarps * 32)
             nfold = 0;
         }
         nfold += cols;
-        if (2 * lane < cld) {
-            const float *pr = sp + 2 * lane;
+        const int cg = ring_groups(cld), lr = lane & (32 / cg - 1);
+        if (2 * lr < cld) {
+            const float *pr = sp + 2 * lr;
             const float4 *gr = reinterpret_cast<const float4 *>(sg);
-            auto column = [&](const float *pc, const float4 *gc) {
-                const float2 p = *reinterpret_cast<const float2 *>(pc);
-                float g[KB];
-#pragma unroll
-                for (int v = 0; v < KB / 4; ++v) {
-                    const float4 g4 = gc[v];
-                    g[4 * v] = g4.x; g[4 * v + 1] = g4.y; g[4 * v + 2] = g4.z; g[4 * v + 3] = g4.w;
-                }
-#pragma unroll
-                for (int q = 0; q < KB; ++q) {
-                    acc.part[0][q] = fmaf(p.x, g[q], acc.part[0][q]);
-                    acc.part[1][q] = fmaf(p.y, g[q], acc.part[1][q]);
-                }
+            auto column = [&](int u) {
+                acc.add(*reinterpret_cast<const float2 *>(pr + u * cld), gr + u * (KB / 4));
             };
-            int u = 0;
-            for (; u + 8 <= cols; u += 8) {
+            if (cg == 1) {
+                int u = 0;
+                for (; u + 8 <= cols; u += 8) {
 #pragma unroll
-                for (int v = 0; v < 8; ++v) column(pr + (u + v) * cld, gr + (u + v) * (KB / 4));
+                    for (int v = 0; v < 8; ++v) column(u + v);
+                }
+                for (; u < cols; ++u) column(u);
+            } else {
+                int u = lane / (32 / cg);
+                for (; u + 3 * cg < cols; u += 4 * cg) {
+#pragma unroll
+                    for (int v = 0; v < 4; ++v) column(u + v * cg);
+                }
+                for (; u < cols; u += cg) column(u);
             }
-            for (; u < cols; ++u) column(pr + u * cld, gr + u * (KB / 4));
         }
         cc += cols;
         if (cc >= cce) {

@@ -545,6 +545,28 @@ struct SegAcc {
 };
 
 
+// Columns of a segment that ring_part takes at once: lane groups of 32 / that many
+// lanes, two rows a lane.
+__device__ __forceinline__ int ring_groups(int ld) { return ld > 32 ? 1 : ld > 16 ? 2 : ld > 8 ? 4 : 8; }
+// The groups' (hi, lo) sums of two rows and KB right-hand sides added into every group
+// of `lanes` lanes (TwoSum: the same in each of them).
+template <int KB, typename H, typename L>
+__device__ __forceinline__ void ring_combine(int lanes, H hi, L lo)
+{
+    for (int o = lanes; o < 32; o <<= 1) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int q = 0; q < KB; ++q) {
+                const float h = hi(i, q), so = __shfl_xor_sync(0xffffffffu, h, o);
+                const float l = lo(i, q) + __shfl_xor_sync(0xffffffffu, lo(i, q), o);
+                const float t = h + so, bp = t - h;
+                hi(i, q) = t;
+                lo(i, q) = l + ((h - (t - bp)) + (so - bp));
+            }
+    }
+}
+
 // The rows of a segment (<= 64) a lane sums: with one or two FP32 right-hand
 // sides lanes 0-15 and 16-31 take alternate columns, each lane four
 // consecutive rows (one 16-byte load per column; lanes 0-15 hold the sums);
