@@ -210,7 +210,8 @@ __global__ void __launch_bounds__(kWideWarps * 32)
     // multiple of 4 and right-hand sides past the chunk are zero-filled
     const int nr4 = (nr + 3) & ~3;
     constexpr int VW = 16 / sizeof(A);                         // values per 16-byte copy
-    if (ma.incx == 1 && Pn.row0 % VW == 0 && ma.ldx % VW == 0 && nr % VW == 0) {
+    if (ma.incx == 1 && Pn.row0 % VW == 0 && ma.ldx % VW == 0 && nr % VW == 0 &&
+        (reinterpret_cast<uintptr_t>(ma.x) & 15) == 0) {
         // rows of every right-hand side start on a 16-byte boundary: 16-byte copies,
         // lane (q, piece) over the QW x nr / VW pieces
         const int per_q = nr / VW;
