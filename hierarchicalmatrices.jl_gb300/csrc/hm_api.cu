@@ -7,11 +7,13 @@
 #include <cstdio>
 #include <cstring>
 #include <algorithm>
+#include <array>
 #include <atomic>
 #include <map>
 #include <set>
 #include <thread>
 #include <tuple>
+#include <memory>
 #include <mutex>
 #include <string>
 #include <type_traits>
@@ -285,6 +287,30 @@ struct hm_handle {
     bool tensor_cores = true;       // use it for FP32 products with many right-hand sides
 
     std::mutex mu;
+    // The launches of one form of product (a key of everything they depend on but the
+    // vectors' addresses) as a CUDA graph; `args` are its kernels that take the vectors.
+    struct ProductGraph {
+        std::array<int64_t, 20> key;
+        int seen = 0;
+        bool bad = false;           // could not be captured: plain launches
+        uint64_t used = 0;
+        cudaGraph_t graph = nullptr;
+        cudaGraphExec_t exec = nullptr;
+        struct Arg {
+            cudaGraphNode_t node;
+            cudaKernelNodeParams p;
+            std::vector<void *> params;
+        };
+        std::vector<Arg> args;
+        const void *x = nullptr;
+        void *y = nullptr;
+        ~ProductGraph()
+        {
+            if (exec) cudaGraphExecDestroy(exec);
+            if (graph) cudaGraphDestroy(graph);
+        }
+    };
+
     // Per caller stream: coefficient scratch (grown stream-ordered), the side
     // stream of the tree passes and the fork/join events.
     struct StreamCtx {
@@ -296,6 +322,9 @@ struct hm_handle {
         cudaStream_t side = nullptr;
         cudaEvent_t fork = nullptr, join = nullptr;
         cudaEvent_t mid = nullptr;  // a point inside the tree passes where the near field may start
+        std::mutex graph_mu;        // graphs, and their updates and launches
+        std::vector<std::unique_ptr<ProductGraph>> graphs;
+        uint64_t graph_clock = 0;
     };
     std::map<void *, StreamCtx> streams;
     void *d_stage = nullptr;
@@ -1715,19 +1744,169 @@ int launch_pipeline(hm_handle *h, const MulArgs<S> &ma, cudaStream_t st, cudaStr
     return launch_expand_k<S, A>(h, ma, s, t, panels, st);
 }
 
+// A product of a middle size is some 12 launches and 6 event calls, 45 to 60 us of
+// host time, longer than its kernels take; as a graph it is one launch, after the
+// addresses of the vectors have been set in the three or four kernels that take them.
+// Per StreamCtx (scratch belongs to it), for up to kGraphs forms of product; a form
+// is captured at its kGraphAfter-th product and runs plainly before.  A product on a
+// capturing stream, with stage timing or with host vectors runs plainly.
+constexpr size_t kGraphs = 8;
+constexpr int kGraphAfter = 3;
+
+// Where the graph is the faster form, us per product, plain / graph, on a grid and
+// on random points: FP32, 1 right-hand side: n = 2^14 35.1 / 21.4 and 33.2 / 25.1, 2^17
+// 50.1 / 42.5 and 53.3 / 47.8, 2^20 212 / 204 and 264 / 258; 8: 2^17 82 / 76 and 89 / 86,
+// but 2^18 120 / 118 and 140 / 150, 2^19 200 / 201 and 254 / 259.  FP64, 1: 2^16 138 / 95
+// and 126 / 113, 2^20 674 / 657 and 886 / 872; 8: 2^15 343 / 331 and 443 / 436, but 2^16 558
+// / 670 and 653 / 636 (the near field then takes the SMs before the far-field stage).
+// HM_DF64, 1: 2^16 112 / 106 and 120 / 116; 8: 222 / 208 and 309 / 297.
+template <typename S>
+bool graph_pays(const hm_handle *h, int k)
+{
+    const int slots = std::max(h->n_xslots, h->n_yslots);
+    if (k <= 2 || k > kPartMaxK || h->storage == HM_DF64 || slots < 2048) return true;
+    return sizeof(S) == 4 && (k <= 4 || slots < 8192);
+}
+
+template <typename S, typename A>
+int capture_product(hm_handle *h, hm_handle::StreamCtx *sc, hm_handle::ProductGraph &g, const MulArgs<S> &ma,
+                    cudaStream_t st, const Sched &run, const void *panels)
+{
+    // streams and events of its own: another thread may be issuing on the context's
+    struct Own {
+        cudaStream_t cap = nullptr, side = nullptr;
+        cudaEvent_t fork = nullptr, join = nullptr, mid = nullptr;
+        ~Own()
+        {
+            if (fork) cudaEventDestroy(fork);
+            if (join) cudaEventDestroy(join);
+            if (mid) cudaEventDestroy(mid);
+            if (side) cudaStreamDestroy(side);
+            if (cap) cudaStreamDestroy(cap);
+        }
+    } o;
+    int prio = 0, least = 0, greatest = 0;
+    HM_CK(cudaStreamGetPriority(st, &prio));
+    HM_CK(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+    HM_CK(cudaStreamCreateWithPriority(&o.cap, cudaStreamNonBlocking, prio));
+    HM_CK(cudaStreamCreateWithPriority(&o.side, cudaStreamNonBlocking, greatest));
+    HM_CK(cudaEventCreateWithFlags(&o.fork, cudaEventDisableTiming));
+    HM_CK(cudaEventCreateWithFlags(&o.join, cudaEventDisableTiming));
+    HM_CK(cudaEventCreateWithFlags(&o.mid, cudaEventDisableTiming));
+    HM_CK(cudaStreamBeginCapture(o.cap, cudaStreamCaptureModeRelaxed));
+    const int rc = launch_pipeline<S, A>(h, ma, o.cap, run.overlap ? o.side : o.cap, o.fork, o.join, sc->p, false, panels,
+                                         run.overlap >= 2 && ma.k <= kPartMaxK ? o.mid : nullptr, sc->sync);
+    const cudaError_t ec = cudaStreamEndCapture(o.cap, &g.graph);
+    if (rc) return rc;
+    HM_CK(ec);
+    size_t n = 0;
+    HM_CK(cudaGraphGetNodes(g.graph, nullptr, &n));
+    std::vector<cudaGraphNode_t> nodes(n);
+    HM_CK(cudaGraphGetNodes(g.graph, nodes.data(), &n));
+    for (cudaGraphNode_t node : nodes) {
+        cudaGraphNodeType type;
+        HM_CK(cudaGraphNodeGetType(node, &type));
+        if (type != cudaGraphNodeTypeKernel) continue;
+        hm_handle::ProductGraph::Arg a;
+        a.node = node;
+        HM_CK(cudaGraphKernelNodeGetParams(node, &a.p));
+        size_t off = 0, size = 0;
+        int np = 0;
+        while (cudaFuncGetParamInfo(a.p.func, np, &off, &size) == cudaSuccess) {
+            if (np == 0 && size != sizeof(MulArgs<S>)) break;          // does not take the vectors
+            a.params.push_back(a.p.kernelParams[np++]);
+        }
+        cudaGetLastError();                                            // past the last parameter
+        if (a.params.empty()) continue;
+        if (std::memcmp(a.params[0], &ma.x, sizeof(ma.x)) != 0) { set_error("graph node without the product's vectors"); return HM_ERR_CUDA; }
+        g.args.push_back(std::move(a));
+    }
+    HM_CK(cudaGraphInstantiate(&g.exec, g.graph, cudaGraphInstantiateFlagUseNodePriority));
+    g.x = ma.x;
+    g.y = ma.y;
+    return HM_OK;
+}
+
+// Runs the product as a graph; *done = false when it has to be launched plainly.
+template <typename S, typename A>
+int graph_mul(hm_handle *h, hm_handle::StreamCtx *sc, MulArgs<S> ma, cudaStream_t st, const Sched &run,
+              const void *panels, bool *done)
+{
+    *done = false;
+    if (ma.xin || ma.yout || h->profile_mask) return HM_OK;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &cs) != cudaSuccess) { cudaGetLastError(); return HM_OK; }
+    if (cs != cudaStreamCaptureStatusNone) return HM_OK;
+    const std::array<int64_t, 20> key = {
+        ma.incx, ma.ldx, ma.incy, ma.ldy, ma.k, ma.accumulate, (int64_t)(reinterpret_cast<uintptr_t>(ma.x) % 16 == 0),
+        (int64_t)reinterpret_cast<uintptr_t>(panels), (int64_t)reinterpret_cast<uintptr_t>(sc->p),
+        run.overlap, run.near_kernel, run.near_stages, run.tensor_cores, run.pdl, run.tile, run.wide,
+        (int64_t)h->wait_ns, h->test_stall, (int64_t)reinterpret_cast<uintptr_t>(sc->sync), sizeof(S)};
+    std::lock_guard<std::mutex> lk(sc->graph_mu);
+    hm_handle::ProductGraph *g = nullptr;
+    for (auto &q : sc->graphs)
+        if (q->key == key) g = q.get();
+    if (!g) {
+        if (sc->graphs.size() >= kGraphs) {
+            size_t old = 0;
+            for (size_t i = 1; i < sc->graphs.size(); ++i)
+                if (sc->graphs[i]->used < sc->graphs[old]->used) old = i;
+            sc->graphs.erase(sc->graphs.begin() + old);
+        }
+        sc->graphs.emplace_back(new hm_handle::ProductGraph());
+        g = sc->graphs.back().get();
+        g->key = key;
+    }
+    g->used = ++sc->graph_clock;
+    if (g->bad || ++g->seen < kGraphAfter) return HM_OK;
+    if (!g->exec) {
+        g->seen = kGraphAfter;
+        // the calls of a capture and an instantiation are legal beside another thread's
+        // capture only in the relaxed mode
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        const int rc = capture_product<S, A>(h, sc, *g, ma, st, run, panels);
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        if (rc) {
+            cudaGetLastError();
+            clear_last_error();
+            g->bad = true;
+            return HM_OK;
+        }
+    }
+    if (g->x != ma.x || g->y != ma.y) {
+        for (auto &a : g->args) {
+            a.params[0] = &ma;
+            a.p.kernelParams = a.params.data();
+            const int rc = cuda_status(cudaGraphExecKernelNodeSetParams(g->exec, a.node, &a.p), "cudaGraphExecKernelNodeSetParams");
+            if (rc) { g->bad = true; return rc; }
+        }
+        g->x = ma.x;
+        g->y = ma.y;
+    }
+    *done = true;
+    return cuda_status(cudaGraphLaunch(g->exec, st), "cudaGraphLaunch");
+}
+
 template <typename S, typename A>
 int run_mul(hm_handle *h, MulArgs<S> ma, cudaStream_t st, const void *panels = nullptr)
 {
     if (ma.k <= 0) return HM_OK;
+    const bool trial = t_sched != nullptr;                 // hm_autotune: plain launches of its candidates
     const Sched sched = sched_for(h, ma.k);
     SchedScope scope(&sched);
     hm_handle::StreamCtx *sc = nullptr;
     HM_TRY(stream_ctx(h, st, stream_scratch_bytes<A>(h, ma.k), &sc));
     if (fused_ok<S, A>(h, ma, sched)) return launch_fused<S, A>(h, ma, st, sc->p, sc->sync, panels ? panels : h->d_P);
-    StageTimer whole(h, 4, st);
     Sched run = sched;
     run.overlap = near_start(h, ma, sched.overlap);
     SchedScope staged(&run);
+    if (!trial && graph_pays<S>(h, ma.k)) {
+        bool done = false;
+        HM_TRY((graph_mul<S, A>(h, sc, ma, st, run, panels ? panels : h->d_P, &done)));
+        if (done) return HM_OK;
+    }
+    StageTimer whole(h, 4, st);
     // above kPartMaxK one panel kernel follows the tree passes: nothing waits for mid
     return launch_pipeline<S, A>(h, ma, st, run.overlap ? sc->side : st, sc->fork, sc->join, sc->p, true, panels,
                                  run.overlap >= 2 && ma.k <= kPartMaxK ? sc->mid : nullptr, sc->sync);
@@ -2825,6 +3004,7 @@ void hm_free(hm_handle *h)
     cudaDeviceSynchronize();
     if (h->trans) hm_free(h->trans);
     for (auto &kv : h->streams) {
+        kv.second.graphs.clear();
         if (kv.second.sync) cudaFree(kv.second.sync);
         if (kv.second.side) cudaStreamDestroy(kv.second.side);
         if (kv.second.fork) cudaEventDestroy(kv.second.fork);

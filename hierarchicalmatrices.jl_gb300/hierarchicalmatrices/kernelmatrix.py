@@ -272,7 +272,8 @@ class KernelMatrix:
         self.mul_drow(dyr, r, transposed=True, accumulate=False, stream=aux)
         gw = torch.empty(self.shape[1], dtype=w.dtype, device=w.device)
         self.mul_t(gw, r, accumulate=False, stream=cur)
-        loss = 0.5 * torch.dot(r.double(), r.double())
+        rd = r.double()
+        loss = 0.5 * torch.dot(rd, rd)
         cur.wait_stream(aux)                                   # the derivative products are done
         gx, gy = r * dxw, w * dyr
         return float(loss), gw, gx, gy
