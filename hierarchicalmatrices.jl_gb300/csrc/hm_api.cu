@@ -918,6 +918,13 @@ constexpr int kWideMinK = 32;                    // right-hand sides from which 
 constexpr int kWideMinK32 = 5;                   // ... of FP32 storage, from kWideSlots32 coefficient slots on
 constexpr int kWideSlots32 = 2048;
 
+// Whether eight panels or row slots per CTA (leaf_flat, m2l_flat) leave every SM one.
+// FP64, us per product, one per warp against eight per CTA: n = 2^14 (546 slots) 54.0 /
+// 58.0 on a grid, 60.0 / 62.9 on random points; 2^16 (2,184) 95.0 / 92.8, 107 / 106; 2^18 216
+// / 198, 272 / 257; 2^20 645 / 627, 867 / 837; 8 right-hand sides at 2^18 1,494 / 1,349,
+// 1,859 / 1,749.
+inline bool flat_fills(const hm_handle *h, int n) { return n >= kFlatRows * std::max(h->sms, 1); }
+
 // Index of the last non-empty band of a band pointer array, or -1.
 inline int last_band(const std::vector<int> &ptr)
 {
@@ -953,6 +960,17 @@ int launch_tree_qc(hm_handle *h, const MulArgs<S> &ma, cudaStream_t st, A *t, A 
                 leaf_up_df<<<warp_ctas(h->n_vp), 32 * kWarpsPerCta, smem, st>>>(
                     ma, h->d_vp, h->n_vp, static_cast<const float2 *>(h->d_V), t, r, h->vp_cap);
                 HM_CK_LAUNCH("leaf_up_df");
+                chain = true;
+                leaf_done = true;
+            }
+        }
+        if constexpr (std::is_same<S, double>::value && std::is_same<A, double>::value) {
+            if (!leaf_done && h->vp_wide && !ma.xin && !lp.rec && r == 20 && flat_fills(h, h->n_vp)) {
+                const size_t smem = (size_t)kFlatRows * h->vp_cap * QC * sizeof(double);
+                HM_TRY(ensure_smem(leaf_flat<QC>, smem));
+                leaf_flat<QC><<<dim3((unsigned)((h->n_vp + kFlatRows - 1) / kFlatRows), (unsigned)nq), kFlatThreads, smem, st>>>(
+                    ma, h->d_vp, h->n_vp, static_cast<const double *>(h->d_V), t, h->vp_cap);
+                HM_CK_LAUNCH("leaf_flat");
                 chain = true;
                 leaf_done = true;
             }
@@ -1045,6 +1063,17 @@ int launch_tree_qc(hm_handle *h, const MulArgs<S> &ma, cudaStream_t st, A *t, A 
                 HM_TRY(launch_k("m2l_k", m2l_k<S, A, QC>, dim3(h->n_m2l_rows), dim3(32 * kWarpsPerCta), smem, st,
                                 pdl_on && chain, h->d_m2l_rows, h->n_m2l_rows, h->d_m2l_ents,
                                 static_cast<const S *>(h->d_F), h->fstride, t, s, r, k));
+                chain = true;
+                done = true;
+            }
+        }
+        if constexpr (std::is_same<S, double>::value && std::is_same<A, double>::value) {
+            if (!done && r == 20 && h->fstride % 2 == 0 && flat_fills(h, h->n_m2l_rows)) {
+                HM_TRY(ensure_smem(m2l_flat<QC>, m2l_flat_bytes(QC)));
+                HM_TRY(launch_k("m2l_flat", m2l_flat<QC>,
+                                dim3((unsigned)((h->n_m2l_rows + kFlatRows - 1) / kFlatRows), (unsigned)nq),
+                                dim3(kFlatThreads), m2l_flat_bytes(QC), st, pdl_on && chain, h->d_m2l_rows,
+                                h->n_m2l_rows, h->d_m2l_ents, static_cast<const double *>(h->d_F), h->fstride, t, s, k));
                 chain = true;
                 done = true;
             }
@@ -1653,8 +1682,11 @@ int launch_fused(hm_handle *h, const MulArgs<S> &ma, cudaStream_t st, void *scra
 //   lane-per-right-hand-side tree kernels): 2^18 164 / 145 / 151, 2^19 330 / 286 / 269,
 //   128 instances 1,009 / 927 / 833.
 //   HM_DF64, 1: n = 2^15 108 / 84 / 86, 2^19 354 / 345 / 357, grid 2^19 288 / 264 /
-//   287; 2: 2^17 190 / 196 / 191.  FP64 (2^20 884 / 865 / 877, grid 672 / 676 / 672;
-//   k = 3, 2^17 590 / 634 / 629) has no line.
+//   287; 2: 2^17 190 / 196 / 191.
+//   FP64, 1: grid 2^16 95 / 107 / 129, 2^17 130 / 129 / 117 (random 206 / 151 / 171),
+//   grid 2^18 246 / 213 / 228, 2^20 636 / 645 / 625 (random 850 / 834 / 822); 2: 2^17 350 /
+//   311 / 343; 4: 2^18 1,009 / 966 / 1,072; 8: grid 2^16 655 / 474 / 495, 2^18 2,014 /
+//   1,775 / 1,860.
 template <typename S>
 int near_start(const hm_handle *h, const MulArgs<S> &ma, int overlap)
 {
@@ -1662,6 +1694,7 @@ int near_start(const hm_handle *h, const MulArgs<S> &ma, int overlap)
     const int slots = std::max(h->n_xslots, h->n_yslots), k = ma.k;
     int m = 2;
     if (h->storage == HM_DF64) m = k == 1 ? 4 : 2;
+    else if (sizeof(S) == 8) m = k <= 2 && slots >= 24576 ? 1 : k == 1 && slots < 4096 ? 2 : 4;
     else if (sizeof(S) == 4) m = k <= 2 ? (slots >= 8192 ? 4 : 2) : k <= 4 ? (slots >= 8192 ? 4 : 1)
                                  : (slots >= 2048 && slots < 16384 ? 4 : 1);
     return m == 1 && ma.xin ? 4 : m;

@@ -163,6 +163,67 @@ __global__ void leaf_up(MulArgs<S> ma, const hm_vpanel *vp, int npanels, const S
                          smem_raw + (size_t)wib * leaf_up_warp_bytes<S, A, QC>(cap, wcap), lp);
 }
 
+// FP64 leaf bases of rank 20, eight panels per CTA of five warps, thread (panel, m), for
+// the reason m2l_flat has: 160 threads hold the 160 coefficients of eight panels.  A
+// panel's rows stream from HBM (20 consecutive values a row, eight rows in flight),
+// the right-hand sides' rows are staged in shared memory.  The sums are those of
+// leaf_panel, in its order.  Upward half of the tree at n = 2^20: one right-hand side 145
+// -> 119 us, two 238 -> 197.
+template <int QC>
+__global__ void __launch_bounds__(kFlatThreads)
+    leaf_flat(MulArgs<double> ma, const hm_vpanel *vp, int npanels, const double *V, double *t, int cap)
+{
+    extern __shared__ __align__(16) double flat_smem[];
+    constexpr int R = 20;
+    const int i = threadIdx.x / R, m = threadIdx.x % R;
+    const int64_t p = (int64_t)blockIdx.x * kFlatRows + i;
+    const int k = ma.k, q0 = blockIdx.y * QC, qc = min(QC, k - q0);
+    pdl_trigger();
+    hm_vpanel P{};
+    if (p < npanels) P = vp[p];
+    double *xs = flat_smem + (size_t)i * cap * QC;             // [row][q]
+    for (int j = m; j < P.nrows; j += R) {
+#pragma unroll
+        for (int q = 0; q < QC; ++q) {
+            double *d = xs + j * QC + q;
+            if (q < qc) async_copy<8>(d, ma.x + (P.row0 + j) * ma.incx + (int64_t)(q0 + q) * ma.ldx);
+            else *d = 0.0;
+        }
+    }
+    async_commit();
+    const double *v = V + P.off + m;
+    double acc[QC];
+#pragma unroll
+    for (int q = 0; q < QC; ++q) acc[q] = 0.0;
+    constexpr int U = 8;
+    double next[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) next[u] = u < P.nrows ? v[R * u] : 0.0;
+    async_wait_all();
+    __syncthreads();                                           // x is staged
+    for (int j = 0; j < P.nrows; j += U) {
+        double vv[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            vv[u] = next[u];
+            if (j + U + u < P.nrows) next[u] = v[(int64_t)R * (j + U + u)];
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (j + u >= P.nrows) break;
+            double xv[QC];
+            ld_vec<QC>(xs + (j + u) * QC, xv);
+#pragma unroll
+            for (int q = 0; q < QC; ++q) acc[q] = fma(vv[u], xv[q], acc[q]);
+        }
+    }
+    if (p < npanels) {
+#pragma unroll
+        for (int q = 0; q < QC; ++q)
+            if (q < qc) t[((int64_t)P.slot * k + q0 + q) * R + P.col0 + m] = acc[q];
+    }
+}
+
 // Upward transfers of one band: t[parent][m] = sum_c sum_m' T_c[m', m] t[child_c][m'].
 // One CTA per task (a subtree cut to the band's levels); the task's steps
 // (levels, deepest first) run in order with a CTA barrier between them, warps
@@ -278,6 +339,84 @@ __global__ void m2l(const hm_m2l_row *rows, int nrows, const hm_m2l_ent *ents, c
     const int q0 = (int)(w % nq) * QC;
     if (r == 20) m2l_row<S, A, QC, 20>(R, q0, ents, F, fstride, t, s, r, k, smem);
     else m2l_row<S, A, QC, 0>(R, q0, ents, F, fstride, t, s, r, k, smem);
+}
+
+// FP64 far field, rank 20: eight row slots per CTA of five warps, thread (row, m).  An
+// FP64 warp instruction takes its 64 cycles with 20 lanes live as with 32, so one row
+// slot per warp (m2l) left three eighths of the pipe unused; here 160 threads hold 160
+// outputs.  Blocks (all eight rows' e-th at a time) and column coefficients are
+// double-buffered in shared memory, a row's by its own 20 threads.  The sums are those
+// of m2l_row, in its order.  Downward half of the tree at n = 2^20: one
+// right-hand side 181 -> 164 us, two 331 -> 286.
+template <int QC>
+__global__ void __launch_bounds__(kFlatThreads)
+    m2l_flat(const hm_m2l_row *rows, int nrows, const hm_m2l_ent *ents, const double *F, int fstride, const double *t,
+             double *s, int k)
+{
+    extern __shared__ __align__(16) double flat_smem[];
+    constexpr int R = 20, LD = R * R + kFlatPad;               // values between the rows' blocks
+    const int i = threadIdx.x / R, m = threadIdx.x % R;
+    const int row = blockIdx.x * kFlatRows + i, q0 = blockIdx.y * QC, qc = min(QC, k - q0);
+    double *Fb = flat_smem;                                    // [stage][row][LD]
+    double *Tb = Fb + 2 * kFlatRows * LD;                      // [stage][row][q][R]
+    pdl_trigger();
+    hm_m2l_row Rw{};
+    if (row < nrows) Rw = rows[row];
+    const int nb = Rw.end - Rw.begin;
+    __shared__ int s_most;
+    if (threadIdx.x == 0) s_most = 0;
+    __syncthreads();
+    if (m == 0) atomicMax(&s_most, nb);
+    auto block = [&](int e) {
+        if (e >= nb) return;
+        const char *src = reinterpret_cast<const char *>(F + ents[Rw.begin + e].foff);
+        char *dst = reinterpret_cast<char *>(Fb + ((e & 1) * kFlatRows + i) * LD);
+#pragma unroll
+        for (int c = 0; c < R * R / 2; c += R) async_copy16(dst + 16 * (c + m), src + 16 * (c + m));
+    };
+    auto coefs = [&](int e) {
+        if (e >= nb) return;
+        const double *src = t + ((int64_t)ents[Rw.begin + e].yslot * k + q0) * R + m;
+        double *dst = Tb + ((e & 1) * kFlatRows + i) * QC * R + m;
+#pragma unroll
+        for (int q = 0; q < QC; ++q) {
+            if (q < qc) async_copy<8>(dst + q * R, src + q * R);
+            else dst[q * R] = 0.0;
+        }
+    };
+    block(0);                                                  // F does not depend on the upward pass
+    pdl_wait();
+    coefs(0);
+    async_commit();
+    double acc[QC];
+#pragma unroll
+    for (int q = 0; q < QC; ++q) acc[q] = 0.0;
+    __syncthreads();
+    const int most = s_most;
+    for (int e = 0; e < most; ++e) {
+        block(e + 1);
+        coefs(e + 1);
+        async_commit();
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncthreads();                                       // the rows' copies are visible
+        if (e < nb) {
+            const double *f = Fb + ((e & 1) * kFlatRows + i) * LD + m;
+            const double *tv = Tb + ((e & 1) * kFlatRows + i) * QC * R;
+#pragma unroll
+            for (int n = 0; n < R; ++n) {
+                const double fv = f[R * n];
+#pragma unroll
+                for (int q = 0; q < QC; ++q) acc[q] = fma(fv, tv[q * R + n], acc[q]);
+            }
+        }
+        __syncthreads();                                       // the stage is refilled by the next step
+    }
+    async_wait_all();
+    if (row < nrows) {
+#pragma unroll
+        for (int q = 0; q < QC; ++q)
+            if (q < qc) s[((int64_t)Rw.slot * k + q0 + q) * R + m] = acc[q];
+    }
 }
 
 // Far field for many right-hand sides (k > QC): one CTA (4 warps) per row
@@ -985,6 +1124,11 @@ __global__ void expand_k(MulArgs<S> ma, const hm_seg *segs, const hm_piece *piec
                                                          const hm_piece *, const S *, const A *, const A *,  \
                                                          int, int, int, int, int, S *, int *,           \
                                                          unsigned long long, int);
+#define HM_INST_FLAT(QC)                                                                                  \
+    template __global__ void m2l_flat<QC>(const hm_m2l_row *, int, const hm_m2l_ent *, const double *, int, \
+                                          const double *, double *, int);                                  \
+    template __global__ void leaf_flat<QC>(MulArgs<double>, const hm_vpanel *, int, const double *, double *, int);
+HM_INST_FLAT(1) HM_INST_FLAT(2) HM_INST_FLAT(4) HM_INST_FLAT(8)
 #define HM_INST_FAR(S, A, KB)                                                                        \
     template __global__ void far_rows<S, A, KB>(MulArgs<S>, const hm_seg *, int, const hm_piece *, const S *, \
                                                 const A *, const A *, int, S *, int64_t);

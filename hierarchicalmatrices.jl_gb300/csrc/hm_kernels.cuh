@@ -205,6 +205,22 @@ template <typename S, typename A, int QC>
 __global__ void m2l(const hm_m2l_row *rows, int nrows, const hm_m2l_ent *ents, const S *F, int fstride,
                     const A *t, A *s, int r, int k);
 
+// m2l_flat: FP64, rank 20, 16-byte aligned blocks (fstride even); grid (row slots /
+// kFlatRows, chunks), shared memory m2l_flat_bytes(QC).
+constexpr int kFlatRows = 8, kFlatThreads = kFlatRows * 20;
+constexpr int kFlatPad = 8;     // a warp reads the ends of two rows' blocks: other banks (64 bytes on)
+__host__ __device__ constexpr size_t m2l_flat_bytes(int qc)
+{
+    return 2 * kFlatRows * (size_t)(400 + kFlatPad + 20 * qc) * sizeof(double);
+}
+// leaf_flat: panels row-major with ld == width == 20 and at most cap rows, grid (panels /
+// kFlatRows, chunks), shared memory kFlatRows * cap * QC values.
+template <int QC>
+__global__ void leaf_flat(MulArgs<double> ma, const hm_vpanel *vp, int npanels, const double *V, double *t, int cap);
+template <int QC>
+__global__ void m2l_flat(const hm_m2l_row *rows, int nrows, const hm_m2l_ent *ents, const double *F, int fstride,
+                         const double *t, double *s, int k);
+
 template <typename S, typename A, int QC>
 __global__ void m2l_k(const hm_m2l_row *rows, int nrows, const hm_m2l_ent *ents, const S *F, int fstride,
                       const A *t, A *s, int r, int k);
