@@ -280,46 +280,58 @@ __device__ __forceinline__ void xfer_up_fetch(const TaskRecs &R, const A *t, A *
 // use them: the level walks are latency bound (a 100,003 x 77,777 FP32 matrix
 // with 3 right-hand sides 84.6 -> 74.6 us per product, n = 2^20 with one 233 ->
 // 226 us).
+// f(e, m) for every output m of the records e of a step: a warp per record, lane m;
+// FP64 rank 20 a thread per output, 160 of them for eight records (an FP64 warp
+// instruction takes as long for 20 lanes as for 32).
+template <typename A, int RC, typename F>
+__device__ __forceinline__ void task_outputs(const hm_step S, int r, F f)
+{
+    if constexpr (sizeof(A) == 8 && RC == 20) {
+        for (int u = threadIdx.x; u < (S.e1 - S.e0) * RC; u += blockDim.x) f(S.e0 + u / RC, u % RC);
+    } else {
+        const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+        if (lane >= r) return;
+        for (int e = S.e0 + (threadIdx.x >> 5); e < S.e1; e += nw) f(e, lane);
+    }
+}
+
 template <typename A, int QC, int RC>
 __device__ __forceinline__ void xfer_up_levels(const TaskRecs &R, const A *Ts, A *t, A *L, int rr, int k, int q0)
 {
     const int r = RC ? RC : rr;
     const int qc = min(QC, k - q0);
-    const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     for (int st = 0; st < R.nsteps; ++st) {
         const hm_step S = R.step[st];
-        for (int e = S.e0 + (threadIdx.x >> 5); e < S.e1; e += nw) {
+        task_outputs<A, RC>(S, r, [&](int e, int lane) {
             const hm_xfer X = R.x[e];
             const A *c0 = L + (int64_t)(X.pad & 0xffff) * QC * r;
             const A *c1 = L + (int64_t)(X.pad >> 16) * QC * r;
             A *out = L + (int64_t)e * QC * r;
-            if (lane < r) {
-                // one sum per child: an FMA per term (a0 v0 + a1 v1 in one expression
-                // is three operations), and neither sum is rounded more often than
-                // when the pair was added first
-                A s0[QC], s1[QC];
+            // one sum per child: an FMA per term (a0 v0 + a1 v1 in one expression
+            // is three operations), and neither sum is rounded more often than
+            // when the pair was added first
+            A s0[QC], s1[QC];
 #pragma unroll
-                for (int qq = 0; qq < QC; ++qq) s0[qq] = s1[qq] = 0;
+            for (int qq = 0; qq < QC; ++qq) s0[qq] = s1[qq] = 0;
 #pragma unroll(RC ? RC : 4)
-                for (int mp = 0; mp < r; ++mp) {
-                    const A a0 = Ts[mp * r + lane], a1 = Ts[r * r + mp * r + lane];
-                    A v0[QC], v1[QC];
-                    ld_vec<QC>(c0 + mp * QC, v0);
-                    ld_vec<QC>(c1 + mp * QC, v1);
-#pragma unroll
-                    for (int qq = 0; qq < QC; ++qq) {
-                        s0[qq] = fma(a0, v0[qq], s0[qq]);
-                        s1[qq] = fma(a1, v1[qq], s1[qq]);
-                    }
-                }
+            for (int mp = 0; mp < r; ++mp) {
+                const A a0 = Ts[mp * r + lane], a1 = Ts[r * r + mp * r + lane];
+                A v0[QC], v1[QC];
+                ld_vec<QC>(c0 + mp * QC, v0);
+                ld_vec<QC>(c1 + mp * QC, v1);
 #pragma unroll
                 for (int qq = 0; qq < QC; ++qq) {
-                    const A sum = s0[qq] + s1[qq];
-                    out[lane * QC + qq] = sum;
-                    if (qq < qc) t[((int64_t)X.slot * k + q0 + qq) * r + lane] = sum;
+                    s0[qq] = fma(a0, v0[qq], s0[qq]);
+                    s1[qq] = fma(a1, v1[qq], s1[qq]);
                 }
             }
-        }
+#pragma unroll
+            for (int qq = 0; qq < QC; ++qq) {
+                const A sum = s0[qq] + s1[qq];
+                out[lane * QC + qq] = sum;
+                if (qq < qc) t[((int64_t)X.slot * k + q0 + qq) * r + lane] = sum;
+            }
+        });
         __syncthreads();
     }
 }
@@ -361,61 +373,58 @@ __device__ __forceinline__ void xfer_down_levels(const TaskRecs &R, const A *Ts,
 {
     const int r = RC ? RC : rr;
     const int qc = min(QC, k - q0);
-    const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     for (int st = 0; st < R.nsteps; ++st) {
         const hm_step S = R.step[st];
-        for (int e = S.e0 + (threadIdx.x >> 5); e < S.e1; e += nw) {
+        task_outputs<A, RC>(S, r, [&](int e, int lane) {
             const hm_xfer X = R.x[e];
             const A *p = L + (int64_t)X.pad * QC * r;
             A *o0 = L + (int64_t)(2 * e) * QC * r;
             A *o1 = o0 + QC * r;
-            if (lane < r) {
-                A a0[QC], a1[QC];
+            A a0[QC], a1[QC];
 #pragma unroll
-                for (int qq = 0; qq < QC; ++qq) { a0[qq] = 0; a1[qq] = 0; }
-                const A *Tl = Ts + lane * r, *Tr = Tl + r * r;
-                if constexpr (RC % 4 == 0 && RC > 0) {
-                    // rows of T and of the parent in 16-byte loads
+            for (int qq = 0; qq < QC; ++qq) { a0[qq] = 0; a1[qq] = 0; }
+            const A *Tl = Ts + lane * r, *Tr = Tl + r * r;
+            if constexpr (RC % 4 == 0 && RC > 0) {
+                // rows of T and of the parent in 16-byte loads
 #pragma unroll
-                    for (int m = 0; m < RC; m += 4) {
-                        A t0[4], t1[4];
-                        ld_vec<4>(Tl + m, t0);
-                        ld_vec<4>(Tr + m, t1);
+                for (int m = 0; m < RC; m += 4) {
+                    A t0[4], t1[4];
+                    ld_vec<4>(Tl + m, t0);
+                    ld_vec<4>(Tr + m, t1);
 #pragma unroll
-                        for (int qq = 0; qq < QC; ++qq) {
-                            A v[4];
-                            ld_vec<4>(p + qq * RC + m, v);
+                    for (int qq = 0; qq < QC; ++qq) {
+                        A v[4];
+                        ld_vec<4>(p + qq * RC + m, v);
 #pragma unroll
-                            for (int u = 0; u < 4; ++u) {
-                                a0[qq] += t0[u] * v[u];
-                                a1[qq] += t1[u] * v[u];
-                            }
-                        }
-                    }
-                } else {
-#pragma unroll 4
-                    for (int m = 0; m < r; ++m) {
-                        const A t0 = Tl[m], t1 = Tr[m];
-#pragma unroll
-                        for (int qq = 0; qq < QC; ++qq) {
-                            const A v = p[qq * r + m];
-                            a0[qq] += t0 * v;
-                            a1[qq] += t1 * v;
+                        for (int u = 0; u < 4; ++u) {
+                            a0[qq] += t0[u] * v[u];
+                            a1[qq] += t1[u] * v[u];
                         }
                     }
                 }
+            } else {
+#pragma unroll 4
+                for (int m = 0; m < r; ++m) {
+                    const A t0 = Tl[m], t1 = Tr[m];
 #pragma unroll
-                for (int qq = 0; qq < QC; ++qq) {
-                    const A v0 = o0[qq * r + lane] + a0[qq], v1 = o1[qq * r + lane] + a1[qq];
-                    o0[qq * r + lane] = v0;
-                    o1[qq * r + lane] = v1;
-                    if (qq < qc) {
-                        s[((int64_t)X.c0 * k + q0 + qq) * r + lane] = v0;
-                        s[((int64_t)X.c1 * k + q0 + qq) * r + lane] = v1;
+                    for (int qq = 0; qq < QC; ++qq) {
+                        const A v = p[qq * r + m];
+                        a0[qq] += t0 * v;
+                        a1[qq] += t1 * v;
                     }
                 }
             }
-        }
+#pragma unroll
+            for (int qq = 0; qq < QC; ++qq) {
+                const A v0 = o0[qq * r + lane] + a0[qq], v1 = o1[qq * r + lane] + a1[qq];
+                o0[qq * r + lane] = v0;
+                o1[qq * r + lane] = v1;
+                if (qq < qc) {
+                    s[((int64_t)X.c0 * k + q0 + qq) * r + lane] = v0;
+                    s[((int64_t)X.c1 * k + q0 + qq) * r + lane] = v1;
+                }
+            }
+        });
         __syncthreads();
     }
 }
