@@ -1318,7 +1318,7 @@ int launch_part_kb(hm_handle *h, const MulArgs<S> &ma, const A *s, const A *t, c
             return launch_df<FAR ? 1 : 0, KB>(h, ma, s, t, panels, yfar, st, pdl, ldf, 0);
         }
     }
-    if constexpr (FAR && KB >= 4 && std::is_same<S, A>::value) {
+    if constexpr (FAR && (KB >= 4 || sizeof(S) == 8) && std::is_same<S, A>::value) {
         // far-field rows one thread per row for 3-8 right-hand sides (the default
         // and ring schedules; the warp and streamed kernels keep their own
         // far-field form).  Measured: 512-instance batch at 8, 0.55 against
