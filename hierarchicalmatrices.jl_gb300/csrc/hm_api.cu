@@ -1532,19 +1532,19 @@ bool fused_ok(const hm_handle *h, const MulArgs<S> &ma, const Sched &sc)
     const size_t kb = ma.k > kPartMaxK ? 0 : ma.k > 4 ? 8 : ma.k > 2 ? 4 : 2;
     if (!fits || kWarpsPerCta * (size_t)h->max_width * kb * (df ? sizeof(float2) : sizeof(A)) > 100 * 1024) return false;
     // The lines, in coefficient slots (about n / 30), where the cluster's 16 SMs
-    // take as long as the stage kernels on all of them (us, fused against stages):
-    // FP32, 1 right-hand side: 21.7 / 30.8 at 144, 24.9 / 30.5 at 272, 38.3 / 33.1
-    // at 578; 8: 33.7 / 41.3 at 144, 42.0 / 41.8 at 272; 16: 41.4 / 43.9 at 60, 54.7
-    // / 51.7 at 144.  FP64, 1: 47.5 / 64.5 at 144, 61.9 / 67.1 at 272, 101 / 83 at 578;
-    // 2: 76 / 88 at 144, 99 / 90 at 272; 8: 256 / 263 at 144.  HM_DF64, 1: 49.8 /
-    // 57.5 at 144, 80.6 / 72.6 at 578; 2: 82 / 85 at 272; 4: 47.6 / 72.2 at 60, 86 / 81 at
-    // 144; 8: 88 / 130 at 60.  Matrices without transfers or far-field blocks
-    // (low-rank factors only) run their one tree stage on all SMs at any size.
+    // take as long as the stage kernels on all of them, launched as a graph (us, fused
+    // against stages): FP32, 1 right-hand side: 16.5 / 17.5 at 28, 17.7 / 19.5 at 124, 23.5 /
+    // 21.5 at 252; 4: 22.1 / 25.5 at 60, 29.5 / 27.3 at 252; 8: 27.0 / 29.8 at 124; 16: 31.4 /
+    // 29.5 at 28.  FP64, 1: 27.6 / 31.3 at 28, 35.5 / 37.7 at 124, 50.1 / 45.8 at 252; 2: 53 /
+    // 54 at 124, 74 / 66 at 148; 4: 79 / 86 at 60, 110 / 103 at 124; 8: 146 / 137 at 28.
+    // HM_DF64, 1: 24.4 / 25.5 at 28, 33.5 / 31.7 at 124; 2: 40.0 / 41.7 at 124, 56 / 47 at
+    // 252; 4: 50 / 56 at 60; 8: 89 / 93 at 60.  Matrices without transfers or far-field
+    // blocks (low-rank factors only) run their one tree stage on all SMs at any size.
     const int slots = std::max(h->n_xslots, h->n_yslots), k = ma.k;
     if (!has_transfers(h)) return k <= kPartMaxK;
-    if (df) return slots <= (k <= 2 ? 288 : k <= 8 ? 80 : 0);
-    if (sizeof(S) == 8) return slots <= (k == 1 ? 320 : k <= 8 ? 160 : 0);
-    return slots <= (k <= 4 ? 320 : k <= 8 ? 160 : k <= 16 ? 64 : 0);
+    if (df) return slots <= (k == 1 ? 40 : k == 2 ? 130 : k <= 8 ? 80 : 0);
+    if (sizeof(S) == 8) return slots <= (k <= 2 ? 140 : k <= 4 ? 100 : 0);
+    return slots <= (k <= 4 ? 200 : k <= 8 ? 160 : 0);
 }
 
 // Clusters of kFusedCtas (beyond the portable 8) for `kernel`, set once per device.
@@ -1612,13 +1612,14 @@ template <typename S, typename A, int KB>
 int launch_both(hm_handle *h, const MulArgs<S> &ma, cudaStream_t st, const A *t, const A *s, const void *panels, bool pdl)
 {
     const int maxw = std::max(h->max_width, 1);
+    const bool far_rows = h->part_width[1] <= 64;          // launch_part_kb's far field
     if constexpr (std::is_same<S, double>::value) {
         if (h->storage == HM_DF64) {
             const size_t smem = (size_t)kWarpsPerCta * maxw * KB * sizeof(float2);
             HM_TRY(ensure_smem(expand_both_df<KB>, smem));
             return launch_k("expand_both_df", expand_both_df<KB>, dim3(warp_ctas(h->n_segs)), dim3(32 * kWarpsPerCta),
                             smem, st, pdl, ma, h->d_segs, h->n_segs, h->d_pieces, static_cast<const float2 *>(panels),
-                            s, t, h->r, maxw);
+                            s, t, h->r, maxw, far_rows);
         }
     }
     const size_t smem = (size_t)kWarpsPerCta * maxw * KB * sizeof(A);
@@ -1626,7 +1627,7 @@ int launch_both(hm_handle *h, const MulArgs<S> &ma, cudaStream_t st, const A *t,
     const int tile = cur_sched(h).tile;
     return launch_k("expand_both", expand_both<S, A, KB>, dim3(warp_ctas(h->n_segs)), dim3(32 * kWarpsPerCta), smem, st,
                     pdl, ma, h->d_segs, h->n_segs, h->d_pieces, static_cast<const S *>(panels), s, t, h->r, maxw,
-                    kRingTile[tile >= 0 && tile < kRingTiles ? tile : 0].pf);
+                    kRingTile[tile >= 0 && tile < kRingTiles ? tile : 0].pf, far_rows);
 }
 
 template <typename S, typename A>
@@ -1685,8 +1686,8 @@ int launch_fused(hm_handle *h, const MulArgs<S> &ma, cudaStream_t st, void *scra
 //   287; 2: 2^17 190 / 196 / 191.
 //   FP64, 1: grid 2^16 95 / 107 / 129, 2^17 130 / 129 / 117 (random 206 / 151 / 171),
 //   grid 2^18 246 / 213 / 228, 2^20 636 / 645 / 625 (random 850 / 834 / 822); 2: 2^17 350 /
-//   311 / 343; 4: 2^18 1,009 / 966 / 1,072; 8: grid 2^16 655 / 474 / 495, 2^18 2,014 /
-//   1,775 / 1,860.
+//   311 / 343; 4: 2^18 1,009 / 966 / 1,072; 8: 2^13 245 / 245 / 224, 2^15 382 / 382 / 382
+//   (grid 312 / 312 / 296), grid 2^16 655 / 474 / 495, 2^18 2,014 / 1,775 / 1,860.
 template <typename S>
 int near_start(const hm_handle *h, const MulArgs<S> &ma, int overlap)
 {
@@ -1694,7 +1695,7 @@ int near_start(const hm_handle *h, const MulArgs<S> &ma, int overlap)
     const int slots = std::max(h->n_xslots, h->n_yslots), k = ma.k;
     int m = 2;
     if (h->storage == HM_DF64) m = k == 1 ? 4 : 2;
-    else if (sizeof(S) == 8) m = k <= 2 && slots >= 24576 ? 1 : k == 1 && slots < 4096 ? 2 : 4;
+    else if (sizeof(S) == 8) m = (k <= 2 && slots >= 24576) || (k > 4 && slots < 1200) ? 1 : k == 1 && slots < 4096 ? 2 : 4;
     else if (sizeof(S) == 4) m = k <= 2 ? (slots >= 8192 ? 4 : 2) : k <= 4 ? (slots >= 8192 ? 4 : 1)
                                  : (slots >= 2048 && slots < 16384 ? 4 : 1);
     return m == 1 && ma.xin ? 4 : m;

@@ -82,33 +82,7 @@ __global__ void expand_df(MulArgs<double> ma, const hm_seg *segs, int nsegs, con
     }
     __syncwarp();
     float sh[2][KB], sl[2][KB];
-#pragma unroll
-    for (int j = 0; j < 2; ++j)
-#pragma unroll
-        for (int q = 0; q < KB; ++q) sh[j][q] = sl[j][q] = 0.f;
-    if (2 * lane < G.ld) {
-        const float4 *base = reinterpret_cast<const float4 *>(P + G.poff + 2 * lane);
-        const int64_t ld2 = G.ld / 2;                         // float4 (two pairs) per column step
-        constexpr int U = KB <= 2 ? 16 : 8;                    // loads in flight per lane
-        int c = c0;
-        auto use = [&](const float4 &p, int cc) {
-            const float2 *gc = g + cc * KB;
-#pragma unroll
-            for (int q = 0; q < KB; ++q) {
-                const float2 gq = gc[q];
-                df_fma(sh[0][q], sl[0][q], p.x, p.y, gq.x, gq.y);
-                df_fma(sh[1][q], sl[1][q], p.z, p.w, gq.x, gq.y);
-            }
-        };
-        for (; c + U <= c1; c += U) {
-            float4 p[U];
-#pragma unroll
-            for (int u = 0; u < U; ++u) p[u] = __ldcs(base + ld2 * (c + u));
-#pragma unroll
-            for (int u = 0; u < U; ++u) use(p[u], c + u);
-        }
-        for (; c < c1; ++c) use(__ldcs(base + ld2 * c), c);
-    }
+    df_columns<KB>(P + G.poff, G.ld, g, c0, c1, true, sh, sl);
     const bool acc_y = PART == 1 ? (yfar == nullptr) : (ma.accumulate != 0);
 #pragma unroll
     for (int q = 0; q < KB; ++q) {

@@ -29,6 +29,71 @@ __device__ __forceinline__ void df_fma(float &sh, float &sl, float ph, float pl,
     sl = __fsub_rn(t, __fsub_rn(sh, s));
 }
 
+// (sh, sl) += sum over columns [c0, c1) of a segment's panel (ld rows, two per lane) times
+// g[c * KB + q]; `groups`: low segments' columns dealt out to lane groups (ring_groups),
+// the groups' sums in every group at the end.
+template <int KB>
+__device__ __forceinline__ void df_columns(const float2 *Pg, int ld, const float2 *g, int c0, int c1, bool groups,
+                                           float (&sh)[2][KB], float (&sl)[2][KB])
+{
+    const int lane = threadIdx.x & 31;
+    const int cg = groups ? ring_groups(ld) : 1, lanes = 32 / cg, lr = lane & (lanes - 1);
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int q = 0; q < KB; ++q) sh[j][q] = sl[j][q] = 0.f;
+    const float4 *base = reinterpret_cast<const float4 *>(Pg + 2 * lr);
+    const int64_t ld2 = ld / 2;                                // float4 (two pairs) per column step
+    auto use = [&](const float4 &p, int cc) {
+        const float2 *gc = g + cc * KB;
+#pragma unroll
+        for (int q = 0; q < KB; ++q) {
+            const float2 gq = gc[q];
+            df_fma(sh[0][q], sl[0][q], p.x, p.y, gq.x, gq.y);
+            df_fma(sh[1][q], sl[1][q], p.z, p.w, gq.x, gq.y);
+        }
+    };
+    if (cg > 1) {
+        if (2 * lr < ld) {
+            constexpr int U = 4;
+            for (int c = c0 + lane / lanes; c < c1; c += U * cg) {
+                float4 p[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                    if (c + u * cg < c1) p[u] = __ldcs(base + ld2 * (c + u * cg));
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                    if (c + u * cg < c1) use(p[u], c + u * cg);
+            }
+        }
+        for (int o = lanes; o < 32; o <<= 1) {
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+#pragma unroll
+                for (int q = 0; q < KB; ++q) {
+                    const float a = sh[j][q], so = __shfl_xor_sync(0xffffffffu, a, o);
+                    const float l = __fadd_rn(sl[j][q], __shfl_xor_sync(0xffffffffu, sl[j][q], o));
+                    float s, e;
+                    two_sum(a, so, s, e);
+                    const float t = __fadd_rn(e, l);
+                    sh[j][q] = __fadd_rn(s, t);
+                    sl[j][q] = __fsub_rn(t, __fsub_rn(sh[j][q], s));
+                }
+        }
+    } else if (2 * lane < ld) {
+        constexpr int U = KB <= 2 ? 16 : 8;                    // loads in flight per lane
+        int c = c0;
+        for (; c + U <= c1; c += U) {
+            float4 p[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) p[u] = __ldcs(base + ld2 * (c + u));
+#pragma unroll
+            for (int u = 0; u < U; ++u) use(p[u], c + u);
+        }
+        for (; c < c1; ++c) use(__ldcs(base + ld2 * c), c);
+    }
+}
+
 // One basis panel by one warp (leaf_up_df); xs: cap pairs of this warp.
 __device__ __forceinline__ void leaf_panel_df(const MulArgs<double> &ma, const hm_vpanel P, const float2 *V, double *t,
                                               int r, int cap, float2 *xs)

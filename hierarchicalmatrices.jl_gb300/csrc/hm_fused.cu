@@ -278,11 +278,12 @@ __device__ __forceinline__ void seg_columns_plain(const S *Pg, int ld, const A *
 }  // namespace
 
 // Both parts of one row segment per warp: the near field before, the far field
-// after the tree passes; y (+)= near, then + far, as the stage kernels do.
+// after the tree passes; y (+)= near, then + far, as the stage kernels do (far_rows: their
+// far field is a thread per row, whose sums run column by column).
 template <typename S, typename A, int KB>
 __global__ void __launch_bounds__(128)
     expand_both(MulArgs<S> ma, const hm_seg *segs, int nsegs, const hm_piece *pieces, const S *P, const A *s,
-                const A *t, int r, int maxw, int pf)
+                const A *t, int r, int maxw, int pf, bool far_rows)
 {
     extern __shared__ __align__(16) unsigned char both_smem[];
     const int wib = threadIdx.x >> 5;
@@ -303,8 +304,14 @@ __global__ void __launch_bounds__(128)
     if (!live) return;
     seg_gather<S, A, true, KB>(ma, G, pieces, s, t, r, g, c0, c1);
     __syncwarp();
-    if constexpr (KB >= 4) seg_columns_plain<S, A, KB>(P + G.poff, G.ld, g, c0, c1, far);
-    else seg_columns<S, A, KB>(P + G.poff, G.ld, g, c0, c1, far);
+    bool plain = KB >= 4;
+    if constexpr (sizeof(S) == 8 && KB < 4) plain = far_rows;
+    if constexpr (NR == 2) {
+        if (plain) seg_columns_plain<S, A, KB>(P + G.poff, G.ld, g, c0, c1, far);
+        else seg_columns<S, A, KB>(P + G.poff, G.ld, g, c0, c1, far);
+    } else {
+        seg_columns<S, A, KB>(P + G.poff, G.ld, g, c0, c1, far);
+    }
 #pragma unroll
     for (int q = 0; q < KB; ++q) {
         if (q >= ma.k) break;
@@ -324,7 +331,7 @@ __global__ void __launch_bounds__(128)
 template <int KB>
 __global__ void __launch_bounds__(128)
     expand_both_df(MulArgs<double> ma, const hm_seg *segs, int nsegs, const hm_piece *pieces, const float2 *P,
-                   const double *s, const double *t, int r, int maxw)
+                   const double *s, const double *t, int r, int maxw, bool far_rows)
 {
     extern __shared__ __align__(16) unsigned char both_smem[];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
@@ -356,35 +363,9 @@ __global__ void __launch_bounds__(128)
         if (c0 < 0) c0 = c1 = 0;
         __syncwarp();
     };
-    auto sums = [&](int c0, int c1, double (&val)[KB][2]) {
+    auto sums = [&](int c0, int c1, bool groups, double (&val)[KB][2]) {
         float sh[2][KB], sl[2][KB];
-#pragma unroll
-        for (int j = 0; j < 2; ++j)
-#pragma unroll
-            for (int q = 0; q < KB; ++q) sh[j][q] = sl[j][q] = 0.f;
-        if (2 * lane < G.ld) {
-            const float4 *base = reinterpret_cast<const float4 *>(P + G.poff + 2 * lane);
-            const int64_t ld2 = G.ld / 2;
-            constexpr int U = KB <= 2 ? 16 : 8;                // loads in flight per lane
-            auto use = [&](const float4 &p, int cc) {
-                const float2 *gc = g + cc * KB;
-#pragma unroll
-                for (int q = 0; q < KB; ++q) {
-                    const float2 gq = gc[q];
-                    df_fma(sh[0][q], sl[0][q], p.x, p.y, gq.x, gq.y);
-                    df_fma(sh[1][q], sl[1][q], p.z, p.w, gq.x, gq.y);
-                }
-            };
-            int c = c0;
-            for (; c + U <= c1; c += U) {
-                float4 p[U];
-#pragma unroll
-                for (int u = 0; u < U; ++u) p[u] = __ldcs(base + ld2 * (c + u));
-#pragma unroll
-                for (int u = 0; u < U; ++u) use(p[u], c + u);
-            }
-            for (; c < c1; ++c) use(__ldcs(base + ld2 * c), c);
-        }
+        df_columns<KB>(P + G.poff, G.ld, g, c0, c1, groups, sh, sl);
 #pragma unroll
         for (int q = 0; q < KB; ++q)
 #pragma unroll
@@ -394,12 +375,12 @@ __global__ void __launch_bounds__(128)
     int c0, c1;
     if (live) {
         gather(false, c0, c1);
-        sums(c0, c1, near);
+        sums(c0, c1, true, near);
     }
     pdl_wait();                                                // the tree passes' coefficients are ready
     if (!live) return;
     gather(true, c0, c1);
-    sums(c0, c1, far);
+    sums(c0, c1, !far_rows, far);                          // far_rows_df sums column by column
 #pragma unroll
     for (int q = 0; q < KB; ++q) {
         if (q >= k) break;
@@ -421,12 +402,12 @@ HM_INST_FUSED(double, 1) HM_INST_FUSED(double, 2) HM_INST_FUSED(double, 4) HM_IN
 template __global__ void tree_fused<double, double, 1, true>(const __grid_constant__ TreeArgs<double, double>);
 #define HM_INST_BOTH(S, KB)                                                                                   \
     template __global__ void expand_both<S, S, KB>(MulArgs<S>, const hm_seg *, int, const hm_piece *, const S *, \
-                                                   const S *, const S *, int, int, int);
+                                                   const S *, const S *, int, int, int, bool);
 HM_INST_BOTH(float, 2) HM_INST_BOTH(float, 4) HM_INST_BOTH(float, 8)
 HM_INST_BOTH(double, 1) HM_INST_BOTH(double, 2) HM_INST_BOTH(double, 4) HM_INST_BOTH(double, 8)
 #define HM_INST_BOTH_DF(KB)                                                                                     \
     template __global__ void expand_both_df<KB>(MulArgs<double>, const hm_seg *, int, const hm_piece *,        \
-                                                const float2 *, const double *, const double *, int, int);
+                                                const float2 *, const double *, const double *, int, int, bool);
 HM_INST_BOTH_DF(1) HM_INST_BOTH_DF(2) HM_INST_BOTH_DF(4) HM_INST_BOTH_DF(8)
 
 }  // namespace hm

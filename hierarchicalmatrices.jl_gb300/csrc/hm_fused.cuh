@@ -38,9 +38,9 @@ __global__ void tree_fused(const __grid_constant__ TreeArgs<S, A> a);
 // 3 to 8 FP32 right-hand sides.
 template <typename S, typename A, int KB>
 __global__ void expand_both(MulArgs<S> ma, const hm_seg *segs, int nsegs, const hm_piece *pieces, const S *P,
-                            const A *s, const A *t, int r, int maxw, int pf);
+                            const A *s, const A *t, int r, int maxw, int pf, bool far_rows);
 template <int KB>
 __global__ void expand_both_df(MulArgs<double> ma, const hm_seg *segs, int nsegs, const hm_piece *pieces,
-                               const float2 *P, const double *s, const double *t, int r, int maxw);
+                               const float2 *P, const double *s, const double *t, int r, int maxw, bool far_rows);
 
 }  // namespace hm
