@@ -1327,7 +1327,7 @@ int launch_part_kb(hm_handle *h, const MulArgs<S> &ma, const A *s, const A *t, c
         const Sched fs = cur_sched(h);
         if (h->stream_ctas > 0 && h->part_width[1] <= 64 && (fs.near_kernel == 0 || fs.near_kernel == 3)) {
             HM_TRY(launch_k("far_rows", far_rows<S, A, KB>, dim3((unsigned)((h->n_segs + 3) / 4)), dim3(256), 0, st,
-                            pdl, ma, h->d_segs, h->n_segs, h->d_pieces, static_cast<const S *>(panels), s, t, h->r,
+                            pdl, ma, h->d_segs, h->n_segs, h->d_pieces, static_cast<const S *>(panels), s, t, h->r, ma.k,
                             yfar, ldf));
             return HM_OK;
         }
@@ -1423,6 +1423,48 @@ int launch_part(hm_handle *h, const MulArgs<S> &ma, const A *s, const A *t, cons
 }
 
 constexpr int kTensorCoreMinK = 16;   // right-hand sides from which the tensor-core panels run
+
+// Whether a product with more than kPartMaxK right-hand sides runs its panels in chunks
+// of them on the kernels for up to kPartMaxK (near field beside the tree passes, far field
+// after them) rather than on expand_k, which reads a panel once per chunk too but has
+// neither their pipelines nor their lane groups; it keeps the sizes where several chunks
+// are several launches that do not fill the chip.  expand_k / chunks, us per product on
+// random points: FP32, 9 right-hand sides: n = 2^14 66 / 55 (grid 51 / 53), 2^16 140 / 85,
+// 2^18 449 / 220; 13: 2^14 67 / 71, 2^16 144 / 92.  FP64, 9: 4,000 points 292 / 242, 2^18
+// 4,185 / 2,141; 16: 4,000 points 294 / 347, 2^14 500 / 440, 2^18 4,214 / 3,174; 64: 2^14
+// 1,537 / 1,619, 2^16 4,497 / 4,069.
+template <typename S, typename A>
+bool chunked_ok(const hm_handle *h, const MulArgs<S> &ma)
+{
+    const Sched sc = cur_sched(h);
+    if (ma.k <= kPartMaxK || h->storage == HM_DF64 || !std::is_same<S, A>::value || sc.near_kernel != 0) return false;
+    if (sizeof(S) == 4 && sc.tensor_cores && h->tc_ok && ma.k >= kTensorCoreMinK) return false;
+    const int slots = std::max(h->n_xslots, h->n_yslots);
+    if (slots < (sizeof(S) == 8 && ma.k <= 32 ? 400 : 1200)) return false;
+    return h->stream_ctas > 0 && h->part_width[1] <= 64;
+}
+
+template <typename S, typename A, bool FAR>
+int launch_chunks(hm_handle *h, const MulArgs<S> &ma, const A *s, const A *t, const void *panels, cudaStream_t st)
+{
+    for (int q0 = 0; q0 < ma.k; q0 += kPartMaxK) {
+        MulArgs<S> mc = ma;
+        mc.x += (int64_t)q0 * ma.ldx;
+        mc.y += (int64_t)q0 * ma.ldy;
+        mc.k = std::min(kPartMaxK, ma.k - q0);
+        if constexpr (!FAR) {
+            HM_TRY((launch_part<S, A, false>(h, mc, s, t, panels, st)));
+        } else if constexpr (std::is_same<S, A>::value) {
+            auto far = mc.k <= 2 ? far_rows<S, A, 2> : mc.k <= 4 ? far_rows<S, A, 4> : far_rows<S, A, 8>;
+            const A *sq = s + (size_t)q0 * h->r, *tq = t + (size_t)q0 * h->r;
+            far<<<(unsigned)((h->n_segs + 3) / 4), 256, 0, st>>>(mc, h->d_segs, h->n_segs, h->d_pieces,
+                                                                 static_cast<const S *>(panels), sq, tq, h->r, ma.k,
+                                                                 static_cast<S *>(nullptr), (int64_t)0);
+            HM_CK_LAUNCH("far_rows");
+        }
+    }
+    return HM_OK;
+}
 
 template <typename S, typename A>
 int launch_expand_k(hm_handle *h, const MulArgs<S> &ma, const A *s, const A *t, const void *panels, cudaStream_t st)
@@ -1772,6 +1814,16 @@ int launch_pipeline(hm_handle *h, const MulArgs<S> &ma, cudaStream_t st, cudaStr
                                             cur_sched(h).pdl && !(h->profile_mask & 0xcu))));
         }
         return HM_OK;
+    }
+    if (!ma.yout && chunked_ok<S, A>(h, ma)) {
+        {
+            StageTimer tm(h, timing ? 2 : -1, st);
+            HM_TRY((launch_chunks<S, A, false>(h, ma, s, t, panels, st)));
+        }
+        if (!tree) return HM_OK;
+        if (split) HM_CK(cudaStreamWaitEvent(st, join, 0));
+        StageTimer tm(h, timing ? 3 : -1, st);
+        return launch_chunks<S, A, true>(h, ma, s, t, panels, st);
     }
     if (tree && split) HM_CK(cudaStreamWaitEvent(st, join, 0));
     StageTimer tm(h, timing ? 2 : -1, st);

@@ -608,12 +608,13 @@ __global__ void expand_part(MulArgs<S> ma, const hm_seg *segs, int nsegs, const 
 // non-X pieces, at most 64 columns, KB right-hand sides) are gathered once into
 // shared memory; thread `row` then reads its row of the column-major basis
 // columns (consecutive threads, consecutive rows: coalesced) and accumulates
-// KB sums with FMA (at most 64 terms, as the warp kernels' folds do).  The
+// KB sums with FMA (at most 64 terms, as the warp kernels' folds do); ks: right-hand
+// sides of the coefficients (ma.k of them from s, t on).  The
 // rows go to yfar (leading dimension ldf) or, without it, are added into y.
 template <typename S, typename A, int KB>
 __global__ void __launch_bounds__(256)
     far_rows(MulArgs<S> ma, const hm_seg *segs, int nsegs, const hm_piece *pieces, const S *P, const A *s,
-             const A *t, int r, S *yfar, int64_t ldf)
+             const A *t, int r, int ks, S *yfar, int64_t ldf)
 {
     __shared__ A cs[4][64 * KB];                               // [segment][column][q]
     pdl_wait();                                                // the downward pass's coefficients are ready
@@ -635,7 +636,7 @@ __global__ void __launch_bounds__(256)
                 Q = pieces[G.piece0 + ++pi];
             }
             A v = A(0);
-            if (q < k) v = (Q.kind == HM_PIECE_TCOEF ? t : s)[((int64_t)Q.src * k + q) * r + (c - pc)];
+            if (q < k) v = (Q.kind == HM_PIECE_TCOEF ? t : s)[((int64_t)Q.src * ks + q) * r + (c - pc)];
             cs[ls][e] = v;
         }
     }
@@ -1131,9 +1132,10 @@ __global__ void expand_k(MulArgs<S> ma, const hm_seg *segs, const hm_piece *piec
 HM_INST_FLAT(1) HM_INST_FLAT(2) HM_INST_FLAT(4) HM_INST_FLAT(8)
 #define HM_INST_FAR(S, A, KB)                                                                        \
     template __global__ void far_rows<S, A, KB>(MulArgs<S>, const hm_seg *, int, const hm_piece *, const S *, \
-                                                const A *, const A *, int, S *, int64_t);
+                                                const A *, const A *, int, int, S *, int64_t);
 HM_INST_FAR(float, float, 4) HM_INST_FAR(float, float, 8) HM_INST_FAR(double, double, 4)
 HM_INST_FAR(double, double, 8) HM_INST_FAR(double, double, 1) HM_INST_FAR(double, double, 2)
+HM_INST_FAR(float, float, 2)
 #define HM_INST_MV(S, A)                                                                             \
     template __global__ void leaf_up<S, A, 1>(MulArgs<S>, const hm_vpanel *, int, const S *, A *, int, int, int, LeafParts<A>); \
     template __global__ void leaf_up<S, A, 2>(MulArgs<S>, const hm_vpanel *, int, const S *, A *, int, int, int, LeafParts<A>); \

@@ -239,7 +239,7 @@ __global__ void add_far(MulArgs<S> ma, int64_t n, const S *yfar, int64_t ldf);
 // CTA of 256 threads); segments' far columns first and at most 64 of them.
 template <typename S, typename A, int KB>
 __global__ void far_rows(MulArgs<S> ma, const hm_seg *segs, int nsegs, const hm_piece *pieces, const S *P,
-                         const A *s, const A *t, int r, S *yfar, int64_t ldf);
+                         const A *s, const A *t, int r, int ks, S *yfar, int64_t ldf);
 
 // Persistent panel streaming (cp.async.bulk into a ring of shared-memory
 // stages).  CTA b owns segments [cta_seg[b], cta_seg[b+1]); FAR selects the
