@@ -35,11 +35,11 @@
 // Measured (ms per call of the panel stage): 32 right-hand sides at n = 2^19 0.436
 // -> 0.201, 256 at n = 2^18 0.584 -> 0.319.  The form before loaded, split and
 // multiplied a chunk between CTA barriers with 24% of the warps active, and its
-// load instructions touched eight lines each.  What bounds it now: the producers
-// (issue slots 62% busy, of which the splitting itself, 11 instructions per two
-// values, is a quarter; then the wait for a chunk's loads, which the registers of
-// 22 warps leave no room to issue a chunk ahead; a second register set at 32 right-
-// hand sides measured 0.245 ms).
+// load instructions touched eight lines each.  What bounds it now: the producers'
+// wait for a chunk's loads, which the registers of 22 warps leave no room to issue a
+// chunk ahead (32 right-hand sides: issue slots 43% busy, of which the splitting itself, 11
+// instructions per two values, is a quarter, tensor pipe 37%; a second register set
+// measured 0.245 ms).
 //
 // Operand layout (SWIZZLE_128B, K-major, 16-bit): a row's 64 columns are 128 bytes,
 // 8-row groups 1,024 bytes apart, the 16-byte columns of row i permuted by XOR

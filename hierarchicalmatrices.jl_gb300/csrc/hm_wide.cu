@@ -1,4 +1,4 @@
-// Tree passes for 32 and more right-hand sides: lane q of a warp owns
+// Tree passes for 32 and more right-hand sides (FP32 from 5 on large trees): lane q of a warp owns
 // right-hand side q of a chunk of 32 and accumulates all R coefficients of it
 // in registers.  Written for sm_103a.
 //
