@@ -1225,11 +1225,22 @@ int launch_tree_wide(hm_handle *h, const MulArgs<S> &ma, cudaStream_t st, A *t, 
             // two right-hand sides per lane from 64 on (half the shared-memory reads per FMA)
             const int qpl = (G == 1 && k >= 64) ? 2 : 1;
             auto kern = qpl == 2 ? m2l_w<A, R, 2, G> : m2l_w<A, R, 1, G>;
+            int qw = QL * qpl, ng = G;                     // right-hand sides of a group, groups of a warp
+            if constexpr (G == 1 && sizeof(A) == 4) {
+                // below 64 two row slots per warp, two right-hand sides per lane of 16: half the
+                // reads per FMA for the same chunk of 32 (downward half of the tree, 32 right-hand
+                // sides at n = 2^19 110 -> 104 us; from 64 on 258 -> 284 at 256 and n = 2^18)
+                if (k < 64) {
+                    kern = m2l_w<A, R, 2, 2>;
+                    qw = 32;
+                    ng = 2;
+                }
+            }
             const size_t smem =
-                (size_t)kWideWarps * G * m2l_w_group_vals(h->fstride, QL * qpl, R, (int)sizeof(A)) * sizeof(A);
+                (size_t)kWideWarps * ng * m2l_w_group_vals(h->fstride, qw, R, (int)sizeof(A)) * sizeof(A);
             HM_TRY(ensure_smem(kern, smem));
-            const int64_t groups = (int64_t)h->n_m2l_rows * ((k + QL * qpl - 1) / (QL * qpl));
-            HM_TRY(launch_k("m2l_w", kern, dim3(ctas(groups)), dim3(32 * kWideWarps), smem, st, pdl_on && chain,
+            const int64_t groups = (int64_t)h->n_m2l_rows * ((k + qw - 1) / qw);
+            HM_TRY(launch_k("m2l_w", kern, dim3((unsigned)((groups + kWideWarps * ng - 1) / (kWideWarps * ng))), dim3(32 * kWideWarps), smem, st, pdl_on && chain,
                             h->d_m2l_rows, h->n_m2l_rows, h->d_m2l_ents, static_cast<const A *>(h->d_F), h->fstride,
                             t, s, k));
             chain = true;

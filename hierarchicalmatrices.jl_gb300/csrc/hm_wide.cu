@@ -433,6 +433,8 @@ __global__ void __launch_bounds__(kWideTaskThreads)
                                                           const A *, A *, int, int);
 HM_INST_WIDE(float, 1, 1) HM_INST_WIDE(float, 2, 1) HM_INST_WIDE(float, 1, 2) HM_INST_WIDE(float, 1, 4)
 HM_INST_WIDE(double, 1, 1) HM_INST_WIDE(double, 2, 1) HM_INST_WIDE(double, 1, 2) HM_INST_WIDE(double, 1, 4)
+template __global__ void m2l_w<float, 20, 2, 2>(const hm_m2l_row *, int, const hm_m2l_ent *, const float *, int,
+                                                const float *, float *, int);
 HM_INST_XFER(float, 1) HM_INST_XFER(float, 2) HM_INST_XFER(float, 4)
 HM_INST_XFER(double, 1) HM_INST_XFER(double, 2) HM_INST_XFER(double, 4)
 
