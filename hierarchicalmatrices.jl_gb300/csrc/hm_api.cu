@@ -1330,11 +1330,11 @@ int launch_part_kb(hm_handle *h, const MulArgs<S> &ma, const A *s, const A *t, c
         }
     }
     if constexpr (FAR && (KB >= 4 || sizeof(S) == 8) && std::is_same<S, A>::value) {
-        // far-field rows one thread per row for 3-8 right-hand sides (the default
-        // and ring schedules; the warp and streamed kernels keep their own
-        // far-field form).  Measured: 512-instance batch at 8, 0.55 against
-        // 0.76 ms; with 1 right-hand side at n = 2^20 the warp kernel's
-        // four-rows-per-lane form stays faster (25 against 41 us)
+        // far-field rows one thread per row for 3-8 right-hand sides and for FP64 (the
+        // default and ring schedules; the warp and streamed kernels keep their own
+        // far-field form).  Measured: 512-instance batch at 8, 0.55 against 0.76 ms;
+        // FP64 at n = 2^20, 1: 45 / 48 us, 2: 80 / 145; with 1 FP32 right-hand side the
+        // warp kernel's four-rows-per-lane form stays faster (25 against 41 us)
         const Sched fs = cur_sched(h);
         if (h->stream_ctas > 0 && h->part_width[1] <= 64 && (fs.near_kernel == 0 || fs.near_kernel == 3)) {
             HM_TRY(launch_k("far_rows", far_rows<S, A, KB>, dim3((unsigned)((h->n_segs + 3) / 4)), dim3(256), 0, st,
