@@ -151,7 +151,9 @@ __device__ __forceinline__ void sqrt_both(float d, float &s, float &y)
 
 // 1 / d: the FP32 reciprocal of d's mantissa and one step of the third-order
 // (Householder) iteration, y = y0 (1 + e + e^2), e = 1 - d y0, which leaves e^3 <
-// 2^-66.  Exponents near the ends of double's range: the division.
+// 2^-66 (within 1 ulp of the division over 8 million values of exponents -600 to 600; of
+// sqrt_both s equals the library's square root there, y is within 1 ulp of 1 / s).
+// Exponents near the ends of double's range: the division.
 __device__ __forceinline__ double recip(double d)
 {
     const int e = exponent_of(d);
