@@ -1319,11 +1319,19 @@ int launch_part_kb(hm_handle *h, const MulArgs<S> &ma, const A *s, const A *t, c
     if constexpr (std::is_same<S, double>::value && std::is_same<A, double>::value) {
         if (h->storage == HM_DF64) {
             if (FAR && h->stream_ctas > 0 && h->part_width[1] <= 64) {
-                // far-field rows one thread per row, right-hand side by right-hand side
-                for (int q0 = 0; q0 < ma.k; ++q0)
-                    HM_TRY(launch_k("far_rows_df", far_rows_df, dim3((unsigned)((h->n_segs + 3) / 4)), dim3(256), 0,
-                                    st, pdl && q0 == 0, ma, h->d_segs, h->n_segs, h->d_pieces,
-                                    static_cast<const float2 *>(panels), s, t, h->r, yfar, ldf, q0));
+                // far-field rows one thread per row: up to four right-hand sides at once on
+                // smaller trees, one by one where the launches' longer tail fills the near
+                // field's (us per product, one by one / at once: 8 right-hand sides at 20,000
+                // points 160 / 153, 2^16 292 / 292, 2^18 grid 598 / 610; 4: 95 / 86, 155 / 155,
+                // 300,007 beta points 497 / 512)
+                const bool few = std::max(h->n_xslots, h->n_yslots) < 4096;
+                constexpr int KF = KB < 4 ? KB : 4;
+                const int step = few ? KF : 1;
+                for (int q0 = 0; q0 < ma.k; q0 += step)
+                    HM_TRY(launch_k("far_rows_df", few ? far_rows_df<KF> : far_rows_df<1>,
+                                    dim3((unsigned)((h->n_segs + 3) / 4)), dim3(256), 0, st, pdl && q0 == 0, ma,
+                                    h->d_segs, h->n_segs, h->d_pieces, static_cast<const float2 *>(panels), s, t,
+                                    h->r, yfar, ldf, q0));
                 return HM_OK;
             }
             return launch_df<FAR ? 1 : 0, KB>(h, ma, s, t, panels, yfar, st, pdl, ldf, 0);

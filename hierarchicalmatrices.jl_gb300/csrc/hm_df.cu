@@ -265,15 +265,18 @@ template __global__ void xfer_df<false>(const hm_task *, const hm_step *, const 
 
 // Far-field rows with HM_DF64 storage, one thread per row (four segments of at
 // most 64 rows per CTA of 256 threads): y_far[row] = sum_c U[row][c] s[c] over
-// the segment's far columns (at most 64), the coefficients split into pairs
-// once per segment in shared memory, the row's pairs read column by column
-// (consecutive threads, consecutive rows), double-float accumulation; one
-// right-hand side q0.  Rows go to yfar or, without it, are added into y.
+// the segment's far columns (at most 64), the coefficients of KB right-hand sides from
+// q0 on split into pairs once per segment in shared memory, the row's pairs read once
+// for all of them, column by column (consecutive threads, consecutive rows),
+// double-float accumulation.  Rows go to yfar or, without it, are added into y.  One
+// launch per right-hand side reads the panels again for each: 8 at 2^16 random points 62 us,
+// four at once 27.
+template <int KB>
 __global__ void __launch_bounds__(256)
     far_rows_df(MulArgs<double> ma, const hm_seg *segs, int nsegs, const hm_piece *pieces, const float2 *P,
                 const double *s, const double *t, int r, double *yfar, int64_t ldf, int q0)
 {
-    __shared__ float2 cs[4][64];
+    __shared__ float2 cs[4][64 * KB];                          // [segment][column][q]
     pdl_wait();                                                // the downward pass's coefficients are ready
     const int ls = threadIdx.x >> 6, row = threadIdx.x & 63;
     const int j = blockIdx.x * 4 + ls;
@@ -283,41 +286,58 @@ __global__ void __launch_bounds__(256)
     if (j < nsegs) {
         G = segs[j];
         nfar = G.nfar;
-        if (row < nfar) {
+        for (int e = row; e < nfar * KB; e += 64) {
+            const int c = e / KB, q = q0 + e % KB;
             int pc = 0, pi = 0;
             hm_piece Q = pieces[G.piece0];
-            while (row >= pc + Q.width) {
+            while (c >= pc + Q.width) {
                 pc += Q.width;
                 Q = pieces[G.piece0 + ++pi];
             }
-            cs[ls][row] = df_split((Q.kind == HM_PIECE_TCOEF ? t : s)[((int64_t)Q.src * k + q0) * r + (row - pc)]);
+            cs[ls][e] = q < k ? df_split((Q.kind == HM_PIECE_TCOEF ? t : s)[((int64_t)Q.src * k + q) * r + (c - pc)])
+                              : make_float2(0.f, 0.f);
         }
     }
     __syncthreads();
     if (j >= nsegs || row >= G.nrows) return;
     if (nfar == 0 && !yfar) return;                            // y += 0
-    float sh = 0.f, sl = 0.f;
+    float sh[KB], sl[KB];
+#pragma unroll
+    for (int q = 0; q < KB; ++q) sh[q] = sl[q] = 0.f;
     const float2 *pr = P + G.poff + row;
+    auto use = [&](const float2 &u, int c) {
+#pragma unroll
+        for (int q = 0; q < KB; ++q) {
+            const float2 g = cs[ls][c * KB + q];
+            df_fma(sh[q], sl[q], u.x, u.y, g.x, g.y);
+        }
+    };
     int c = 0;
     for (; c + 4 <= nfar; c += 4) {
         float2 u[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) u[i] = pr[(int64_t)(c + i) * G.ld];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) df_fma(sh, sl, u[i].x, u[i].y, cs[ls][c + i].x, cs[ls][c + i].y);
+        for (int i = 0; i < 4; ++i) use(u[i], c + i);
     }
-    for (; c < nfar; ++c) {
-        const float2 u = pr[(int64_t)c * G.ld];
-        df_fma(sh, sl, u.x, u.y, cs[ls][c].x, cs[ls][c].y);
-    }
-    const double v = __dadd_rn((double)sh, (double)sl);
-    if (yfar) {
-        yfar[(G.row0 + row) + (int64_t)q0 * ldf] = v;
-    } else {
-        double *yp = ma.y + (G.row0 + row) * ma.incy + (int64_t)q0 * ma.ldy;
-        *yp = *yp + v;
+    for (; c < nfar; ++c) use(pr[(int64_t)c * G.ld], c);
+#pragma unroll
+    for (int q = 0; q < KB; ++q) {
+        if (q0 + q >= k) break;
+        const double v = __dadd_rn((double)sh[q], (double)sl[q]);
+        if (yfar) {
+            yfar[(G.row0 + row) + (int64_t)(q0 + q) * ldf] = v;
+        } else {
+            double *yp = ma.y + (G.row0 + row) * ma.incy + (int64_t)(q0 + q) * ma.ldy;
+            *yp = *yp + v;
+        }
     }
 }
+#define HM_INST_FAR_DF(KB)                                                                                      \
+    template __global__ void far_rows_df<KB>(MulArgs<double>, const hm_seg *, int, const hm_piece *,             \
+                                             const float2 *, const double *, const double *, int, double *,      \
+                                             int64_t, int);
+HM_INST_FAR_DF(1) HM_INST_FAR_DF(2) HM_INST_FAR_DF(4)
 
 #define HM_INST_DF(PART)                                                                                        \
     template __global__ void expand_df<PART, 1>(MulArgs<double>, const hm_seg *, int, const hm_piece *,          \

@@ -335,8 +335,9 @@ constexpr int kM2lDfWarps = 4, kM2lDfStages = 3;
 template <int NS>
 __global__ void m2l_df_ring(const hm_m2l_row *rows, int nrows, const hm_m2l_ent *ents, const float2 *F, const double *t,
                             double *s, int k);
-// far_rows_df: far-field rows of right-hand side q0, one thread per row, four
+// far_rows_df: far-field rows of KB right-hand sides from q0 on, one thread per row, four
 // segments of at most 64 rows per CTA of 256 threads (at most 64 far columns).
+template <int KB>
 __global__ void far_rows_df(MulArgs<double> ma, const hm_seg *segs, int nsegs, const hm_piece *pieces,
                             const float2 *P, const double *s, const double *t, int r, double *yfar, int64_t ldf,
                             int q0);
