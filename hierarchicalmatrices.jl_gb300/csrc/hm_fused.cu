@@ -103,6 +103,10 @@ __global__ void __launch_bounds__(kFusedThreads) tree_fused(const __grid_constan
         }
     }
     if (a.n_rows) {
+        // m2l_first writes between this warp's arrival and its wait, into shared memory
+        // that other warps may still read leaf panels from; a band's last level ended
+        // with a CTA barrier, without bands there was none since
+        if (a.n_up == 0) __syncthreads();
         const int nm = DF ? 1 : nq;
         const int64_t items = (int64_t)a.n_rows * nm, i0 = (int64_t)wib * ctas + cta;
         const bool mine = wib < a.m2l_warps && i0 < items;
