@@ -54,7 +54,7 @@ __global__ void __launch_bounds__(kFusedThreads) tree_fused(const __grid_constan
     const int wib = threadIdx.x >> 5, ctas = gridDim.x, cta = blockIdx.x;
     const int r = a.r, k = a.ma.k, nq = DF ? k : (k + QC - 1) / QC;
     pdl_trigger();                                             // expand_both may start its near field
-    {
+    if (a.n_up || a.n_down) {                                  // without bands there is no T (assembled matrices)
         const TS *T = static_cast<const TS *>(a.T);
         for (int i = threadIdx.x; i < 2 * r * r; i += kFusedThreads) Ts[i] = T[i];
     }

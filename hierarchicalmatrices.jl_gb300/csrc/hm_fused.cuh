@@ -16,7 +16,7 @@ template <typename S, typename A>
 struct TreeArgs {
     MulArgs<S> ma;
     const hm_vpanel *vp;
-    const void *V, *T, *F;
+    const void *V, *T, *F;             // T: read only where there are bands (null in assembled matrices)
     LeafParts<A> lp;
     const hm_task *up_tasks, *down_tasks;
     const hm_step *up_steps, *down_steps;
