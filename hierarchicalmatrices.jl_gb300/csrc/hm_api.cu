@@ -1463,6 +1463,14 @@ bool chunked_ok(const hm_handle *h, const MulArgs<S> &ma)
     return h->stream_ctas > 0 && h->part_width[1] <= 64;
 }
 
+// Whether the near field runs in launches of its own, which may start before the tree
+// passes end; else one panel kernel follows them.
+template <typename S, typename A>
+bool near_apart(const hm_handle *h, const MulArgs<S> &ma)
+{
+    return ma.k <= kPartMaxK || (!ma.yout && chunked_ok<S, A>(h, ma));
+}
+
 template <typename S, typename A, bool FAR>
 int launch_chunks(hm_handle *h, const MulArgs<S> &ma, const A *s, const A *t, const void *panels, cudaStream_t st)
 {
@@ -1749,10 +1757,12 @@ int launch_fused(hm_handle *h, const MulArgs<S> &ma, cudaStream_t st, void *scra
 //   grid 2^18 246 / 213 / 228, 2^20 636 / 645 / 625 (random 850 / 834 / 822); 2: 2^17 350 /
 //   311 / 343; 4: 2^18 1,009 / 966 / 1,072; 8: 2^13 245 / 245 / 224, 2^15 382 / 382 / 382
 //   (grid 312 / 312 / 296), grid 2^16 655 / 474 / 495, 2^18 2,014 / 1,775 / 1,860.
+// Chunks of more than kPartMaxK right-hand sides start at once.
 template <typename S>
 int near_start(const hm_handle *h, const MulArgs<S> &ma, int overlap)
 {
-    if (overlap != 2 || ma.k > kPartMaxK) return overlap;
+    if (overlap != 2) return overlap;
+    if (ma.k > kPartMaxK) return ma.xin ? 4 : 1;
     const int slots = std::max(h->n_xslots, h->n_yslots), k = ma.k;
     int m = 2;
     if (h->storage == HM_DF64) m = k == 1 ? 4 : 2;
@@ -1834,7 +1844,8 @@ int launch_pipeline(hm_handle *h, const MulArgs<S> &ma, cudaStream_t st, cudaStr
         }
         return HM_OK;
     }
-    if (!ma.yout && chunked_ok<S, A>(h, ma)) {
+    if (near_apart<S, A>(h, ma)) {
+        if (split && mid) HM_CK(cudaStreamWaitEvent(st, mid, 0));
         {
             StageTimer tm(h, timing ? 2 : -1, st);
             HM_TRY((launch_chunks<S, A, false>(h, ma, s, t, panels, st)));
@@ -1900,7 +1911,7 @@ int capture_product(hm_handle *h, hm_handle::StreamCtx *sc, hm_handle::ProductGr
     HM_CK(cudaEventCreateWithFlags(&o.mid, cudaEventDisableTiming));
     HM_CK(cudaStreamBeginCapture(o.cap, cudaStreamCaptureModeRelaxed));
     const int rc = launch_pipeline<S, A>(h, ma, o.cap, run.overlap ? o.side : o.cap, o.fork, o.join, sc->p, false, panels,
-                                         run.overlap >= 2 && ma.k <= kPartMaxK ? o.mid : nullptr, sc->sync);
+                                         run.overlap >= 2 && near_apart<S, A>(h, ma) ? o.mid : nullptr, sc->sync);
     const cudaError_t ec = cudaStreamEndCapture(o.cap, &g.graph);
     if (rc) return rc;
     HM_CK(ec);
@@ -2012,9 +2023,8 @@ int run_mul(hm_handle *h, MulArgs<S> ma, cudaStream_t st, const void *panels = n
         if (done) return HM_OK;
     }
     StageTimer whole(h, 4, st);
-    // above kPartMaxK one panel kernel follows the tree passes: nothing waits for mid
     return launch_pipeline<S, A>(h, ma, st, run.overlap ? sc->side : st, sc->fork, sc->join, sc->p, true, panels,
-                                 run.overlap >= 2 && ma.k <= kPartMaxK ? sc->mid : nullptr, sc->sync);
+                                 run.overlap >= 2 && near_apart<S, A>(h, ma) ? sc->mid : nullptr, sc->sync);
 }
 
 // Row-derivative panels (same layout as the panels), filled once.
