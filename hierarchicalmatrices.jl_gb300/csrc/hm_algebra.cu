@@ -1042,6 +1042,14 @@ int64_t leaf_chol_max()
     while (((n + 1) * (n + 2) + (n + 1)) * (int64_t)sizeof(T) <= 200 * 1024) ++n;
     return n;
 }
+// Whether a pivot up to j has failed (flag: the failing pivot + 1), asked by every warp
+// after the barrier that published pivot j.  A fast warp 0 may already have set the
+// flag for pivot j + 1 by then: the index tells, so all warps leave at the same step.
+__device__ __forceinline__ bool failed_by(const int *flag, int j)
+{
+    const int f = *reinterpret_cast<const volatile int *>(flag);
+    return f && f <= j + 1;
+}
 template <typename T>
 __global__ void __launch_bounds__(kThreads) leaf_chol(const LeafChol g, int *info)
 {
@@ -1068,7 +1076,7 @@ __global__ void __launch_bounds__(kThreads) leaf_chol(const LeafChol g, int *inf
     };
     if (warp == 0) pivot(0);
     __syncthreads();
-    for (int j = 0; j < n && !s_fail; ++j) {
+    for (int j = 0; j < n && !failed_by(&s_fail, j); ++j) {
         if (warp == 0) {
             if (j + 1 < n) {
                 const T a = S[j + ls * (j + 1)];
@@ -1170,7 +1178,7 @@ __global__ void __launch_bounds__(kThreads) leaf_chol_regs(const LeafChol g, int
     __syncthreads();
     if (warp == 0) pivot(0);
     __syncthreads();
-    for (int j = 0; j < n && !s_fail; ++j) {
+    for (int j = 0; j < n && !failed_by(&s_fail, j); ++j) {
         if (warp == 0) {
             if (j + 1 < n) {
                 const T a = S[j + ls * (j + 1)];
