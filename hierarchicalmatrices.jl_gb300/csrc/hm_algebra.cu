@@ -246,9 +246,10 @@ __device__ void house_qr(T *A, int64_t ld, int64_t m, int k, T *tau, T *ss, int 
                     const bool live = c < k && c > j;
                     T *y = A + ld * (c < k ? c : k - 1);
                     if (b != cb) w = group_sum(strided_dot(x, y, j + 1 + lg, m, G), G);
+                    const T yj = live ? y[j] : T(0);
+                    __syncwarp();                                      // all lanes of a group have it
                     if (live) {
-                        const T yj = y[j], f = t * fma(w, sc, yj), fs = f * sc;
-                        __syncwarp(__activemask());
+                        const T f = t * fma(w, sc, yj), fs = f * sc;
                         if (lg == 0) y[j] = yj - f;
                         for (int64_t i = j + 1 + lg; i < m; i += G) y[i] = fma(-fs, x[i], y[i]);
                     }
