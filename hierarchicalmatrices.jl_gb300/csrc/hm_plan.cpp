@@ -309,7 +309,7 @@ int build_plan(const double *x, int64_t nx, const double *y, int64_t ny, double 
             vp.width = r;
             vp.slot = n.slot;
             vp.col0 = 0;
-            vp.pad = 0;
+            vp.zeros = 0;
             vp.off = off;
             off += round_up((int64_t)vp.nrows * r, 32);
             P.vpanels.push_back(vp);
@@ -588,7 +588,8 @@ int build_hier_plan(int64_t m, int64_t n, const std::vector<HierBlock> &blocks, 
             const int w = (int)std::min<int64_t>(32, b.rank - c0);
             hm_vpanel vp;
             vp.row0 = b.col0; vp.nrows = (int32_t)b.cols; vp.ld = w; vp.width = w; vp.slot = slot[i];
-            vp.col0 = (int32_t)c0; vp.pad = 0;
+            vp.col0 = (int32_t)c0;
+            vp.zeros = b.kind == 2 ? R - w : 0;       // the core is padded to R x R: its products read R coefficients
             vp.off = (int64_t)vstore.size();
             for (int64_t j = 0; j < b.cols; ++j)
                 for (int c = 0; c < w; ++c) {

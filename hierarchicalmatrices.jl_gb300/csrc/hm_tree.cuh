@@ -83,7 +83,8 @@ __device__ __forceinline__ bool last_arrival(int *count, int n, int lane)
 // once in shared memory (cp.async) and the chunks' x values double-buffered
 // beside them; longer panels are read directly.  Plain FMA accumulation
 // (the coefficients feed only the far field).  Coefficients of a slot are r
-// apart per right-hand side.
+// apart per right-hand side; those past a block of lower rank are set to zero
+// (hm_vpanel.zeros), because the far-field blocks read all r.
 // smem: leaf_up_warp_bytes of this warp.
 template <typename S, typename A, int QC>
 __device__ __forceinline__ void leaf_panel(const MulArgs<S> &ma, const hm_vpanel P, const hm_vpart part, const S *V,
@@ -101,10 +102,10 @@ __device__ __forceinline__ void leaf_panel(const MulArgs<S> &ma, const hm_vpanel
     A *out = part.nparts ? lp.sums + (int64_t)part.part * k * 32 : t + (int64_t)P.slot * k * r + P.col0;
     const int ldo = part.nparts ? 32 : r;
     auto store = [&](int q0, int qc, PlainAcc<A> *acc) {
-        if (lane < pw) {
+        if (lane < pw + P.zeros) {
 #pragma unroll
             for (int qq = 0; qq < QC; ++qq)
-                if (qq < qc) out[(int64_t)(q0 + qq) * ldo + lane] = acc[qq].value();
+                if (qq < qc) out[(int64_t)(q0 + qq) * ldo + lane] = lane < pw ? acc[qq].value() : A(0);
         }
     };
     if (P.nrows <= cap && P.ld == pw && pw <= wcap) {
@@ -204,7 +205,7 @@ __device__ __forceinline__ void leaf_panel(const MulArgs<S> &ma, const hm_vpanel
     if (part.nparts && last_arrival(lp.count + part.group, part.nparts, lane)) {
         A *tp = t + (int64_t)P.slot * k * r + P.col0 + lane;
         A *gp = lp.sums + (int64_t)(part.gpart + part.group - part.group0) * k * 32 + lane;
-        if (lane < pw) {
+        if (lane < pw + P.zeros) {                             // (the parts hold the zeros too)
             for (int q = 0; q < k; ++q) {
                 const A v = sum_parts(lp.sums, part.part0, part.nparts, k, q, lane);
                 if (part.ngroups == 1) tp[(int64_t)q * r] = v;
@@ -212,7 +213,7 @@ __device__ __forceinline__ void leaf_panel(const MulArgs<S> &ma, const hm_vpanel
             }
         }
         __syncwarp();
-        if (part.ngroups > 1 && last_arrival(lp.count + part.panel, part.ngroups, lane) && lane < pw)
+        if (part.ngroups > 1 && last_arrival(lp.count + part.panel, part.ngroups, lane) && lane < pw + P.zeros)
             for (int q = 0; q < k; ++q) tp[(int64_t)q * r] = sum_parts(lp.sums, part.gpart, part.ngroups, k, q, lane);
     }
 }

@@ -26,7 +26,8 @@ struct hm_vpanel {      // explicit basis panel: coef[slot][col0 + m] = (P^T x[r
     int32_t width;      // number of basis columns (<= 32)
     int32_t slot;
     int32_t col0;       // first coefficient of the slot this panel produces
-    int32_t pad;
+    int32_t zeros;      // coefficients after the panel's that are set to zero: a far-field block of
+                        // lower rank than the slots' (assembled matrices; width + zeros <= 32)
 };
 
 // One row part of a tall basis panel (a hm_vpanel record of its own, with the
