@@ -304,11 +304,15 @@ struct hm_handle {
         std::vector<Arg> args;
         const void *x = nullptr;
         void *y = nullptr;
-        ~ProductGraph()
+        void drop()
         {
             if (exec) cudaGraphExecDestroy(exec);
             if (graph) cudaGraphDestroy(graph);
+            exec = nullptr;
+            graph = nullptr;
+            args.clear();
         }
+        ~ProductGraph() { drop(); }
     };
 
     // Per caller stream: coefficient scratch (grown stream-ordered), the side
@@ -327,6 +331,8 @@ struct hm_handle {
         uint64_t graph_clock = 0;
     };
     std::map<void *, StreamCtx> streams;
+    // products by the form they ran in (hm_stats)
+    std::atomic<int64_t> fused_products{0}, graph_products{0}, failed_captures{0};
     void *d_stage = nullptr;
     size_t stage_bytes = 0;
     cudaStream_t host_stream = nullptr;
@@ -1876,11 +1882,14 @@ constexpr int kGraphAfter = 3;
 // and 126 / 113, 2^20 674 / 657 and 886 / 872; 8: 2^15 343 / 331 and 443 / 436, but 2^16 558
 // / 670 and 653 / 636 (the near field then takes the SMs before the far-field stage).
 // HM_DF64, 1: 2^16 112 / 106 and 120 / 116; 8: 222 / 208 and 309 / 297.
-template <typename S>
-bool graph_pays(const hm_handle *h, int k)
+// Panels in chunks of more than kPartMaxK right-hand sides stay plain launches: a chunk's
+// kernels take vectors of their own, which the update of a graph's addresses does not cover.
+template <typename S, typename A>
+bool graph_pays(const hm_handle *h, const MulArgs<S> &ma)
 {
-    const int slots = std::max(h->n_xslots, h->n_yslots);
-    if (k <= 2 || k > kPartMaxK || h->storage == HM_DF64 || slots < 2048) return true;
+    const int slots = std::max(h->n_xslots, h->n_yslots), k = ma.k;
+    if (k > kPartMaxK) return !near_apart<S, A>(h, ma);
+    if (k <= 2 || h->storage == HM_DF64 || slots < 2048) return true;
     return sizeof(S) == 4 && (k <= 4 || slots < 8192);
 }
 
@@ -1987,6 +1996,8 @@ int graph_mul(hm_handle *h, hm_handle::StreamCtx *sc, MulArgs<S> ma, cudaStream_
             cudaGetLastError();
             clear_last_error();
             g->bad = true;
+            g->drop();
+            ++h->failed_captures;
             return HM_OK;
         }
     }
@@ -2001,6 +2012,7 @@ int graph_mul(hm_handle *h, hm_handle::StreamCtx *sc, MulArgs<S> ma, cudaStream_
         g->y = ma.y;
     }
     *done = true;
+    ++h->graph_products;
     return cuda_status(cudaGraphLaunch(g->exec, st), "cudaGraphLaunch");
 }
 
@@ -2013,11 +2025,14 @@ int run_mul(hm_handle *h, MulArgs<S> ma, cudaStream_t st, const void *panels = n
     SchedScope scope(&sched);
     hm_handle::StreamCtx *sc = nullptr;
     HM_TRY(stream_ctx(h, st, stream_scratch_bytes<A>(h, ma.k), &sc));
-    if (fused_ok<S, A>(h, ma, sched)) return launch_fused<S, A>(h, ma, st, sc->p, sc->sync, panels ? panels : h->d_P);
+    if (fused_ok<S, A>(h, ma, sched)) {
+        ++h->fused_products;
+        return launch_fused<S, A>(h, ma, st, sc->p, sc->sync, panels ? panels : h->d_P);
+    }
     Sched run = sched;
     run.overlap = near_start(h, ma, sched.overlap);
     SchedScope staged(&run);
-    if (!trial && graph_pays<S>(h, ma.k)) {
+    if (!trial && graph_pays<S, A>(h, ma)) {
         bool done = false;
         HM_TRY((graph_mul<S, A>(h, sc, ma, st, run, panels ? panels : h->d_P, &done)));
         if (done) return HM_OK;
@@ -2764,7 +2779,8 @@ int hm_stats(const hm_handle *h, int64_t *out, int nout)
     const int64_t v[] = {h->stats.n_bary, h->stats.n_dense, h->stats.depth, h->stats.n_xslots,
                          h->stats.n_yslots, h->stats.canonical_values, h->stats.reference_values,
                          h->stats.stored_values, h->stats.dense_values, h->stats.n_segments,
-                         h->stats.max_width, h->device_bytes, h->launches_per_mul};
+                         h->stats.max_width, h->device_bytes, h->launches_per_mul,
+                         h->fused_products.load(), h->graph_products.load(), h->failed_captures.load()};
     const int nv = (int)(sizeof(v) / sizeof(v[0]));
     const int w = std::min(nv, nout);
     for (int i = 0; i < w; ++i) out[i] = v[i];

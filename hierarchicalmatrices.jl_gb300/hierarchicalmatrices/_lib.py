@@ -70,7 +70,7 @@ PLAN_SIZES = ("r", "nx", "ny", "n_xslots", "n_yslots", "vstore", "fstore", "psto
               "dense_values", "n_segments")
 STATS = ("n_bary", "n_dense", "depth", "n_xslots", "n_yslots", "canonical_values",
          "reference_values", "stored_values", "dense_values", "n_segments", "max_width",
-         "device_bytes", "launches_per_mul")
+         "device_bytes", "launches_per_mul", "fused_products", "graph_products", "failed_captures")
 STAGES = ("up", "down", "expand", "far", "product")
 
 EXPORTED = (

@@ -160,7 +160,9 @@ int hm_storage(const hm_handle *h);
    column slots, canonical stored values, reference-layout values, values this
    build stores, dense values, row segments, max panel width, device bytes,
    kernel launches per single-RHS hm_mul as stages with the side stream on (the
-   default beyond small trees, whose product is two launches).
+   default beyond small trees, whose product is two launches), products run
+   so far in two launches, as a CUDA graph, and forms of product whose capture
+   as a graph failed (they stay plain launches).
    Returns the number of values written (<= nout). */
 int hm_stats(const hm_handle *h, int64_t *out, int nout);
 
@@ -180,7 +182,9 @@ int hm_device_status(hm_handle *h, int *code, int reset);
    passes run on a side stream forked from and joined back into `stream`; a form
    of product (nrhs, leading dimensions, options) that a stream sees for the third
    time is captured as a CUDA graph, which later products launch with their own
-   u and v (not on a capturing stream, which gets the plain launches).
+   u and v (not on a capturing stream, which gets the plain launches, nor where
+   more than eight right-hand sides run without the tensor cores on large trees:
+   their panels are launched in chunks).
    nrhs = 0 reads and writes nothing (u and v may then be NULL), here and in
    hm_mul_t, hm_mul_drow and hm_mul_host. */
 int hm_mul(hm_handle *h, const void *v, int64_t ldv, void *u, int64_t ldu, int nrhs,
