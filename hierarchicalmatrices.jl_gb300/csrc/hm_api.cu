@@ -251,6 +251,7 @@ struct hm_handle {
     hm_vpanel *d_vp_split = nullptr;
     hm_vpart *d_vparts = nullptr;
     int n_vp_split = 0, n_part_slots = 0, n_part_counts = 0;
+    int part_cols = 0;              // most columns (with hm_vpanel's zeros) of a split panel
     hm_xfer *d_up = nullptr;
     std::vector<int> up_ptr;
     hm_m2l_row *d_m2l_rows = nullptr;
@@ -556,6 +557,7 @@ int split_tall_panels(hm_handle *h, const std::vector<hm_vpanel> &vps, cudaStrea
     std::vector<hm_vpanel> recs;
     std::vector<hm_vpart> parts;
     int64_t nslots = 0, ngroups = 0, npanels = 0;
+    int cols = 1;
     for (const hm_vpanel &p : vps) {
         if (p.nrows <= kPartRows) {
             recs.push_back(p);
@@ -584,6 +586,7 @@ int split_tall_panels(hm_handle *h, const std::vector<hm_vpanel> &vps, cudaStrea
         nslots += np + (ng > 1 ? ng : 0);
         ngroups += ng;
         npanels += 1;
+        cols = std::max(cols, p.width + p.zeros);
     }
     if ((int64_t)recs.size() > INT32_MAX || nslots > INT32_MAX) return HM_OK;      // whole panels
     for (hm_vpart &v : parts) v.panel += (int32_t)ngroups;
@@ -593,6 +596,7 @@ int split_tall_panels(hm_handle *h, const std::vector<hm_vpanel> &vps, cudaStrea
     h->n_vp_split = (int)recs.size();
     h->n_part_slots = (int)nslots;
     h->n_part_counts = (int)(ngroups + npanels);
+    h->part_cols = cols;
     return HM_OK;
 }
 
@@ -858,9 +862,10 @@ size_t parts_off(const hm_handle *h, int k)
     return L.yfar_off + (k <= 8 ? align256((size_t)h->nx * k * sizeof(A)) : 0);
 }
 template <typename A>
-size_t stream_scratch_bytes(const hm_handle *h, int k)
+size_t stream_scratch_bytes(const hm_handle *h, int k, bool parts)
 {
-    return parts_off<A>(h, k) + align256((size_t)h->n_part_slots * k * 32 * sizeof(A));
+    return parts_off<A>(h, k) +
+           (parts ? align256((size_t)h->n_part_slots * std::min(k, kPartRhs) * h->part_cols * sizeof(A)) : 0);
 }
 
 // Scratch, side stream and fork/join events for products issued on stream st.
@@ -985,9 +990,14 @@ int launch_tree_qc(hm_handle *h, const MulArgs<S> &ma, cudaStream_t st, A *t, A 
             const int cap = lp.rec ? kPartRows : h->vp_cap, n = lp.rec ? h->n_vp_split : h->n_vp;
             const size_t smem = (size_t)kWarpsPerCta * leaf_up_warp_bytes<S, A, QC>(cap, h->vp_wcap);
             HM_TRY(ensure_smem(leaf_up<S, A, QC>, smem));
-            leaf_up<S, A, QC><<<warp_ctas(n), 32 * kWarpsPerCta, smem, st>>>(
-                ma, lp.rec ? h->d_vp_split : h->d_vp, n, static_cast<const S *>(h->d_V), t, r, cap, h->vp_wcap, lp);
-            HM_CK_LAUNCH("leaf_up");
+            LeafParts<A> w = lp;
+            const int step = lp.rec ? kPartRhs : k;
+            for (w.q0 = 0; w.q0 < k; w.q0 += step) {
+                w.nq = std::min(step, k - w.q0);
+                leaf_up<S, A, QC><<<warp_ctas(n), 32 * kWarpsPerCta, smem, st>>>(
+                    ma, lp.rec ? h->d_vp_split : h->d_vp, n, static_cast<const S *>(h->d_V), t, r, cap, h->vp_wcap, w);
+                HM_CK_LAUNCH("leaf_up");
+            }
             chain = true;
         }
         if (mid && mid_after == 2) { HM_CK(cudaEventRecord(mid, st)); chain = false; }  // leaf bases done
@@ -1717,6 +1727,8 @@ int launch_fused(hm_handle *h, const MulArgs<S> &ma, cudaStream_t st, void *scra
         lp.rec = h->d_vparts;
         lp.sums = reinterpret_cast<A *>(static_cast<char *>(scratch) + parts_off<A>(h, k));
         lp.count = sync;
+        lp.width = h->part_cols;
+        lp.nq = k;
     }
     StageTimer whole(h, 4, st);
     bool done = false;             // the tree passes are launched
@@ -1801,6 +1813,7 @@ int launch_pipeline(hm_handle *h, const MulArgs<S> &ma, cudaStream_t st, cudaStr
         lp.rec = h->d_vparts;
         lp.sums = reinterpret_cast<A *>(static_cast<char *>(scratch) + parts_off<A>(h, k));
         lp.count = part_count;
+        lp.width = h->part_cols;
     }
     bool tree_chain = false;         // the tree passes ended with a kernel: the next launch may be dependent
     if (tree) {
@@ -2024,8 +2037,11 @@ int run_mul(hm_handle *h, MulArgs<S> ma, cudaStream_t st, const void *panels = n
     const Sched sched = sched_for(h, ma.k);
     SchedScope scope(&sched);
     hm_handle::StreamCtx *sc = nullptr;
-    HM_TRY(stream_ctx(h, st, stream_scratch_bytes<A>(h, ma.k), &sc));
-    if (fused_ok<S, A>(h, ma, sched)) {
+    const bool fused = fused_ok<S, A>(h, ma, sched);
+    // the lane-per-right-hand-side kernels take whole panels
+    const bool parts = h->d_vparts && (fused || !wide_tree_ok<S, A>(h, ma, sched.wide));
+    HM_TRY(stream_ctx(h, st, stream_scratch_bytes<A>(h, ma.k, parts), &sc));
+    if (fused) {
         ++h->fused_products;
         return launch_fused<S, A>(h, ma, st, sc->p, sc->sync, panels ? panels : h->d_P);
     }

@@ -67,7 +67,7 @@ __global__ void __launch_bounds__(kFusedThreads) tree_fused(const __grid_constan
             } else {
                 hm_vpart part{};
                 if (a.lp.rec) part = a.lp.rec[i];
-                leaf_panel<S, A, QC>(a.ma, a.vp[i], part, static_cast<const S *>(a.V), a.t, r, a.cap, a.wcap,
+                leaf_panel<S, A, QC>(a.ma, k, a.vp[i], part, static_cast<const S *>(a.V), a.t, r, a.cap, a.wcap,
                                      work + (size_t)wib * leaf_up_warp_bytes<S, A, QC>(a.cap, a.wcap), a.lp);
             }
             __syncwarp();

@@ -158,8 +158,15 @@ __global__ void leaf_up(MulArgs<S> ma, const hm_vpanel *vp, int npanels, const S
     const int64_t w = (int64_t)blockIdx.x * (blockDim.x >> 5) + wib;
     if (w >= (int64_t)npanels) return;
     hm_vpart part{};
-    if (lp.rec) part = lp.rec[w];
-    leaf_panel<S, A, QC>(ma, vp[w], part, V, t, r, cap, wcap,
+    const int kt = ma.k;
+    if (lp.rec) {
+        part = lp.rec[w];
+        ma.x += (int64_t)lp.q0 * ma.ldx;
+        if (ma.xin) ma.xin += (int64_t)lp.q0 * ma.ldx;
+        ma.k = lp.nq;
+        t += (int64_t)lp.q0 * r;
+    }
+    leaf_panel<S, A, QC>(ma, kt, vp[w], part, V, t, r, cap, wcap,
                          smem_raw + (size_t)wib * leaf_up_warp_bytes<S, A, QC>(cap, wcap), lp);
 }
 

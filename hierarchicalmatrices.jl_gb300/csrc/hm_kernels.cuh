@@ -165,13 +165,17 @@ __global__ void fill_segments(FillArgs fa, const hm_seg *segs, const hm_piece *p
 // ---------------------------------------------------------------- matvec
 
 // Tall basis panels split by rows: one hm_vpart per vp record (nullptr when no
-// panel is split), `sums` 32 values per (partial slot, right-hand side) and
-// `count` one zeroed arrival counter per group and panel (left zero again).
+// panel is split), `sums` `width` values per (partial slot, right-hand side of the
+// launch) and `count` one zeroed arrival counter per group and panel (left zero
+// again).  A launch takes the nq right-hand sides from q0 on: the partial sums of a
+// tall matrix are as large as its vectors, so no more than kPartRhs have them at once.
+constexpr int kPartRhs = 32;
 template <typename A>
 struct LeafParts {
     const hm_vpart *rec = nullptr;
     A *sums = nullptr;
     int *count = nullptr;
+    int width = 0, q0 = 0, nq = 0;
 };
 template <typename S, typename A, int QC>
 __global__ void leaf_up(MulArgs<S> ma, const hm_vpanel *vp, int npanels, const S *V, A *t, int r, int cap, int wcap,

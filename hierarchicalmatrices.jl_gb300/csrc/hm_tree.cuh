@@ -35,11 +35,11 @@ __device__ __forceinline__ void ld_vec(const A *p, A *v)
 // Adds `n` consecutive partial slots of lane's column in order, eight loads in
 // flight, for one right-hand side.
 template <typename A>
-__device__ __forceinline__ A sum_parts(const A *sums, int64_t first, int n, int k, int q, int lane)
+__device__ __forceinline__ A sum_parts(const A *sums, int64_t first, int n, int k, int q, int width, int lane)
 {
     A v = A(0);
-    const A *p = sums + (first * k + q) * 32 + lane;
-    const int64_t step = (int64_t)k * 32;
+    const A *p = sums + (first * k + q) * width + lane;
+    const int64_t step = (int64_t)k * width;
     int i = 0;
     for (; i + 8 <= n; i += 8) {
         A u[8];
@@ -83,12 +83,12 @@ __device__ __forceinline__ bool last_arrival(int *count, int n, int lane)
 // once in shared memory (cp.async) and the chunks' x values double-buffered
 // beside them; longer panels are read directly.  Plain FMA accumulation
 // (the coefficients feed only the far field).  Coefficients of a slot are r
-// apart per right-hand side; those past a block of lower rank are set to zero
+// apart per right-hand side (kt of them in all, ma.k of them here); those past a block of lower rank are set to zero
 // (hm_vpanel.zeros), because the far-field blocks read all r.
 // smem: leaf_up_warp_bytes of this warp.
 template <typename S, typename A, int QC>
-__device__ __forceinline__ void leaf_panel(const MulArgs<S> &ma, const hm_vpanel P, const hm_vpart part, const S *V,
-                                           A *t, int r, int cap, int wcap, unsigned char *smem,
+__device__ __forceinline__ void leaf_panel(const MulArgs<S> &ma, int kt, const hm_vpanel P, const hm_vpart part,
+                                           const S *V, A *t, int r, int cap, int wcap, unsigned char *smem,
                                            const LeafParts<A> &lp)
 {
     const int lane = threadIdx.x & 31;
@@ -99,8 +99,8 @@ __device__ __forceinline__ void leaf_panel(const MulArgs<S> &ma, const hm_vpanel
     const S *xsrc = ma.xin ? ma.xin : ma.x;
     S *xcopy = ma.xin ? const_cast<S *>(ma.x) : nullptr;
     // a whole panel's sums are its coefficients, a part's go to its partial slot
-    A *out = part.nparts ? lp.sums + (int64_t)part.part * k * 32 : t + (int64_t)P.slot * k * r + P.col0;
-    const int ldo = part.nparts ? 32 : r;
+    A *out = part.nparts ? lp.sums + (int64_t)part.part * k * lp.width : t + (int64_t)P.slot * kt * r + P.col0;
+    const int ldo = part.nparts ? lp.width : r;
     auto store = [&](int q0, int qc, PlainAcc<A> *acc) {
         if (lane < pw + P.zeros) {
 #pragma unroll
@@ -203,18 +203,19 @@ __device__ __forceinline__ void leaf_panel(const MulArgs<S> &ma, const hm_vpanel
         }
     }
     if (part.nparts && last_arrival(lp.count + part.group, part.nparts, lane)) {
-        A *tp = t + (int64_t)P.slot * k * r + P.col0 + lane;
-        A *gp = lp.sums + (int64_t)(part.gpart + part.group - part.group0) * k * 32 + lane;
+        A *tp = t + (int64_t)P.slot * kt * r + P.col0 + lane;
+        A *gp = lp.sums + (int64_t)(part.gpart + part.group - part.group0) * k * lp.width + lane;
         if (lane < pw + P.zeros) {                             // (the parts hold the zeros too)
             for (int q = 0; q < k; ++q) {
-                const A v = sum_parts(lp.sums, part.part0, part.nparts, k, q, lane);
+                const A v = sum_parts(lp.sums, part.part0, part.nparts, k, q, lp.width, lane);
                 if (part.ngroups == 1) tp[(int64_t)q * r] = v;
-                else gp[(int64_t)q * 32] = v;
+                else gp[(int64_t)q * lp.width] = v;
             }
         }
         __syncwarp();
         if (part.ngroups > 1 && last_arrival(lp.count + part.panel, part.ngroups, lane) && lane < pw + P.zeros)
-            for (int q = 0; q < k; ++q) tp[(int64_t)q * r] = sum_parts(lp.sums, part.gpart, part.ngroups, k, q, lane);
+            for (int q = 0; q < k; ++q)
+                tp[(int64_t)q * r] = sum_parts(lp.sums, part.gpart, part.ngroups, k, q, lp.width, lane);
     }
 }
 
