@@ -194,6 +194,7 @@ void transfer_matrices(int r, const std::vector<double> &x, const std::vector<do
 }
 
 // The options one product runs with (hm_configure's HM_OPT_* values).
+constexpr int kOverlapRule = 5;        // HM_OPT_OVERLAP's default: near_start, or the two-launch schedule
 struct Sched {
     int overlap, near_kernel, near_stages, tensor_cores, pdl;
     int tile = 0;      // per-warp ring tile (kRingTile index) for 3-8 FP32 right-hand sides
@@ -358,11 +359,11 @@ struct hm_handle {
     int64_t stage_launches[HM_NSTAGES] = {0};
     int launches_per_mul = 0;
     // 0: every stage in order on the caller's stream; 1: tree passes on a side
-    // stream from the start of the product, the near field beside them; 2 (the
-    // default): the near field starts after the upward pass, whose streaming
-    // leaf stage it would otherwise slow; 3: after the far-field (M2L) stage;
-    // 4: after the leaf stage only
-    int overlap = 2;
+    // stream from the start of the product, the near field beside them; 2: the
+    // near field starts after the upward pass, whose streaming leaf stage it
+    // would otherwise slow; 3: after the far-field (M2L) stage; 4: after the leaf
+    // stage only; 5 (the default): 1, 2 or 4 by near_start, or two launches (fused_ok)
+    int overlap = kOverlapRule;
     int near_stages = 4;            // ring stages of the near-field streaming kernel
     int near_kernel = 0;            // 0 default (one warp per segment), 1 the same, 2 streamed CTAs
     // programmatic dependent launches along the tree passes: on for FP32
@@ -1595,12 +1596,12 @@ bool fused_plan_k(const hm_handle *h, int k, bool split, FusedPlan &fp)
 }
 
 // Whether a product takes the fused schedule: the default stream schedule
-// (HM_OPT_OVERLAP 2) with the default panel kernels, ordinary device vectors, no
+// (HM_OPT_OVERLAP 5) with the default panel kernels, ordinary device vectors, no
 // stage timing, and a tree small enough.
 template <typename S, typename A>
 bool fused_ok(const hm_handle *h, const MulArgs<S> &ma, const Sched &sc)
 {
-    if (sc.overlap != 2 || sc.near_kernel != 0 || ma.xin || ma.yout || (h->profile_mask & 0xfu)) return false;
+    if (sc.overlap != kOverlapRule || sc.near_kernel != 0 || ma.xin || ma.yout || (h->profile_mask & 0xfu)) return false;
     if (!(h->n_vp || h->n_m2l_rows) || !h->n_segs || !h->stream_ctas) return false;
     if (ma.k > 2 && h->part_width[1] > 64) return false;
     const bool df = h->storage == HM_DF64;
@@ -1760,7 +1761,7 @@ int launch_fused(hm_handle *h, const MulArgs<S> &ma, cudaStream_t st, void *scra
 }
 
 // The stage of the tree passes that the near field starts after under the default
-// schedule (the result keeps its bits wherever it starts); HM_OPT_OVERLAP's values:
+// schedule (the result keeps its bits wherever it starts), as HM_OPT_OVERLAP's values:
 // 1 none, 2 the upward pass, 4 the leaf stage.  Right-hand sides in host memory
 // (MulArgs::xin) are brought in by the leaf stage, so the near field waits for it.
 // Measured, us per product, start after 2 / 4 / 1 (random points unless a grid):
@@ -1779,7 +1780,7 @@ int launch_fused(hm_handle *h, const MulArgs<S> &ma, cudaStream_t st, void *scra
 template <typename S>
 int near_start(const hm_handle *h, const MulArgs<S> &ma, int overlap)
 {
-    if (overlap != 2) return overlap;
+    if (overlap != kOverlapRule) return overlap;
     if (ma.k > kPartMaxK) return ma.xin ? 4 : 1;
     const int slots = std::max(h->n_xslots, h->n_yslots), k = ma.k;
     int m = 2;
@@ -1788,6 +1789,21 @@ int near_start(const hm_handle *h, const MulArgs<S> &ma, int overlap)
     else if (sizeof(S) == 4) m = k <= 2 ? (slots >= 8192 ? 4 : 2) : k <= 4 ? (slots >= 8192 ? 4 : 1)
                                  : (slots >= 2048 && slots < 16384 ? 4 : 1);
     return m == 1 && ma.xin ? 4 : m;
+}
+
+// A schedule's overlap as hm_autotune and hm_autotune_choice report it: for the rule
+// where k right-hand sides on the device start the near field (2 also for a product in
+// two launches).
+int shown_overlap(const hm_handle *h, int overlap, int k)
+{
+    if (f64_vectors(h->storage)) {
+        MulArgs<double> ma{};
+        ma.k = k;
+        return near_start(h, ma, overlap);
+    }
+    MulArgs<float> ma{};
+    ma.k = k;
+    return near_start(h, ma, overlap);
 }
 
 // One product.  With a side stream the tree passes and the far-field rows
@@ -2243,7 +2259,7 @@ int autotune(hm_handle *h, int k, int reps, cudaStream_t st, int32_t *choice, do
     }
     drop_host_graph(h);             // it was captured with the previous schedule
     if (choice) {
-        choice[0] = cand[bi].overlap;
+        choice[0] = shown_overlap(h, cand[bi].overlap, k);
         choice[1] = cand[bi].near_kernel;
         choice[2] = cand[bi].near_stages;
         choice[3] = cand[bi].tensor_cores;
@@ -2989,7 +3005,7 @@ int hm_autotune_choice(const hm_handle *h, int nrhs, int32_t *out, int nout)
         std::lock_guard<std::mutex> lk(const_cast<hm_handle *>(h)->mu);
         sc = h->tuned_ok[b] ? h->tuned[b] : configured_sched(h);
     }
-    const int32_t v[7] = {sc.overlap, sc.near_kernel, sc.near_stages, sc.tensor_cores, sc.pdl, sc.tile, sc.wide};
+    const int32_t v[7] = {shown_overlap(h, sc.overlap, nrhs), sc.near_kernel, sc.near_stages, sc.tensor_cores, sc.pdl, sc.tile, sc.wide};
     const int n = std::min(nout, 7);
     for (int i = 0; i < n; ++i) out[i] = v[i];
     return n;
@@ -3046,7 +3062,7 @@ int hm_configure(hm_handle *h, int option, int64_t value)
     }
     switch (option) {
     case HM_OPT_OVERLAP:
-        if (value < 0 || value > 4) { set_error("HM_OPT_OVERLAP must be in [0, 4]"); return HM_ERR_INVALID_ARG; }
+        if (value < 0 || value > kOverlapRule) { set_error("HM_OPT_OVERLAP must be in [0, 5]"); return HM_ERR_INVALID_ARG; }
         break;
     case HM_OPT_TENSOR_CORES: break;
     case HM_OPT_NEAR_KERNEL:

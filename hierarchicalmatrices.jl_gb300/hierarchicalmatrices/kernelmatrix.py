@@ -334,11 +334,11 @@ class KernelMatrix:
 
     def set_overlap(self, enable=True):
         """Tree passes on a side stream beside the near-field panels: the near
-        field from the start (1), after the far-field stage (3), after the
-        leaf-basis stage (4) or where size and right-hand sides make it
-        fastest, a small matrix's product in two kernels (2; True, the
-        default); or every stage in order (False or 0)."""
-        mode = int(enable) if not isinstance(enable, bool) else (2 if enable else 0)
+        field from the start (1), after the upward pass (2), after the
+        far-field stage (3), after the leaf-basis stage (4) or where size and
+        right-hand sides make it fastest, a small matrix's product in two
+        kernels (5; True, the default); or every stage in order (False or 0)."""
+        mode = int(enable) if not isinstance(enable, bool) else (5 if enable else 0)
         check(lib.hm_configure(self._h, _lib.HM_OPT_OVERLAP, mode))
 
     def set_pdl(self, enable=True):

@@ -239,13 +239,13 @@ int hm_mul_host(hm_handle *h, const void *v, void *u, int nrhs, int accumulate);
 int hm_direct_rows(hm_handle *h, const double *b, const int64_t *rows, int64_t nrows, double *out,
                    void *stream);
 
-/* Handle options.  HM_OPT_OVERLAP (default 2): 1 runs the tree passes of
+/* Handle options.  HM_OPT_OVERLAP (default 5): 1 runs the tree passes of
    hm_mul on a side stream concurrently with the near-field panels from the
-   start, 3 starts the near field after the far-field (M2L) stage, 4 after the
-   leaf-basis stage of the upward pass, 2 where storage, size and right-hand
-   sides make it fastest (after the upward pass, as 4 or as 1), with a small
-   matrix's product in two kernels; 0 runs every stage in order on the
-   caller's stream. */
+   start, 2 starts the near field after the upward pass, 3 after the
+   far-field (M2L) stage, 4 after the leaf-basis stage of the upward pass; 5
+   takes the one of 1, 2 and 4 that storage, size and right-hand sides make
+   fastest, and a small matrix's product in two kernels; 0 runs every stage in
+   order on the caller's stream. */
 enum {
     HM_OPT_OVERLAP = 1,
     /* HM_OPT_NEAR_STAGES (default 4, 2..16): shared-memory stages (8 KB each)
@@ -311,8 +311,8 @@ int hm_configure(hm_handle *h, int option, int64_t value);
    two rounds with the better time kept) and keeps the fastest for nrhs's
    bucket (1, 2, 3-4, 5-8, 9-16, 17-32, 33-64, 65-128, 129+): later hm_mul,
    hm_mul_strided, hm_mul_host and hm_mul_drow calls of that bucket run with
-   it, including inside stream capture.  Candidates: HM_OPT_OVERLAP 0..4
-   (0..1 above 8 right-hand sides), HM_OPT_NEAR_KERNEL 0 (with each of the
+   it, including inside stream capture.  Candidates: the configured options,
+   HM_OPT_OVERLAP 0..4 (0..1 above 8 right-hand sides), HM_OPT_NEAR_KERNEL 0 (with each of the
    three ring tiles for 3-8 FP32 right-hand sides), 1 (FP32 with 3-8
    right-hand sides) or 2 with HM_OPT_NEAR_STAGES 3, 4 or 6 (up to 8
    right-hand sides), HM_OPT_WIDE_TREE on or off,
@@ -320,7 +320,7 @@ int hm_configure(hm_handle *h, int option, int64_t value);
    on or off (FP32, 16 or more), HM_OPT_PDL on or off.  Inputs are scratch vectors allocated on
    `stream` and freed before return; synchronous; not allowed while `stream`
    is being captured.  choice (host, 5 values, may be NULL) receives the
-   chosen overlap, near kernel, near stages, tensor-core flag and PDL flag; ms (host, 2
+   chosen overlap (HM_OPT_OVERLAP 5 as the value it takes, 2 for two kernels), near kernel, near stages, tensor-core flag and PDL flag; ms (host, 2
    values, may be NULL) the chosen schedule's time per product and that of
    the configured options.  Like hm_configure, it changes the handle: do not
    call it while products on the same handle are being issued from other
