@@ -1603,6 +1603,7 @@ bool fused_ok(const hm_handle *h, const MulArgs<S> &ma, const Sched &sc)
 {
     if (sc.overlap != kOverlapRule || sc.near_kernel != 0 || ma.xin || ma.yout || (h->profile_mask & 0xfu)) return false;
     if (!(h->n_vp || h->n_m2l_rows) || !h->n_segs || !h->stream_ctas) return false;
+    if (sc.wide >= 2 && wide_tree_ok<S, A>(h, ma, sc.wide)) return false;      // HM_OPT_WIDE_TREE 2 names its kernels
     if (ma.k > 2 && h->part_width[1] > 64) return false;
     const bool df = h->storage == HM_DF64;
     if (df && h->n_m2l_rows && h->r != 20) return false;
