@@ -1601,7 +1601,7 @@ bool fused_plan_k(const hm_handle *h, int k, bool split, FusedPlan &fp)
 template <typename S, typename A>
 bool fused_ok(const hm_handle *h, const MulArgs<S> &ma, const Sched &sc)
 {
-    if (sc.overlap != kOverlapRule || sc.near_kernel != 0 || ma.xin || ma.yout || (h->profile_mask & 0xfu)) return false;
+    if (sc.overlap != kOverlapRule || sc.near_kernel != 0 || ma.k > kPartMaxK || ma.xin || ma.yout || (h->profile_mask & 0xfu)) return false;
     if (!(h->n_vp || h->n_m2l_rows) || !h->n_segs || !h->stream_ctas) return false;
     if (sc.wide >= 2 && wide_tree_ok<S, A>(h, ma, sc.wide)) return false;      // HM_OPT_WIDE_TREE 2 names its kernels
     if (ma.k > 2 && h->part_width[1] > 64) return false;
@@ -1616,7 +1616,7 @@ bool fused_ok(const hm_handle *h, const MulArgs<S> &ma, const Sched &sc)
     else
         fits = fused_plan_k<S, A>(h, ma.k, split, fp);
     // expand_both gathers whole segments; wider ones keep the streaming kernels
-    const size_t kb = ma.k > kPartMaxK ? 0 : ma.k > 4 ? 8 : ma.k > 2 ? 4 : 2;
+    const size_t kb = ma.k > 4 ? 8 : ma.k > 2 ? 4 : 2;
     if (!fits || kWarpsPerCta * (size_t)h->max_width * kb * (df ? sizeof(float2) : sizeof(A)) > 100 * 1024) return false;
     // The lines, in coefficient slots (about n / 30), where the cluster's 16 SMs
     // take as long as the stage kernels on all of them, launched as a graph (us, fused
@@ -1628,10 +1628,10 @@ bool fused_ok(const hm_handle *h, const MulArgs<S> &ma, const Sched &sc)
     // 252; 4: 50 / 56 at 60; 8: 89 / 93 at 60.  Matrices without transfers or far-field
     // blocks (low-rank factors only) run their one tree stage on all SMs at any size.
     const int slots = std::max(h->n_xslots, h->n_yslots), k = ma.k;
-    if (!has_transfers(h)) return k <= kPartMaxK;
-    if (df) return slots <= (k == 1 ? 40 : k == 2 ? 130 : k <= 8 ? 80 : 0);
+    if (!has_transfers(h)) return true;
+    if (df) return slots <= (k == 1 ? 40 : k == 2 ? 130 : 80);
     if (sizeof(S) == 8) return slots <= (k <= 2 ? 140 : k <= 4 ? 100 : 0);
-    return slots <= (k <= 4 ? 200 : k <= 8 ? 160 : 0);
+    return slots <= (k <= 4 ? 200 : 160);
 }
 
 // Clusters of kFusedCtas (beyond the portable 8) for `kernel`, set once per device.
@@ -1648,7 +1648,7 @@ int allow_cluster(K kernel)
 }
 
 template <typename S, typename A, int QC, bool DF>
-int launch_tree_fused(hm_handle *h, const MulArgs<S> &ma, cudaStream_t st, A *t, A *s, const LeafParts<A> &lp, int *sync)
+int launch_tree_fused(hm_handle *h, const MulArgs<S> &ma, cudaStream_t st, A *t, A *s, const LeafParts<A> &lp)
 {
     TreeArgs<S, A> a;
     a.ma = ma;
@@ -1741,18 +1741,17 @@ int launch_fused(hm_handle *h, const MulArgs<S> &ma, cudaStream_t st, void *scra
     if constexpr (std::is_same<S, double>::value) {
         if (!done && h->storage == HM_DF64) {
             done = true;
-            HM_TRY((launch_tree_fused<S, A, 1, true>(h, ma, st, t, s, lp, sync)));
+            HM_TRY((launch_tree_fused<S, A, 1, true>(h, ma, st, t, s, lp)));
         }
     }
     if (!done) {
         const int qc = tree_chunk(k);
-        HM_TRY((qc == 1   ? launch_tree_fused<S, A, 1, false>(h, ma, st, t, s, lp, sync)
-                : qc == 2 ? launch_tree_fused<S, A, 2, false>(h, ma, st, t, s, lp, sync)
-                : qc == 4 ? launch_tree_fused<S, A, 4, false>(h, ma, st, t, s, lp, sync)
-                          : launch_tree_fused<S, A, 8, false>(h, ma, st, t, s, lp, sync)));
+        HM_TRY((qc == 1   ? launch_tree_fused<S, A, 1, false>(h, ma, st, t, s, lp)
+                : qc == 2 ? launch_tree_fused<S, A, 2, false>(h, ma, st, t, s, lp)
+                : qc == 4 ? launch_tree_fused<S, A, 4, false>(h, ma, st, t, s, lp)
+                          : launch_tree_fused<S, A, 8, false>(h, ma, st, t, s, lp)));
     }
-    if (k > kPartMaxK) return launch_expand_k<S, A>(h, ma, s, t, panels, st);
-    const bool pdl = h->pdl != 0;
+    const bool pdl = cur_sched(h).pdl != 0;
     if constexpr (sizeof(S) == 8) {
         if (k == 1) return launch_both<S, A, 1>(h, ma, st, t, s, panels, pdl);
     }
