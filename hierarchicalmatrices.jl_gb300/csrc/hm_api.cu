@@ -1566,6 +1566,45 @@ struct FusedPlan {
     int leaf_warps, m2l_warps;
 };
 
+// Whether the device places a cluster of kFusedCtas CTAs (beyond the portable 8) of
+// `kernel` with that shared memory, asked once per device, kernel and shared memory: a
+// whole GB300 does, a partition of one may not, and a launch there would fail.
+std::map<std::tuple<int, const void *, size_t>, bool> g_cluster_fits;
+template <typename K>
+bool cluster_fits(K kernel, size_t smem)
+{
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return false;
+    const auto key = std::make_tuple(dev, reinterpret_cast<const void *>(kernel), smem);
+    {
+        std::lock_guard<std::mutex> lk(g_smem_mu);
+        const auto it = g_cluster_fits.find(key);
+        if (it != g_cluster_fits.end()) return it->second;
+    }
+    int n = 0;
+    bool ok = ensure_smem(kernel, smem) == HM_OK &&
+              cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+    if (ok) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(kFusedCtas);
+        cfg.blockDim = dim3(kFusedThreads);
+        cfg.dynamicSmemBytes = smem;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = kFusedCtas;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        ok = cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) == cudaSuccess && n > 0;
+    }
+    if (!ok) {                                     // the stage kernels run: not an error
+        cudaGetLastError();
+        clear_last_error();
+    }
+    std::lock_guard<std::mutex> lk(g_smem_mu);
+    return g_cluster_fits[key] = ok;
+}
+
 template <typename S, typename A, int QC, bool DF>
 bool fused_plan(const hm_handle *h, bool split, FusedPlan &fp)
 {
@@ -1582,7 +1621,7 @@ bool fused_plan(const hm_handle *h, bool split, FusedPlan &fp)
     const size_t lv = (size_t)(DF ? 1 : QC) * h->r * es;
     fp.smem = ts + std::max(std::max(h->n_vp ? fp.leaf_warps * lb : 0, h->n_m2l_rows ? fp.m2l_warps * mb : 0),
                             (size_t)std::max(h->band_locals[0], h->band_locals[1]) * lv);
-    return fp.smem <= kTaskSmemMax;
+    return fp.smem <= kTaskSmemMax && (!has_transfers(h) || cluster_fits(tree_fused<S, A, QC, DF>, fp.smem));
 }
 
 template <typename S, typename A>
@@ -1608,16 +1647,6 @@ bool fused_ok(const hm_handle *h, const MulArgs<S> &ma, const Sched &sc)
     const bool df = h->storage == HM_DF64;
     if (df && h->n_m2l_rows && h->r != 20) return false;
     if (h->up_band_ptr.size() > kFusedBands + 1 || h->down_band_ptr.size() > kFusedBands + 1) return false;
-    const bool split = h->d_vparts != nullptr;
-    FusedPlan fp;
-    bool fits;
-    if constexpr (std::is_same<S, double>::value)
-        fits = df ? fused_plan<S, A, 1, true>(h, split, fp) : fused_plan_k<S, A>(h, ma.k, split, fp);
-    else
-        fits = fused_plan_k<S, A>(h, ma.k, split, fp);
-    // expand_both gathers whole segments; wider ones keep the streaming kernels
-    const size_t kb = ma.k > 4 ? 8 : ma.k > 2 ? 4 : 2;
-    if (!fits || kWarpsPerCta * (size_t)h->max_width * kb * (df ? sizeof(float2) : sizeof(A)) > 100 * 1024) return false;
     // The lines, in coefficient slots (about n / 30), where the cluster's 16 SMs
     // take as long as the stage kernels on all of them, launched as a graph (us, fused
     // against stages): FP32, 1 right-hand side: 16.5 / 17.5 at 28, 17.7 / 19.5 at 124, 23.5 /
@@ -1627,24 +1656,18 @@ bool fused_ok(const hm_handle *h, const MulArgs<S> &ma, const Sched &sc)
     // HM_DF64, 1: 24.4 / 25.5 at 28, 33.5 / 31.7 at 124; 2: 40.0 / 41.7 at 124, 56 / 47 at
     // 252; 4: 50 / 56 at 60; 8: 89 / 93 at 60.  Matrices without transfers or far-field
     // blocks (low-rank factors only) run their one tree stage on all SMs at any size.
-    const int slots = std::max(h->n_xslots, h->n_yslots), k = ma.k;
-    if (!has_transfers(h)) return true;
-    if (df) return slots <= (k == 1 ? 40 : k == 2 ? 130 : 80);
-    if (sizeof(S) == 8) return slots <= (k <= 2 ? 140 : k <= 4 ? 100 : 0);
-    return slots <= (k <= 4 ? 200 : 160);
-}
-
-// Clusters of kFusedCtas (beyond the portable 8) for `kernel`, set once per device.
-std::set<std::pair<int, const void *>> g_cluster_set;
-template <typename K>
-int allow_cluster(K kernel)
-{
-    int dev = 0;
-    HM_CK(cudaGetDevice(&dev));
-    std::lock_guard<std::mutex> lk(g_smem_mu);
-    if (!g_cluster_set.insert({dev, reinterpret_cast<const void *>(kernel)}).second) return HM_OK;
-    HM_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    return HM_OK;
+    const int k = ma.k, most = df ? (k == 1 ? 40 : k == 2 ? 130 : 80)
+                               : sizeof(S) == 8 ? (k <= 2 ? 140 : k <= 4 ? 100 : 0) : (k <= 4 ? 200 : 160);
+    if (has_transfers(h) && std::max(h->n_xslots, h->n_yslots) > most) return false;
+    // expand_both gathers whole segments; wider ones keep the streaming kernels
+    const size_t kb = k > 4 ? 8 : k > 2 ? 4 : 2;
+    if (kWarpsPerCta * (size_t)h->max_width * kb * (df ? sizeof(float2) : sizeof(A)) > 100 * 1024) return false;
+    const bool split = h->d_vparts != nullptr;
+    FusedPlan fp;
+    if constexpr (std::is_same<S, double>::value) {
+        if (df) return fused_plan<S, A, 1, true>(h, split, fp);
+    }
+    return fused_plan_k<S, A>(h, k, split, fp);
 }
 
 template <typename S, typename A, int QC, bool DF>
@@ -1680,7 +1703,6 @@ int launch_tree_fused(hm_handle *h, const MulArgs<S> &ma, cudaStream_t st, A *t,
     a.m2l_warps = fp.m2l_warps;
     auto kern = tree_fused<S, A, QC, DF>;
     HM_TRY(ensure_smem(kern, fp.smem));
-    HM_TRY(allow_cluster(kern));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(kFusedCtas);
     cfg.blockDim = dim3(kFusedThreads);
