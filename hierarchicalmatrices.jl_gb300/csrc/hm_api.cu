@@ -2003,10 +2003,11 @@ int capture_product(hm_handle *h, hm_handle::StreamCtx *sc, hm_handle::ProductGr
     return HM_OK;
 }
 
-// Runs the product as a graph; *done = false when it has to be launched plainly.
+// Runs the product as a graph from the form's product number `after` on; *done = false when
+// it has to be launched plainly.
 template <typename S, typename A>
 int graph_mul(hm_handle *h, hm_handle::StreamCtx *sc, MulArgs<S> ma, cudaStream_t st, const Sched &run,
-              const void *panels, bool *done)
+              const void *panels, int after, bool *done)
 {
     *done = false;
     if (ma.xin || ma.yout || h->profile_mask) return HM_OK;
@@ -2034,7 +2035,7 @@ int graph_mul(hm_handle *h, hm_handle::StreamCtx *sc, MulArgs<S> ma, cudaStream_
         g->key = key;
     }
     g->used = ++sc->graph_clock;
-    if (g->bad || ++g->seen < kGraphAfter) return HM_OK;
+    if (g->bad || ++g->seen < after) return HM_OK;
     if (!g->exec) {
         g->seen = kGraphAfter;
         // the calls of a capture and an instantiation are legal beside another thread's
@@ -2071,7 +2072,7 @@ template <typename S, typename A>
 int run_mul(hm_handle *h, MulArgs<S> ma, cudaStream_t st, const void *panels = nullptr)
 {
     if (ma.k <= 0) return HM_OK;
-    const bool trial = t_sched != nullptr;                 // hm_autotune: plain launches of its candidates
+    const bool trial = t_sched != nullptr;                 // a candidate of hm_autotune: timed in the form it will run in
     const Sched sched = sched_for(h, ma.k);
     SchedScope scope(&sched);
     hm_handle::StreamCtx *sc = nullptr;
@@ -2086,9 +2087,9 @@ int run_mul(hm_handle *h, MulArgs<S> ma, cudaStream_t st, const void *panels = n
     Sched run = sched;
     run.overlap = near_start(h, ma, sched.overlap);
     SchedScope staged(&run);
-    if (!trial && graph_pays<S, A>(h, ma)) {
+    if (graph_pays<S, A>(h, ma)) {
         bool done = false;
-        HM_TRY((graph_mul<S, A>(h, sc, ma, st, run, panels ? panels : h->d_P, &done)));
+        HM_TRY((graph_mul<S, A>(h, sc, ma, st, run, panels ? panels : h->d_P, trial ? 1 : kGraphAfter, &done)));
         if (done) return HM_OK;
     }
     StageTimer whole(h, 4, st);
