@@ -273,7 +273,9 @@ enum {
        far-field rows after them) are launched as programmatic dependents of
        the kernel before them on the stream, so that each is scheduled while
        its predecessor finishes and stages its constant inputs before it waits
-       for the predecessor's results; 0 launches them plainly. */
+       for the predecessor's results; 0 launches them plainly.  The second
+       launch of a small matrix's product is one for every storage type
+       unless this option was set to 0. */
     HM_OPT_PDL = 6,
     /* HM_OPT_WAIT_LIMIT_NS (default 2e9, 1..2e9): nanoseconds after which a
        wait of the streamed near-field kernel (HM_OPT_NEAR_KERNEL 2) or of the
