@@ -1587,7 +1587,6 @@ struct LrPlan {
 // Shared memory up to which panels are staged: whole SMs while a launch has an SM
 // per problem, a third of one for larger batches (whose CTAs share the SMs).
 constexpr size_t kPanelSmemBytes = 224 * 1024, kPanelSmemBytesMany = 72 * 1024;
-constexpr int kPanelFew = 152;
 
 template <typename T>
 int lr_svd_plan(int nprob, const LrJob *jobs, LrPlan &pl)
@@ -1661,7 +1660,10 @@ int lr_svd_plan(int nprob, const LrJob *jobs, LrPlan &pl)
         pl.smem = (size_t)(xoff + xmax) * sizeof(T);
     }
     pl.soff = (int64_t)((pl.smem + 15) / 16 * 16 / sizeof(T));
-    const size_t most = nprob <= kPanelFew ? kPanelSmemBytes : kPanelSmemBytesMany;
+    int dev = 0, sms = 0;
+    ALG_CK(cudaGetDevice(&dev));
+    ALG_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    const size_t most = nprob <= sms ? kPanelSmemBytes : kPanelSmemBytesMany;
     for (int i = 0; i < nprob; ++i) {
         const hm_lr_problem &p = jobs[i].p;
         const int64_t v = p.qr_left || p.qr_right ? lr_panel_vals(p) : 0;
