@@ -547,7 +547,7 @@ void set_vp_caps(hm_handle *h, const std::vector<hm_vpanel> &vps)
 // Rows of a basis panel one warp takes: a taller panel is split into parts of
 // this many rows, its parts into groups of kPartGroup (leaf_up).  128 rows is
 // what leaf_up stages in shared memory; a 16,384-row HODLR product in FP64 took
-// 1,350 us with one warp per panel and takes 47 us (what issuing its five launches takes) with these parts.
+// 1,350 us with one warp per panel; with these parts 47 us as five launches, 25 as two.
 constexpr int kPartRows = 128, kPartGroup = 64;
 
 int split_tall_panels(hm_handle *h, const std::vector<hm_vpanel> &vps, cudaStream_t st)

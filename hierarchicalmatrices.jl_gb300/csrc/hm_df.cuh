@@ -1,5 +1,5 @@
 // Device bodies of the double-float (HM_DF64) tree passes, for the stage kernels
-// (hm_df.cu).  Written for sm_103a.
+// (hm_df.cu) and the two-launch schedule (hm_fused.cu).  Written for sm_103a.
 #pragma once
 #include "hm_async.cuh"
 #include "hm_kernels.cuh"

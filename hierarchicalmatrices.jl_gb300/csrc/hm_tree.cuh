@@ -1,5 +1,6 @@
 // Device bodies of the tree passes and of a row segment's sums, for the stage
-// kernels (one launch per stage, hm_kernels.cu, hm_df.cu).  Written for sm_103a.
+// kernels (one launch per stage, hm_kernels.cu, hm_df.cu) and the two-launch
+// schedule of small matrices (hm_fused.cu).  Written for sm_103a.
 #pragma once
 #include "hm_async.cuh"
 #include "hm_kernels.cuh"
