@@ -244,7 +244,7 @@ struct hm_handle {
     int n_vp = 0;
     int vp_cap = 64, vp_wcap = HM_RMAX;   // leaf_up's shared-memory panel: rows (multiple of 32) x columns
     bool vp_covers_x = false;             // the leaf panels' rows partition [0, ny): leaf_up reads every x once
-    bool vp_wide = false;                 // every leaf panel row-major with ld == width == 20 (leaf_up_w)
+    bool vp_wide = false;                 // every leaf panel row-major, ld == width == 20, <= 128 rows (leaf_up_w, leaf_flat): none is split
     int wide_tree = 1;                    // lane-per-RHS tree kernels: 0 never, 1 by rule, 2 from 2 (HM_OPT_WIDE_TREE)
     int ring_tile = 0;                    // per-warp ring tile (HM_OPT_RING_TILE)
     // the panels with those of more than kPartRows rows split by rows (leaf_up's
@@ -863,10 +863,9 @@ size_t parts_off(const hm_handle *h, int k)
     return L.yfar_off + (k <= 8 ? align256((size_t)h->nx * k * sizeof(A)) : 0);
 }
 template <typename A>
-size_t stream_scratch_bytes(const hm_handle *h, int k, bool parts)
+size_t stream_scratch_bytes(const hm_handle *h, int k)
 {
-    return parts_off<A>(h, k) +
-           (parts ? align256((size_t)h->n_part_slots * std::min(k, kPartRhs) * h->part_cols * sizeof(A)) : 0);
+    return parts_off<A>(h, k) + align256((size_t)h->n_part_slots * std::min(k, kPartRhs) * h->part_cols * sizeof(A));
 }
 
 // Scratch, side stream and fork/join events for products issued on stream st.
@@ -2080,11 +2079,8 @@ int run_mul(hm_handle *h, MulArgs<S> ma, cudaStream_t st, const void *panels = n
     const Sched sched = sched_for(h, ma.k);
     SchedScope scope(&sched);
     hm_handle::StreamCtx *sc = nullptr;
-    const bool fused = fused_ok<S, A>(h, ma, sched);
-    // the lane-per-right-hand-side kernels take whole panels
-    const bool parts = h->d_vparts && (fused || !wide_tree_ok<S, A>(h, ma, sched.wide));
-    HM_TRY(stream_ctx(h, st, stream_scratch_bytes<A>(h, ma.k, parts), &sc));
-    if (fused) {
+    HM_TRY(stream_ctx(h, st, stream_scratch_bytes<A>(h, ma.k), &sc));
+    if (fused_ok<S, A>(h, ma, sched)) {
         ++h->fused_products;
         return launch_fused<S, A>(h, ma, st, sc->p, sc->sync, panels ? panels : h->d_P);
     }
